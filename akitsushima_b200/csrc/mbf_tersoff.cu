@@ -1,24 +1,36 @@
-// Tersoff bond-order potential: zeta/bond-order kernel, force kernel with
-// per-slot three-body forces, gather through the reverse-slot index.
+// Tersoff bond-order potential: one kernel per evaluation over the centres
+// (zeta, bond orders, energies, the force of every centre's own terms on its
+// neighbours), then the gather of the slots.
 //
 // Replaces engine/tersoff.py:1208-1711 (single-species :1233-1513 with m = 3
 // and gamma = 1, multi-species :1518-1711 with its dense species tables
-// :1606-1653).  Energy E = sum_{i<j} fc (fR + b_avg fA), b_avg the mean of
-// the two bond orders (engine/tersoff.py:6-19).
+// :1606-1653).  The energy sum_{i<j} fc (fR + b_avg fA), b_avg the mean of the
+// two bond orders (engine/tersoff.py:6-19), is the sum over centres of
+//   U_i = 1/2 sum_j fc_ij (fR_ij + b_ij fA_ij),
+// which needs the centre's own bond orders only.
 //
 // Owner computes, no atomics: the lane group of centre i evaluates every
-// zeta-term gradient of its angles, keeps the force on i and writes the force
-// its angles put on neighbour x into x's own slot (x -> i); atom a later sums
-// its own row of slots (gather_reduce).
+// term of U_i, keeps the force on i and writes -dU_i/dr_x into x's own slot
+// (x -> i); atom a later sums its own row of slots (gather_reduce).
 #include "mbf_util.cuh"
 
 namespace mbf {
 
 // Lanes per atom (LPA) is a template parameter chosen by the host (the
-// autotuner); lane groups per block keep the staged rows under 48 KB.
+// autotuner); GPB lane groups per block keep the staged rows near 20 KB, so
+// the blocks of one SM end at different times and its last wave is short
+// (eight groups against sixteen, 32,768-atom SiC: 89 against 92 us).
 template <int MAXN, int LPA> struct TeGeom {
-    static constexpr int GPB = 512 / MAXN;
+    static constexpr int GPB = 256 / MAXN;
     static constexpr int BLOCK = GPB * LPA;
+    // Resident threads per SM the kernel is compiled for, its register
+    // budget: 128 in float64, 96 in mixed precision.  SiC, 8 lanes, us at 384
+    // / 512 / 640 / 768 threads: 86 / 80 / 82 / 97 in float64; in mixed, at
+    // 512 / 640 / 768 / 1024: 72 / 64 / 64 / 70.
+    static constexpr int min_blocks(int size) {
+        const int b = (size == 8 ? 512 : 640) / BLOCK;
+        return b < 32 ? b : 32;
+    }
 };
 
 struct TeDev {
@@ -28,17 +40,21 @@ struct TeDev {
     double rc;
 };
 
-template <typename T>
-__device__ __forceinline__ T te_fc(T r, T R, T D) {
-    if (r < R - D) return T(1);
-    if (r > R + D) return T(0);
-    return T(0.5) - T(0.5) * RT<T>::sn(T(0.5) * T(3.14159265358979323846) * (r - R) / D);
-}
+__device__ __forceinline__ void te_sincospi(double x, double &s, double &c) { sincospi(x, &s, &c); }
+__device__ __forceinline__ void te_sincospi(float x, float &s, float &c) { sincospif(x, &s, &c); }
 
+// The cutoff function fc and its derivative (engine/tersoff.py:48-60).
 template <typename T>
-__device__ __forceinline__ T te_dfc(T r, T R, T D) {
-    if (r < R - D || r > R + D) return T(0);
-    return T(-0.25) * T(3.14159265358979323846) / D * RT<T>::cs(T(0.5) * T(3.14159265358979323846) * (r - R) / D);
+__device__ __forceinline__ void te_cut(T r, T R, T D, T &fc, T &dfc) {
+    fc = T(1);
+    dfc = T(0);
+    if (r < R - D) return;
+    fc = T(0);
+    if (r > R + D) return;
+    T s, c;
+    te_sincospi(T(0.5) * (r - R) / D, s, c);
+    fc = T(0.5) - T(0.5) * s;
+    dfc = T(-0.25) * T(3.14159265358979323846) / D * c;
 }
 
 // (l3 u)^m for m = 1 or 3 by multiplication, pow otherwise.
@@ -49,377 +65,474 @@ __device__ __forceinline__ T te_arg(T l3, T u, T m) {
     return RT<T>::pw(l3, m) * RT<T>::pw(u, m);
 }
 
-// Angular function g = 1 + c^2/d^2 - c^2/(d^2 + (h - cos)^2), written as
+// The angular function g = 1 + c^2/d^2 - c^2/(d^2 + (h - cos)^2), written as
 // 1 + c^2 (h - cos)^2 / (d^2 (d^2 + (h - cos)^2)): the same value without
 // the cancellation of two ~c^2/d^2 terms (c^2/d^2 ~ 4e7 for silicon), which
 // float32 cannot afford.
 template <typename T>
-__device__ __forceinline__ T te_g(T c, T d, T hc) {
-    T d2 = d * d, hc2 = hc * hc;
-    return T(1) + (c * c) * hc2 / (d2 * (d2 + hc2));
+__device__ __forceinline__ T te_g(T c2, T d2, T hc) {
+    const T hc2 = hc * hc;
+    return T(1) + c2 * hc2 / (d2 * (d2 + hc2));
 }
 
-// Analytic gradient of one zeta term (engine/tersoff.py:161-202).
+// g and dg/dcos from one reciprocal.
 template <typename T>
-__device__ __forceinline__ void te_zgrad(T rijx, T rijy, T rijz, T r_ij, T rikx, T riky, T rikz, T r_ik,
-                                         T fc_ik, T dfc_ik, T c, T d, T h, T l3, T m, T gam, T dzj[3],
-                                         T dzk[3]) {
-    T inv_ij = T(1) / r_ij, inv_ik = T(1) / r_ik;
-    T cos_t = (rijx * rikx + rijy * riky + rijz * rikz) * inv_ij * inv_ik;
-    T hc = h - cos_t;
-    T q = d * d + hc * hc;
-    T g = te_g<T>(c, d, hc);
-    T dg = T(-2) * c * c * hc / (q * q);
-    T u = r_ij - r_ik;
-    T ex = clamped_exp<T>(te_arg<T>(l3, u, m));
-    T dex;
+__device__ __forceinline__ void te_gdg(T c2, T d2, T hc, T &g, T &dg) {
+    const T hc2 = hc * hc, w = T(1) / (d2 * (d2 + hc2)), q = d2 * w;
+    g = T(1) + c2 * hc2 * w;
+    dg = T(-2) * c2 * hc * (q * q);
+}
+
+// An (i, j, k) record as the angle loops read it.
+template <typename T>
+struct TeTri {
+    T c2, d2, h, gam, l3, m, valid, pad;
+};
+
+template <typename T>
+__device__ __forceinline__ TeTri<T> te_tri_row(const double *__restrict__ t) {
+    TeTri<T> q;
+    const T c = (T)__ldg(t + 1), d = (T)__ldg(t + 2);
+    q.c2 = c * c;
+    q.d2 = d * d;
+    q.h = (T)__ldg(t + 3);
+    q.gam = (T)__ldg(t + 6);
+    q.l3 = (T)__ldg(t + 4);
+    q.m = (T)__ldg(t + 5);
+    q.valid = __ldg(t) != 0.0 ? T(1) : T(0);
+    q.pad = T(0);
+    return q;
+}
+
+// The tables of up to TE_SH species in shared memory: the pair rows, the
+// squared reach of every pair, the triplet records in T, and per centre
+// species whether its records are all the same, valid and without lambda3
+// (one element, or the Tersoff-1989 mixing rules): then one record serves
+// every angle of the centre.
+constexpr int TE_SH = 4;
+template <typename T>
+struct TeTab {
+    double tb[TE_SH * TE_SH * 10];
+    double reach2[TE_SH * TE_SH];
+    TeTri<T> tri[TE_SH * TE_SH * TE_SH];
+    int plain[TE_SH];
+};
+
+// The square of the largest r at which the pair (a, b) takes part in any
+// term, from either atom (negative: none): a leg beyond it contributes
+// nothing to its centre or to its neighbour's terms, and both atoms of the
+// pair agree on it.
+__device__ __forceinline__ double te_reach2(const TeDev &P, int a, int b) {
+    const double *t = P.tb + 10 * (a * P.ns + b), *u = P.tb + 10 * (b * P.ns + a);
+    const double x = __ldg(t) != 0.0 ? __ldg(t + 5) + __ldg(t + 6) : -1.0;
+    const double y = __ldg(u) != 0.0 ? __ldg(u + 5) + __ldg(u + 6) : -1.0;
+    const double r = x > y ? x : y;
+    return r > 0.0 ? r * r : -1.0;
+}
+
+template <typename T>
+__device__ __forceinline__ void te_load_tab(const TeDev &P, TeTab<T> &B) {
+    const int ns = P.ns;
+    if (ns > TE_SH) return;
+    for (int q = threadIdx.x; q < 10 * ns * ns; q += blockDim.x) B.tb[q] = P.tb[q];
+    for (int q = threadIdx.x; q < ns * ns; q += blockDim.x) B.reach2[q] = te_reach2(P, q / ns, q % ns);
+    for (int q = threadIdx.x; q < ns * ns * ns; q += blockDim.x) B.tri[q] = te_tri_row<T>(P.tri + 8 * q);
+    __syncthreads();
+    for (int a = threadIdx.x; a < ns; a += blockDim.x) {
+        const TeTri<T> *t = B.tri + a * ns * ns;
+        bool same = t[0].valid != T(0) && t[0].l3 == T(0) && (t[0].m == T(3) || t[0].m == T(1));
+        for (int q = 1; q < ns * ns; ++q)
+            same = same && t[q].valid != T(0) && t[q].l3 == T(0) && (t[q].m == T(3) || t[q].m == T(1)) &&
+                   t[q].c2 == t[0].c2 && t[q].d2 == t[0].d2 && t[q].h == t[0].h && t[q].gam == t[0].gam;
+        B.plain[a] = same ? 1 : 0;
+    }
+    __syncthreads();
+}
+
+// r in float64 (the two-body part is float64 in both precisions): a column
+// of its own beside float32 rows only.
+template <typename T, int MAXN> struct TeDist { double rd[MAXN]; };
+template <int MAXN> struct TeDist<double, MAXN> {};
+
+// One centre's legs (neighbours inside their pair's cutoff) in shared
+// memory, compacted in slot order: displacement, length and its inverse, the
+// cutoff function of the leg as a zeta term's third atom (record (i, k)) and
+// its derivative, the bond's zeta-gradient coefficient and pair part.
+// Groups of a warp lie 32 bytes apart modulo the banks' 128, so the lanes'
+// broadcast reads of different groups do not meet in a bank.
+template <typename T, int MAXN>
+struct TeRow {
+    T x[MAXN], y[MAXN], z[MAXN], r[MAXN], ir[MAXN], fk[MAXN], dfk[MAXN], coef[MAXN];
+    TeDist<T, MAXN> dist;
+    double cx[MAXN];  // r^2 while staging
+    int rev[MAXN];    // the leg's reverse slot
+    int meta[MAXN];   // slot in the row | (i < j) << 8 | species << 9
+    char pad[32];
+};
+
+template <int MAXN> __device__ __forceinline__ void te_put_r(TeRow<double, MAXN> &R, int q, double r) { R.r[q] = r; }
+template <int MAXN> __device__ __forceinline__ double te_get_r(const TeRow<double, MAXN> &R, int q) { return R.r[q]; }
+template <int MAXN> __device__ __forceinline__ void te_put_r(TeRow<float, MAXN> &R, int q, double r) {
+    R.r[q] = (float)r;
+    R.dist.rd[q] = r;
+}
+template <int MAXN> __device__ __forceinline__ double te_get_r(const TeRow<float, MAXN> &R, int q) { return R.dist.rd[q]; }
+
+// The (l3 u)^m exponential of a zeta term and its derivative in u; 1 and 0
+// without lambda3.
+template <typename T>
+__device__ __forceinline__ void te_expo(T l3, T m, T u, T &ex, T &dex) {
+    ex = T(1);
+    dex = T(0);
+    if (l3 == T(0) && (m == T(3) || m == T(1))) return;
+    ex = clamped_exp<T>(te_arg<T>(l3, u, m));
     if (m == T(3)) dex = ex * T(3) * (l3 * l3 * l3) * (u * u);
     else if (m == T(1)) dex = ex * l3;
     else dex = ex * m * RT<T>::pw(l3, m) * RT<T>::pw(u, m - T(1));
-    T a_j = gam * fc_ik * dg * ex;
-    T b_j = gam * fc_ik * g * dex * inv_ij;
-    T b_k = gam * (dfc_ik * g * ex - fc_ik * g * dex) * inv_ik;
-    T ii_k = inv_ij * inv_ik;
-    T cj = cos_t * inv_ij * inv_ij;
-    T ck = cos_t * inv_ik * inv_ik;
-    dzj[0] = a_j * (rikx * ii_k - cj * rijx) + b_j * rijx;
-    dzj[1] = a_j * (riky * ii_k - cj * rijy) + b_j * rijy;
-    dzj[2] = a_j * (rikz * ii_k - cj * rijz) + b_j * rijz;
-    dzk[0] = a_j * (rijx * ii_k - ck * rikx) + b_k * rikx;
-    dzk[1] = a_j * (rijy * ii_k - ck * riky) + b_k * riky;
-    dzk[2] = a_j * (rijz * ii_k - ck * rikz) + b_k * rikz;
 }
 
-// Shared-memory row staging of one lane group.
-template <typename T, int MAXN>
-struct TeRow {
-    T x[MAXN], y[MAXN], z[MAXN], r[MAXN], coef[MAXN];
-    int sp[MAXN];
-    int ok[MAXN];
-};
-
+// Every term of a centre.  A group of LPA lanes takes one centre; in the
+// angle loops four legs at a time, each by LPA / 4 lanes that share the loop
+// over the third atom.  The bound is instruction issue and latency, not
+// memory (32,768-atom SiC, float64: 0.6 % of DRAM bandwidth), so the work is
+// cut to what the terms need: legs beyond their own pair's cutoff are dropped
+// before any loop, the cutoff functions are evaluated once per leg and not
+// per angle, one angle gives zeta_j's term k and zeta_k's term j one common
+// geometry, and g and g' take one reciprocal.  With the gather: 80 us (SiC
+// above), against 415 us for a zeta and a force kernel of a lane per bond
+// that evaluated the cutoff functions per angle, each gradient from both of
+// its bonds, and a bond order for the partner atom to read.
 template <typename T, int MAXN, int LPA>
-__device__ __forceinline__ void te_stage(const SysView &S, const int *__restrict__ nbr, int i, int beg,
-                                         int n, double rc, TeRow<T, MAXN> &R, int sub) {
-    const double *cell = cell_of(S, i);
-    double xi = S.pos[3 * (size_t)i], yi = S.pos[3 * (size_t)i + 1], zi = S.pos[3 * (size_t)i + 2];
-    for (int s = sub; s < n; s += LPA) {
-        int j = nbr[beg + s];
-        double dx, dy, dz;
-        mic_exact(cell, S.pos[3 * (size_t)j] - xi, S.pos[3 * (size_t)j + 1] - yi,
-                  S.pos[3 * (size_t)j + 2] - zi, dx, dy, dz);
-        double r = sqrt(dx * dx + dy * dy + dz * dz);
-        R.x[s] = (T)dx;
-        R.y[s] = (T)dy;
-        R.z[s] = (T)dz;
-        R.r[s] = (T)r;
-        R.sp[s] = S.types[j];
-        R.ok[s] = (r < rc && r > 1e-12) ? 1 : 0;
-    }
-}
-
-template <typename T, int MAXN, int LPA>
-__global__ void te_zeta(SysView S, const int *__restrict__ row_off, const int *__restrict__ nbr, TeDev P,
-                        double *__restrict__ slot_b, int *__restrict__ err) {
+__global__ void __launch_bounds__(TeGeom<MAXN, LPA>::BLOCK, TeGeom<MAXN, LPA>::min_blocks(sizeof(T)))
+    te_center(SysView S, const int *__restrict__ row_off, const int *__restrict__ nbr, const int *__restrict__ rev,
+              TeDev P, double *__restrict__ slot_G, double *__restrict__ f_local, double *__restrict__ per_atom,
+              unsigned *__restrict__ live_mask, ClearWords clr, SiteOut so) {
     constexpr int GPB = TeGeom<MAXN, LPA>::GPB;
+    constexpr int NB = 4, KS = LPA / NB;
+    static_assert(LPA >= NB && LPA < 32, "te_center: 4 to 16 lanes per centre");
     __shared__ TeRow<T, MAXN> rows[GPB];
-    const int sub = threadIdx.x & (LPA - 1);
+    __shared__ TeTab<T> B;
+    clr.run();
+    te_load_tab<T>(P, B);
+    const int sub = threadIdx.x & (LPA - 1), gl = threadIdx.x & 31 & ~(LPA - 1);
+    const unsigned gones = (1u << LPA) - 1u, gmask = gones << gl;
+    const int lt = sub & (NB - 1), ks = sub / NB;
     TeRow<T, MAXN> &R = rows[threadIdx.x / LPA];
     const int ns = P.ns;
-    for (int base = blockIdx.x * GPB; base < S.n_atoms; base += gridDim.x * GPB) {
-        int i = base + threadIdx.x / LPA;
-        int beg = 0, n = 0;
-        bool live = i < S.n_atoms;
-        if (live) {
-            beg = row_off[i];
-            n = row_off[i + 1] - beg;
-            if (n > MAXN) {
-                if (sub == 0) atomicOr(err, MBF_DEV_ROW_TOO_LONG);
-                live = false;
-            }
-        }
-        if (live) te_stage<T, MAXN, LPA>(S, nbr, i, beg, n, P.rc, R, sub);
-        __syncwarp();
-        if (live) {
-            int si = S.types[i];
-            for (int s = sub; s < n; s += LPA) {
-                double b = 1.0, db = 0.0;
-                if (R.ok[s]) {
-                    int j = nbr[beg + s];
-                    int sj = R.sp[s];
-                    int lo = i < j ? si : sj, hi = i < j ? sj : si;
-                    if (P.tb[10 * (lo * ns + hi)] != 0.0) {
-                        T zeta = T(0);
-                        T rs = R.r[s];
-                        for (int k = 0; k < n; ++k) {
-                            if (k == s || !R.ok[k]) continue;
-                            int sk = R.sp[k];
-                            const double *tk = P.tb + 10 * (si * ns + sk);
-                            const double *t3 = P.tri + 8 * ((si * ns + sj) * ns + sk);
-                            if (tk[0] == 0.0 || t3[0] == 0.0) continue;
-                            T fc = te_fc<T>(R.r[k], (T)tk[5], (T)tk[6]);
-                            if (fc == T(0)) continue;
-                            T cos_t = (R.x[s] * R.x[k] + R.y[s] * R.y[k] + R.z[s] * R.z[k]) / (rs * R.r[k]);
-                            T c = (T)t3[1], d = (T)t3[2], h = (T)t3[3];
-                            T hc = h - cos_t;
-                            T g = te_g<T>(c, d, hc);
-                            zeta += (T)t3[6] * fc * g * clamped_exp<T>(te_arg<T>((T)t3[4], rs - R.r[k], (T)t3[5]));
-                        }
-                        const double *tij = P.tb + 10 * (si * ns + sj);
-                        double beta = tij[7], nn = tij[8];
-                        double z = (double)zeta;
-                        if (z > 0.0 && beta != 0.0) {
-                            double bz = pow(beta * z, nn);
-                            b = pow(1.0 + bz, -0.5 / nn);
-                            db = -0.5 * b * bz / (z * (1.0 + bz));
-                        }
-                    }
-                }
-                slot_b[2 * (size_t)(beg + s)] = b;
-                slot_b[2 * (size_t)(beg + s) + 1] = db;
-            }
-        }
-        __syncwarp();
+    const bool small = ns <= TE_SH;
+    const double *const tb = small ? B.tb : P.tb;
+    auto tri_row = [&](int q) { return small ? B.tri[q] : te_tri_row<T>(P.tri + 8 * (size_t)q); };
+    const int i = blockIdx.x * GPB + threadIdx.x / LPA;
+    double fx = 0, fy = 0, fz = 0, e = 0;
+    double v[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+    int nl = 0, nok = 0, beg = 0, n = 0, si = 0;
+    if (i < S.n_atoms) {
+        beg = row_off[i];
+        n = row_off[i + 1] - beg;
+        if (n > MAXN) n = 0;  // reported by the gather, which sees every row
+        si = S.types[i];
     }
-}
-
-template <typename T, int MAXN, int LPA>
-__global__ void te_force(SysView S, const int *__restrict__ row_off, const int *__restrict__ nbr,
-                         const int *__restrict__ rev, TeDev P, const double *__restrict__ slot_b,
-                         double *__restrict__ slot_G, double *__restrict__ f_local,
-                         double *__restrict__ per_atom, int *__restrict__ err, SiteOut so) {
-    constexpr int GPB = TeGeom<MAXN, LPA>::GPB;
-    __shared__ TeRow<T, MAXN> rows[GPB];
-    const int sub = threadIdx.x & (LPA - 1);
-    TeRow<T, MAXN> &R = rows[threadIdx.x / LPA];
-    const int ns = P.ns;
-    for (int base = blockIdx.x * GPB; base < S.n_atoms; base += gridDim.x * GPB) {
-        int i = base + threadIdx.x / LPA;
-        int beg = 0, n = 0;
-        bool live = i < S.n_atoms;
-        if (live) {
-            beg = row_off[i];
-            n = row_off[i + 1] - beg;
-            if (n > MAXN) {
-                if (sub == 0) atomicOr(err, MBF_DEV_ROW_TOO_LONG);
-                live = false;
-            }
-        }
-        if (live) te_stage<T, MAXN, LPA>(S, nbr, i, beg, n, P.rc, R, sub);
-        __syncwarp();
-        double fx = 0, fy = 0, fz = 0, e = 0, npair = 0, e_site = 0;
-        double v[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-        int si = live ? S.types[i] : 0;
-        // pass 1: pair terms and the zeta-gradient coefficients
-        double cxs[(MAXN + LPA - 1) / LPA];
-        double cxs_site[(MAXN + LPA - 1) / LPA];  // site split: own bond order (engine/site_terms.py:312-437)
-        double pair_r[(MAXN + LPA - 1) / LPA];
-        if (live) {
-            const double *cell = cell_of(S, i);
-            double xi = S.pos[3 * (size_t)i], yi = S.pos[3 * (size_t)i + 1], zi = S.pos[3 * (size_t)i + 2];
-            int q = 0;
-            for (int s = sub; s < n; s += LPA, ++q) {
-                {
-                    int j = nbr[beg + s];
-                    double dx, dy, dz;
-                    mic_exact(cell, S.pos[3 * (size_t)j] - xi, S.pos[3 * (size_t)j + 1] - yi,
-                              S.pos[3 * (size_t)j + 2] - zi, dx, dy, dz);
-                    pair_r[q] = sqrt(dx * dx + dy * dy + dz * dz);
-                }
-                T coef = T(0);
-                double cx = 0.0, cx_site = 0.0;
-                if (R.ok[s]) {
-                    int j = nbr[beg + s];
-                    int sj = R.sp[s];
-                    int lo = i < j ? si : sj, hi = i < j ? sj : si;
-                    const double *tp = P.tb + 10 * (lo * ns + hi);
-                    if (tp[0] != 0.0) {
-                        double b_own = slot_b[2 * (size_t)(beg + s)];
-                        double db_own = slot_b[2 * (size_t)(beg + s) + 1];
-                        double b_rev = slot_b[2 * (size_t)rev[beg + s]];
-                        double bavg = i < j ? 0.5 * (b_own + b_rev) : 0.5 * (b_rev + b_own);
-                        // the two-body part is per bond, not per angle: float64
-                        // in both precisions
-                        double r = pair_r[q];
-                        double Rr = tp[5], Dd = tp[6];
-                        double fc = te_fc<double>(r, Rr, Dd), dfc = te_dfc<double>(r, Rr, Dd);
-                        if (fc != 0.0 || dfc != 0.0) {
-                            double l1 = tp[3], l2 = tp[4];
-                            double fr = tp[1] * clamped_exp<double>(-l1 * r);
-                            double fa = -tp[2] * clamped_exp<double>(-l2 * r);
-                            e += 0.5 * (fc * (fr + bavg * fa));
-                            double dEdr = dfc * (fr + bavg * fa) + fc * (-l1 * fr + bavg * (-l2 * fa));
-                            cx = dEdr / r;
-                            if (so.dudv) {
-                                e_site += 0.5 * (fc * (fr + b_own * fa));
-                                cx_site = 0.5 * (dfc * (fr + b_own * fa) + fc * (-l1 * fr - l2 * b_own * fa)) / r;
-                            }
-                            if (fabs(db_own) > 1e-30) coef = (T)(0.5 * fc * fa * db_own);
-                        }
-                    }
-                }
-                R.coef[s] = coef;
-                cxs[q] = cx;
-                cxs_site[q] = cx_site;
-            }
-        }
-        __syncwarp();
-        // pass 2: three-body forces per slot
-        if (live) {
-            int q = 0;
-            for (int s = sub; s < n; s += LPA, ++q) {
-                double Gx = 0, Gy = 0, Gz = 0;
-                double dx = (double)R.x[s], dy = (double)R.y[s], dz = (double)R.z[s];
-                if (R.ok[s]) {
-                    int sx_ = R.sp[s];
-                    T dzj[3], dzk[3];
-                    // slot s as the bond partner j of zeta_{i s}
-                    T cs = R.coef[s];
-                    if (cs != T(0)) {
-                        for (int k = 0; k < n; ++k) {
-                            if (k == s || !R.ok[k]) continue;
-                            int sk = R.sp[k];
-                            const double *tk = P.tb + 10 * (si * ns + sk);
-                            const double *t3 = P.tri + 8 * ((si * ns + sx_) * ns + sk);
-                            if (tk[0] == 0.0 || t3[0] == 0.0) continue;
-                            T Rk = (T)tk[5], Dk = (T)tk[6];
-                            T fck = te_fc<T>(R.r[k], Rk, Dk);
-                            if (fck == T(0)) continue;
-                            te_zgrad<T>(R.x[s], R.y[s], R.z[s], R.r[s], R.x[k], R.y[k], R.z[k], R.r[k], fck,
-                                        te_dfc<T>(R.r[k], Rk, Dk), (T)t3[1], (T)t3[2], (T)t3[3], (T)t3[4],
-                                        (T)t3[5], (T)t3[6], dzj, dzk);
-                            Gx -= (double)(cs * dzj[0]);
-                            Gy -= (double)(cs * dzj[1]);
-                            Gz -= (double)(cs * dzj[2]);
-                        }
-                    }
-                    // slot s as the third atom k of zeta_{i j}
-                    const double *ts = P.tb + 10 * (si * ns + sx_);
-                    if (ts[0] != 0.0) {
-                        T Rs = (T)ts[5], Ds = (T)ts[6];
-                        T fcs = te_fc<T>(R.r[s], Rs, Ds);
-                        if (fcs != T(0)) {
-                            T dfcs = te_dfc<T>(R.r[s], Rs, Ds);
-                            for (int jj = 0; jj < n; ++jj) {
-                                if (jj == s || !R.ok[jj]) continue;
-                                T cj = R.coef[jj];
-                                if (cj == T(0)) continue;
-                                const double *t3 = P.tri + 8 * ((si * ns + R.sp[jj]) * ns + sx_);
-                                if (t3[0] == 0.0) continue;
-                                te_zgrad<T>(R.x[jj], R.y[jj], R.z[jj], R.r[jj], R.x[s], R.y[s], R.z[s], R.r[s],
-                                            fcs, dfcs, (T)t3[1], (T)t3[2], (T)t3[3], (T)t3[4], (T)t3[5],
-                                            (T)t3[6], dzj, dzk);
-                                Gx -= (double)(cj * dzk[0]);
-                                Gy -= (double)(cj * dzk[1]);
-                                Gz -= (double)(cj * dzk[2]);
-                            }
-                        }
-                    }
-                }
-                double cx = cxs[q];
-                fx += cx * dx - Gx;
-                fy += cx * dy - Gy;
-                fz += cx * dz - Gz;
-                double hx = 0.5 * cx * dx, hy = 0.5 * cx * dy, hz = 0.5 * cx * dz;
-                v[0] += -hx * dx + Gx * dx;
-                v[1] += -hx * dy + Gx * dy;
-                v[2] += -hx * dz + Gx * dz;
-                v[3] += -hy * dx + Gy * dx;
-                v[4] += -hy * dy + Gy * dy;
-                v[5] += -hy * dz + Gy * dz;
-                v[6] += -hz * dx + Gz * dx;
-                v[7] += -hz * dy + Gz * dy;
-                v[8] += -hz * dz + Gz * dz;
-                npair += R.ok[s] ? 1.0 : 0.0;
-                if (so.dudv) {
-                    size_t os = 3 * (size_t)(beg + s);
-                    double cs_ = cxs_site[q];
-                    so.dudv[os] = cs_ * dx - Gx;
-                    so.dudv[os + 1] = cs_ * dy - Gy;
-                    so.dudv[os + 2] = cs_ * dz - Gz;
+    // the legs, compacted in slot order; every loop has the same trip count
+    // over a group
+    if (n > 0) {
+        const double *cell = cell_of(S, i);
+        const double xi = S.pos[3 * (size_t)i], yi = S.pos[3 * (size_t)i + 1], zi = S.pos[3 * (size_t)i + 2];
+        const double rc2 = P.rc * P.rc;
+        unsigned word = 0;
+        for (int s0 = 0; s0 < n; s0 += LPA) {
+            const int s = s0 + sub;
+            bool ok = false, lv = false;
+            int j = 0, sj = 0, rs = 0;
+            double dx = 0, dy = 0, dz = 0, r2 = 0;
+            if (s < n) {
+                j = nbr[beg + s];
+                rs = rev[beg + s];
+                sj = S.types[j];
+                mic_exact(cell, S.pos[3 * (size_t)j] - xi, S.pos[3 * (size_t)j + 1] - yi, S.pos[3 * (size_t)j + 2] - zi,
+                          dx, dy, dz);
+                r2 = dx * dx + dy * dy + dz * dz;
+                ok = r2 < rc2 && r2 > 1e-24;
+                lv = ok && r2 <= (small ? B.reach2[si * ns + sj] : te_reach2(P, si, sj));
+                if (so.vec) {
+                    const size_t os = 3 * (size_t)(beg + s);
                     so.vec[os] = dx;
                     so.vec[os + 1] = dy;
                     so.vec[os + 2] = dz;
                 }
-                // the force on neighbour x goes to x's own slot (x -> i)
-                size_t o = 3 * (size_t)rev[beg + s];
-                slot_G[o] = Gx;
-                slot_G[o + 1] = Gy;
-                slot_G[o + 2] = Gz;
+            }
+            const unsigned b = (__ballot_sync(gmask, lv) >> gl) & gones;
+            nok += __popc((__ballot_sync(gmask, ok) >> gl) & gones);
+            if (lv) {
+                const int q = nl + __popc(b & ((1u << sub) - 1u));
+                R.x[q] = (T)dx;
+                R.y[q] = (T)dy;
+                R.z[q] = (T)dz;
+                R.cx[q] = r2;
+                R.rev[q] = rs;
+                R.meta[q] = s | (i < j ? 1 << 8 : 0) | sj << 9;
+            }
+            nl += __popc(b);
+            word |= b << (s0 & 31);
+            if (((s0 + LPA) & 31) == 0 || s0 + LPA >= n) {
+                if (sub == 0) live_mask[4 * (size_t)i + (s0 >> 5)] = word;
+                word = 0;
             }
         }
-        fx = group_sum<LPA>(fx);
-        fy = group_sum<LPA>(fy);
-        fz = group_sum<LPA>(fz);
-        e = group_sum<LPA>(e);
-        npair = group_sum<LPA>(npair);
-        e_site = group_sum<LPA>(e_site);
-#pragma unroll
-        for (int q = 0; q < 9; ++q) v[q] = group_sum<LPA>(v[q]);
-        if (sub == 0 && i < S.n_atoms && so.e) so.e[i] = e_site;
-        if (sub == 0 && i < S.n_atoms) {
-            f_local[3 * (size_t)i] = fx;
-            f_local[3 * (size_t)i + 1] = fy;
-            f_local[3 * (size_t)i + 2] = fz;
-            double *pa = per_atom + (size_t)i * ATOM_ACC;
-            pa[0] = e;
-#pragma unroll
-            for (int q = 0; q < 9; ++q) pa[1 + q] = v[q];
-            pa[10] = npair;
+    }
+    __syncwarp(gmask);
+    for (int q = sub; q < nl; q += LPA) {
+        const double r = sqrt(R.cx[q]);
+        const double *tk = tb + 10 * (si * ns + (R.meta[q] >> 9));
+        T fk = T(0), dfk = T(0);
+        if (tk[0] != 0.0) te_cut<T>((T)r, (T)tk[5], (T)tk[6], fk, dfk);
+        te_put_r(R, q, r);
+        R.ir[q] = T(1) / (T)r;
+        R.fk[q] = fk;
+        R.dfk[q] = dfk;
+    }
+    __syncwarp(gmask);
+    const bool plain = small && B.plain[si];
+    const TeTri<T> own = plain ? B.tri[si * ns * ns] : TeTri<T>();
+    // zeta of every bond
+    for (int t0 = 0; t0 < nl; t0 += NB) {
+        const int t = t0 + lt;
+        T zeta = T(0);
+        if (t < nl) {
+            const T xs = R.x[t], ys = R.y[t], zs = R.z[t], irs = R.ir[t];
+            if (plain) {
+                for (int k = ks; k < nl; k += KS) {
+                    const T fk = R.fk[k];
+                    if (k == t || fk == T(0)) continue;
+                    const T cs = (xs * R.x[k] + ys * R.y[k] + zs * R.z[k]) * (irs * R.ir[k]);
+                    zeta += own.gam * fk * te_g<T>(own.c2, own.d2, own.h - cs);
+                }
+            } else {
+                const T rs = R.r[t];
+                const int row = (si * ns + (R.meta[t] >> 9)) * ns;
+                for (int k = ks; k < nl; k += KS) {
+                    const T fk = R.fk[k];
+                    if (k == t || fk == T(0)) continue;
+                    const TeTri<T> q = tri_row(row + (R.meta[k] >> 9));
+                    if (q.valid == T(0)) continue;
+                    const T cs = (xs * R.x[k] + ys * R.y[k] + zs * R.z[k]) * (irs * R.ir[k]);
+                    T ex, dex;
+                    te_expo<T>(q.l3, q.m, rs - R.r[k], ex, dex);
+                    zeta += q.gam * fk * te_g<T>(q.c2, q.d2, q.h - cs) * ex;
+                }
+            }
         }
-        __syncwarp();
+#pragma unroll
+        for (int o = NB; o < LPA; o <<= 1) zeta += __shfl_xor_sync(gmask, zeta, o, LPA);
+        if (t < nl && ks == 0) R.coef[t] = zeta;
+    }
+    __syncwarp(gmask);
+    // the bonds, one lane each: bond order, energy, pair part and the
+    // coefficient of zeta's gradient; the two-body part is per bond, not per
+    // angle, and float64 in both precisions
+    for (int t = sub; t < nl; t += LPA) {
+        const int mt = R.meta[t], sj = mt >> 9;
+        const double *tij = tb + 10 * (si * ns + sj);
+        const double *tp = mt & 256 ? tij : tb + 10 * (sj * ns + si);
+        const double z = (double)R.coef[t];
+        T coef = T(0);
+        double cx = 0.0;
+        if (tp[0] != 0.0) {
+            const double r = te_get_r(R, t);
+            double fc, dfc;
+            te_cut<double>(r, tp[5], tp[6], fc, dfc);
+            if (fc != 0.0 || dfc != 0.0) {
+                // b = (1 + (beta zeta)^n)^(-1 / (2 n)) by logarithms (beta
+                // zeta > 0): half the cost of two pow()
+                const double beta = tij[7], nn = tij[8];
+                double b = 1.0, db = 0.0;
+                if (z > 0.0 && beta != 0.0) {
+                    double bz;
+                    if (beta > 0.0) {
+                        bz = exp(nn * log(beta * z));
+                        b = exp(-0.5 / nn * log(1.0 + bz));
+                    } else {
+                        bz = pow(beta * z, nn);
+                        b = pow(1.0 + bz, -0.5 / nn);
+                    }
+                    db = -0.5 * b * bz / (z * (1.0 + bz));
+                }
+                const double l1 = tp[3], l2 = tp[4];
+                const double fr = tp[1] * clamped_exp<double>(-l1 * r);
+                const double fa = -tp[2] * clamped_exp<double>(-l2 * r);
+                e += 0.5 * (fc * (fr + b * fa));
+                cx = 0.5 * (dfc * (fr + b * fa) + fc * (-l1 * fr - l2 * b * fa)) / r;
+                if (fabs(db) > 1e-30) coef = (T)(0.5 * fc * fa * db);
+            }
+        }
+        R.coef[t] = coef;
+        R.cx[t] = cx;
+    }
+    __syncwarp(gmask);
+    // dU_i / dr of every leg: t as the bond partner of zeta_t's terms and as
+    // the third atom of the other bonds' terms.  With c = cos(t, k), both
+    // parts point along d_k and d_t:
+    //   d = A (d_k / (r_t r_k) - c d_t / r_t^2) + B d_t
+    for (int t0 = 0; t0 < nl; t0 += NB) {
+        const int t = t0 + lt;
+        const bool act = t < nl;
+        double gx = 0, gy = 0, gz = 0, gs = 0;
+        T xs = T(0), ys = T(0), zs = T(0);
+        if (act) {
+            xs = R.x[t];
+            ys = R.y[t];
+            zs = R.z[t];
+            const T irs = R.ir[t], ct = R.coef[t], ft = R.fk[t], dft = R.dfk[t], ir2 = irs * irs;
+            auto add = [&](T A, T B_, T c, T ii, T xk, T yk, T zk) {
+                const T Ai = A * ii;
+                gx += (double)(Ai * xk);
+                gy += (double)(Ai * yk);
+                gz += (double)(Ai * zk);
+                gs += (double)(B_ - A * c * ir2);
+            };
+            if (plain) {
+                for (int k = ks; k < nl; k += KS) {
+                    const T ck = R.coef[k], w = ct * R.fk[k] + ck * ft;
+                    if (k == t || (w == T(0) && ck == T(0))) continue;
+                    const T xk = R.x[k], yk = R.y[k], zk = R.z[k], ii = irs * R.ir[k];
+                    const T c = (xs * xk + ys * yk + zs * zk) * ii;
+                    T g, dg;
+                    te_gdg<T>(own.c2, own.d2, own.h - c, g, dg);
+                    add(own.gam * w * dg, own.gam * ck * dft * g * irs, c, ii, xk, yk, zk);
+                }
+            } else {
+                const T rs = R.r[t];
+                const int st = R.meta[t] >> 9;
+                for (int k = ks; k < nl; k += KS) {
+                    const T fk = R.fk[k], ck = R.coef[k];
+                    const bool as_j = ct != T(0) && fk != T(0), as_k = ck != T(0) && ft != T(0);
+                    if (k == t || !(as_j || as_k)) continue;
+                    const int sk = R.meta[k] >> 9;
+                    const T xk = R.x[k], yk = R.y[k], zk = R.z[k], ii = irs * R.ir[k];
+                    const T c = (xs * xk + ys * yk + zs * zk) * ii;
+                    T A = T(0), B_ = T(0), g, dg, ex, dex;
+                    if (as_j) {
+                        const TeTri<T> q = tri_row((si * ns + st) * ns + sk);
+                        if (q.valid != T(0)) {
+                            te_gdg<T>(q.c2, q.d2, q.h - c, g, dg);
+                            te_expo<T>(q.l3, q.m, rs - R.r[k], ex, dex);
+                            const T w = ct * q.gam * fk;
+                            A += w * dg * ex;
+                            B_ += w * g * dex * irs;
+                        }
+                    }
+                    if (as_k) {
+                        const TeTri<T> q = tri_row((si * ns + sk) * ns + st);
+                        if (q.valid != T(0)) {
+                            te_gdg<T>(q.c2, q.d2, q.h - c, g, dg);
+                            te_expo<T>(q.l3, q.m, R.r[k] - rs, ex, dex);
+                            const T w = ck * q.gam;
+                            A += w * ft * dg * ex;
+                            B_ += w * g * (dft * ex - ft * dex) * irs;
+                        }
+                    }
+                    add(A, B_, c, ii, xk, yk, zk);
+                }
+            }
+        }
+#pragma unroll
+        for (int o = NB; o < LPA; o <<= 1) {
+            gx += __shfl_xor_sync(gmask, gx, o, LPA);
+            gy += __shfl_xor_sync(gmask, gy, o, LPA);
+            gz += __shfl_xor_sync(gmask, gz, o, LPA);
+            gs += __shfl_xor_sync(gmask, gs, o, LPA);
+        }
+        if (act && ks == 0) {
+            const double dx = (double)xs, dy = (double)ys, dz = (double)zs;
+            gs += R.cx[t];
+            const double Dx = gx + gs * dx, Dy = gy + gs * dy, Dz = gz + gs * dz;
+            fx += Dx;
+            fy += Dy;
+            fz += Dz;
+            v[0] -= Dx * dx;
+            v[1] -= Dx * dy;
+            v[2] -= Dx * dz;
+            v[3] -= Dy * dx;
+            v[4] -= Dy * dy;
+            v[5] -= Dy * dz;
+            v[6] -= Dz * dx;
+            v[7] -= Dz * dy;
+            v[8] -= Dz * dz;
+            if (so.dudv) {  // engine/site_terms.py:312-437: own bond order
+                const size_t os = 3 * (size_t)(beg + (R.meta[t] & 255));
+                so.dudv[os] = Dx;
+                so.dudv[os + 1] = Dy;
+                so.dudv[os + 2] = Dz;
+            }
+            // the force on neighbour x goes to x's own slot (x -> i)
+            const size_t o = 3 * (size_t)R.rev[t];
+            slot_G[o] = -Dx;
+            slot_G[o + 1] = -Dy;
+            slot_G[o + 2] = -Dz;
+        }
+    }
+    __syncwarp();
+    // f and v: only the first lane of each leg holds sums
+    fx = group_sum<NB>(fx);
+    fy = group_sum<NB>(fy);
+    fz = group_sum<NB>(fz);
+    e = group_sum<LPA>(e);
+#pragma unroll
+    for (int q = 0; q < 9; ++q) v[q] = group_sum<NB>(v[q]);
+    if (sub == 0 && i < S.n_atoms) {
+        if (so.e) so.e[i] = e;
+        f_local[3 * (size_t)i] = fx;
+        f_local[3 * (size_t)i + 1] = fy;
+        f_local[3 * (size_t)i + 2] = fz;
+        double *pa = per_atom + (size_t)i * ATOM_ACC;
+        pa[0] = e;
+#pragma unroll
+        for (int q = 0; q < 9; ++q) pa[1 + q] = v[q];
+        pa[10] = (double)nok;
     }
 }
 
+// Everything one launch needs besides the shape.
+struct TeArgs {
+    SysView S;
+    const mbf_nlist *nl;
+    TeDev P;
+    double *slot_G, *f_local, *per_atom;
+    unsigned *live_mask;
+    ClearWords clr;
+    SiteOut so;
+};
+
 template <typename T, int MAXN, int LPA>
-static int te_launch(const SysView &S, const mbf_nlist *nl, const TeDev &P, double *slot_b, double *slot_G,
-                     double *f_local, double *per_atom, double *forces, int *err, const SiteOut &so,
-                     cudaStream_t st) {
+static int te_launch(const TeArgs &A, cudaStream_t st) {
     constexpr int GPB = TeGeom<MAXN, LPA>::GPB, BLOCK = TeGeom<MAXN, LPA>::BLOCK;
-    int blocks = (S.n_atoms + GPB - 1) / GPB;
-    int g = persistent_grid(blocks, BLOCK, (const void *)te_zeta<T, MAXN, LPA>);
-    PROF_BEGIN("te_zeta", st);
-    te_zeta<T, MAXN, LPA><<<g, BLOCK, 0, st>>>(S, nl->row_off, nl->nbr, P, slot_b, err);
-    PROF_END("te_zeta", st);
-    MBF_CHECK_LAUNCH();
-    g = persistent_grid(blocks, BLOCK, (const void *)te_force<T, MAXN, LPA>);
-    PROF_BEGIN("te_force", st);
-    te_force<T, MAXN, LPA><<<g, BLOCK, 0, st>>>(S, nl->row_off, nl->nbr, nl->rev, P, slot_b, slot_G, f_local,
-                                         per_atom, err, so);
-    PROF_END("te_force", st);
+    const int blocks = (A.S.n_atoms + GPB - 1) / GPB;
+    PROF_BEGIN("te_center", st);
+    te_center<T, MAXN, LPA><<<blocks, BLOCK, 0, st>>>(A.S, A.nl->row_off, A.nl->nbr, A.nl->rev, A.P, A.slot_G, A.f_local,
+                                                      A.per_atom, A.live_mask, A.clr, A.so);
+    PROF_END("te_center", st);
     MBF_CHECK_LAUNCH();
     return MBF_OK;   // the eval's gather_reduce adds the slot forces
 }
 
 template <typename T, int MAXN>
-static int te_lpa(int lpa, const SysView &S, const mbf_nlist *nl, const TeDev &P, double *slot_b,
-                  double *slot_G, double *f_local, double *per_atom, double *forces, int *err, const SiteOut &so,
-                  cudaStream_t st) {
+static int te_lpa(int lpa, const TeArgs &A, cudaStream_t st) {
     switch (lpa) {
-        case 4: return te_launch<T, MAXN, 4>(S, nl, P, slot_b, slot_G, f_local, per_atom, forces, err, so, st);
-        case 8: return te_launch<T, MAXN, 8>(S, nl, P, slot_b, slot_G, f_local, per_atom, forces, err, so, st);
-        case 16: return te_launch<T, MAXN, 16>(S, nl, P, slot_b, slot_G, f_local, per_atom, forces, err, so, st);
+        case 4: return te_launch<T, MAXN, 4>(A, st);
+        case 8: return te_launch<T, MAXN, 8>(A, st);
+        case 16: return te_launch<T, MAXN, 16>(A, st);
         default: return MBF_ERR_ARGUMENT;
     }
 }
 
 template <typename T>
-static int te_rows(int mr, int lpa, const SysView &S, const mbf_nlist *nl, const TeDev &P, double *slot_b,
-                   double *slot_G, double *f_local, double *per_atom, double *forces, int *err, const SiteOut &so,
-                   cudaStream_t st) {
-    if (mr <= 32) return te_lpa<T, 32>(lpa, S, nl, P, slot_b, slot_G, f_local, per_atom, forces, err, so, st);
-    if (mr <= 64) return te_lpa<T, 64>(lpa, S, nl, P, slot_b, slot_G, f_local, per_atom, forces, err, so, st);
-    return te_lpa<T, 128>(lpa, S, nl, P, slot_b, slot_G, f_local, per_atom, forces, err, so, st);
+static int te_rows(int mr, int lpa, const TeArgs &A, cudaStream_t st) {
+    if (mr <= 32) return te_lpa<T, 32>(lpa, A, st);
+    if (mr <= 64) return te_lpa<T, 64>(lpa, A, st);
+    return te_lpa<T, 128>(lpa, A, st);
 }
 
-static int te_dispatch(int precision, int mr, int lpa, const SysView &S, const mbf_nlist *nl, const TeDev &P,
-                       double *slot_b, double *slot_G, double *f_local, double *per_atom, double *forces,
-                       int *err, const SiteOut &so, cudaStream_t st) {
-    if (lpa <= 0) lpa = 8;
-    return precision == MBF_FP64
-               ? te_rows<double>(mr, lpa, S, nl, P, slot_b, slot_G, f_local, per_atom, forces, err, so, st)
-               : te_rows<float>(mr, lpa, S, nl, P, slot_b, slot_G, f_local, per_atom, forces, err, so, st);
-}
+// The longest row te_rows' choice for `mr` stages.
+static int te_row_limit(int mr) { return mr <= 32 ? 32 : (mr <= 64 ? 64 : 128); }
 
 }  // namespace mbf
 
@@ -441,24 +554,30 @@ static int tersoff_eval(const mbf_system *sys, const mbf_nlist *nl, const mbf_te
         return MBF_OK;
     }
     if (nl->max_row > 128) return MBF_ERR_ROW_TOO_LONG;
-    SysView S = make_view(sys);
-    TeDev P;
-    P.ns = tab->ns;
-    P.tb = tab->tb;
-    P.tri = tab->tri;
-    P.rc = tab->r_cut;
+    // the per-structure completion counters live in a region of n_chunks
+    // words; every structure owns at least one chunk
+    if (plan->n_chunks <= 0 || sys->n_struct <= 0 || plan->n_chunks < sys->n_struct) return MBF_ERR_ARGUMENT;
+    TeArgs A;
+    A.S = make_view(sys);
+    A.nl = nl;
+    A.P.ns = tab->ns;
+    A.P.tb = tab->tb;
+    A.P.tri = tab->tri;
+    A.P.rc = tab->r_cut;
+    A.slot_G = ws_at<double>(workspace, L.slot);
+    A.f_local = ws_at<double>(workspace, L.f_local);
+    A.per_atom = ws_at<double>(workspace, L.per_atom);
+    A.live_mask = ws_at<unsigned>(workspace, L.atom_aux);
+    unsigned *sdone = ws_at<unsigned>(workspace, L.sdone);
     int *err = ws_at<int>(workspace, L.err);
-    if (cudaMemsetAsync(err, 0, ERR_CLEAR_BYTES, st) != cudaSuccess) return MBF_ERR_CUDA;
-    double *per_atom = ws_at<double>(workspace, L.per_atom);
-    double *f_local = ws_at<double>(workspace, L.f_local);
-    double *slot_G = ws_at<double>(workspace, L.slot);
-    double *slot_b = ws_at<double>(workspace, L.slot_b);
-    double *partial = ws_at<double>(workspace, L.partial);
-    int rc = te_dispatch(precision, nl->max_row, lanes_per_atom, S, nl, P, slot_b, slot_G, f_local, per_atom,
-                         forces, err, so, st);
+    A.clr = {(unsigned *)err, ERR_CLEAR_BYTES / 4, sdone, sys->n_struct};
+    A.so = so;
+    const int lpa = lanes_per_atom > 0 ? lanes_per_atom : 8;
+    int rc = precision == MBF_FP64 ? te_rows<double>(nl->max_row, lpa, A, st) : te_rows<float>(nl->max_row, lpa, A, st);
     if (rc != MBF_OK) return rc;
-    return gather_reduce(sys->n_struct, sys->n_atoms, nl->row_off, slot_G, f_local, forces, per_atom, plan, partial,
-                         energy, virial, ws_at<unsigned>(workspace, L.sdone), st);
+    return gather_live(sys->n_struct, sys->n_atoms, nl->row_off, A.slot_G, A.live_mask, te_row_limit(nl->max_row), err,
+                       A.f_local, forces, A.per_atom, plan, ws_at<double>(workspace, L.partial), energy, virial, sdone,
+                       st);
 }
 
 extern "C" int mbf_tersoff_eval(const mbf_system *sys, const mbf_nlist *nl, const mbf_tersoff_tables *tab,

@@ -193,6 +193,96 @@ int gather_reduce(int n_struct, int n_atoms, const int *row_off, const double *G
     return MBF_OK;
 }
 
+// gather_reduce_rows over the slots whose live bit is set: a list radius of
+// cutoff + skin holds two to three times the slots that carry a force
+// (32,768-atom SiC: 15.5 listed, 4 live), and the others are neither
+// written nor read.  Up to four slots a lane are in flight at once.
+template <int NT>
+__global__ void __launch_bounds__(NT) gather_live_rows(const int *__restrict__ row_off, const double *__restrict__ G,
+                                                       const uint4 *__restrict__ live_mask, int row_limit,
+                                                       int *__restrict__ err, const double *__restrict__ f_local,
+                                                       double *__restrict__ forces, ChunkSums cs) {
+    constexpr int LPA = 8, NG = NT / LPA;
+    const int c = blockIdx.x;
+    const int s = cs.chunk[3 * c], a0 = cs.chunk[3 * c + 1], a1 = cs.chunk[3 * c + 2];
+    const int sub = threadIdx.x & (LPA - 1), grp = threadIdx.x / LPA;
+    double r0 = 0.0, r1 = 0.0;
+    int nb = 0, ne = 0;
+    if (a0 + grp < a1) {
+        nb = row_off[a0 + grp];
+        ne = row_off[a0 + grp + 1];
+    }
+    for (int base = a0; base < a1; base += NG) {  // uniform over the block
+        const int a = base + grp, beg = nb, n = ne - nb;
+        if (a + NG < a1) {
+            nb = row_off[a + NG];
+            ne = row_off[a + NG + 1];
+        }
+        double fx = 0, fy = 0, fz = 0, fl = 0;
+        if (a < a1) {
+            const uint4 m4 = live_mask[a];
+            const double *pa = cs.per_atom + (size_t)a * ATOM_ACC;
+            const double ra = pa[sub];
+            const double rb = sub < ATOM_ACC - LPA ? pa[LPA + sub] : 0.0;
+            if (sub < 3) fl = f_local[3 * (size_t)a + sub];
+            if (n > row_limit) {
+                if (sub == 0) atomicOr(err, MBF_DEV_ROW_TOO_LONG);
+            } else {
+                const unsigned m[4] = {m4.x, m4.y, m4.z, m4.w};
+#pragma unroll
+                for (int w = 0; w < 4; ++w) {
+                    if (32 * w >= n) break;
+                    double x[4], y[4], z[4];
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        x[k] = y[k] = z[k] = 0.0;
+                        if (m[w] >> (sub + LPA * k) & 1u) {
+                            const double *g = G + 3 * (size_t)(beg + 32 * w + sub + LPA * k);
+                            x[k] = __ldcs(g);
+                            y[k] = __ldcs(g + 1);
+                            z[k] = __ldcs(g + 2);
+                        }
+                    }
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        fx += x[k];
+                        fy += y[k];
+                        fz += z[k];
+                    }
+                }
+            }
+            r0 += ra;
+            r1 += rb;
+        }
+        fx = group_sum<LPA>(fx);
+        fy = group_sum<LPA>(fy);
+        fz = group_sum<LPA>(fz);
+        // lane k (k < 3) of the group writes component k
+        const double g = sub == 0 ? fx : (sub == 1 ? fy : fz);
+        if (sub < 3 && a < a1) forces[3 * (size_t)a + sub] = fl + g;
+    }
+    chunk_sums_finish<NT>(cs, c, s, r0, r1);
+}
+
+int gather_live(int n_struct, int n_atoms, const int *row_off, const double *G, const unsigned *live_mask, int row_limit,
+                int *err, const double *f_local, double *forces, const double *per_atom, const mbf_reduce_plan *plan,
+                double *partial, double *energy, double *virial, unsigned *sdone, cudaStream_t st) {
+    if (plan->n_chunks <= 0 || n_struct <= 0 || plan->n_chunks < n_struct || !sdone) return MBF_ERR_ARGUMENT;
+    ChunkSums cs = {plan->chunk, plan->chunk_first, per_atom, partial, energy, virial, sdone};
+    const uint4 *mask = reinterpret_cast<const uint4 *>(live_mask);
+    PROF_BEGIN("gather_reduce", st);
+    const int nt = chunk_block(n_atoms, plan->n_chunks);
+    if (nt == 128)
+        gather_live_rows<128><<<plan->n_chunks, 128, 0, st>>>(row_off, G, mask, row_limit, err, f_local, forces, cs);
+    else if (nt == 256)
+        gather_live_rows<256><<<plan->n_chunks, 256, 0, st>>>(row_off, G, mask, row_limit, err, f_local, forces, cs);
+    else
+        gather_live_rows<512><<<plan->n_chunks, 512, 0, st>>>(row_off, G, mask, row_limit, err, f_local, forces, cs);
+    PROF_END("gather_reduce", st);
+    MBF_CHECK_LAUNCH();
+    return MBF_OK;
+}
+
 }  // namespace mbf
 
 extern "C" {

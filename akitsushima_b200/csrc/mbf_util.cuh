@@ -24,6 +24,31 @@ int gather_reduce(int n_struct, int n_atoms, const int *row_off, const double *G
                   double *forces, const double *per_atom, const mbf_reduce_plan *plan, double *partial,
                   double *energy, double *virial, unsigned *sdone, cudaStream_t st);
 
+// gather_reduce for an evaluation whose slots hold a force only where the
+// row's bit in live_mask (4 words an atom, slot s of the row in word s / 32)
+// is set.  A row of more than row_limit entries (the evaluation's staging
+// bound) adds nothing and sets MBF_DEV_ROW_TOO_LONG in err.  sdone must have
+// been cleared by an earlier kernel of the evaluation (ClearWords).
+int gather_live(int n_struct, int n_atoms, const int *row_off, const double *G, const unsigned *live_mask, int row_limit,
+                int *err, const double *f_local, double *forces, const double *per_atom, const mbf_reduce_plan *plan,
+                double *partial, double *energy, double *virial, unsigned *sdone, cudaStream_t st);
+
+// Words an evaluation needs zero in its later kernels (error words, the
+// completion counters), cleared by its first kernel instead of by memsets of
+// their own: a memset node costs a launch-bound step about 1.5 us.
+struct ClearWords {
+    unsigned *a;
+    int na;
+    unsigned *b;
+    int nb;
+    __device__ __forceinline__ void run() const {
+        for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < na + nb; k += gridDim.x * blockDim.x) {
+            if (k < na) a[k] = 0u;
+            else b[k - na] = 0u;
+        }
+    }
+};
+
 // Threads per block of the fused gather kernels: 8 lanes per atom of the
 // plan's mean chunk, at least 128 and at most 512.
 static inline int chunk_block(int n_atoms, int n_chunks) {
