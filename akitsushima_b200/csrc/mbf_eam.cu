@@ -32,24 +32,17 @@ constexpr int EAM_NZ = 20;         // Zhou parameters per element row
 constexpr int EAM_NCOL = 2 * EAM_NZ + 3;
 constexpr int EAM_MAXSP = 8;       // species staged in shared memory (fused path)
 constexpr int EAM_BLOCK = 128;
-// Resident blocks per SM the float32 force kernel is compiled for (it sets
-// the register budget: 65536 / (EAM_BLOCK * MBF_EAM_MINB)).
-#ifndef MBF_EAM_MINB
-#define MBF_EAM_MINB 5
-#endif
-// With the cell as a launch argument (CellView<2>) the kernels need fewer
-// registers: the force pass fits seven blocks per SM at 68 (74 at six,
-// where it measured 126.0 against 123.2 us), the density pass twelve at 40.
-#ifndef MBF_EAM_MINB_BOX
-#define MBF_EAM_MINB_BOX 7
-#endif
-#ifndef MBF_EAM_DENS_MINB_BOX
-#define MBF_EAM_DENS_MINB_BOX 12
-#endif
-// The same for the float32 density kernel (47 registers, no spills).
-#ifndef MBF_EAM_DENS_MINB
-#define MBF_EAM_DENS_MINB 10
-#endif
+
+// Resident blocks per SM the density and force kernels are compiled for
+// (their register budget: 65536 / (EAM_BLOCK * blocks)) in float32; float64
+// kernels take what they need.  With the cell as a launch argument
+// (CellView<2>) the Zhou kernels need fewer registers: the force pass fits
+// seven blocks per SM at 68 (74 at six, where it measured 126.0 against
+// 123.2 us), the density pass twelve at 40; else five and ten (47 registers).
+struct ZhouBounds {
+    static constexpr int dens(int size, int cm) { return size == 4 ? (cm == 2 ? 12 : 10) : 1; }
+    static constexpr int force(int size, int cm) { return size == 4 ? (cm == 2 ? 7 : 5) : 1; }
+};
 
 enum { F_SPLINE = 1, F_SPLINE_R = 2, F_Z_DENS = 3, F_Z_PAIR = 4, F_Z_CROSS = 5, F_Z_EMB = 6 };
 
@@ -436,7 +429,10 @@ __device__ __forceinline__ void dist_ir(double r2, double &r, double &ir) {
 
 template <typename T>
 struct PolGeneric {
+    typedef ZTab<T> Shared;
+    typedef ZhouBounds Bounds;
     static constexpr bool species_addresses = true;  // species index the tables
+    static constexpr bool boxed = false;             // no CellView<2> kernels
     EamDev E;
     __device__ __forceinline__ void setup(ZTab<T> &) const {}
     __device__ __forceinline__ T dens1(const ZTab<T> &, int sj, double r2) const {
@@ -456,6 +452,171 @@ struct PolGeneric {
     }
 };
 
+// ---- setfl tables: cubic splines on one uniform r grid -----------------------
+// The pair and density tables of a setfl alloy share one uniform grid in r,
+// so a pair finds its interval and offset once for its three functions, and
+// each function is one aligned vector load of an interval's four
+// coefficients (float4, or double4 in float64) from a table packed into the
+// workspace at the start of the evaluation (4 us).  256k atoms, 2000 knots,
+// mixed: density 289 -> 121 us, force 470 -> 161 us against PolGeneric's
+// search and strided loads (code, parameter row, two knots, four columns, one
+// after the other), which wait on memory.  What bounds it now is the L1 data
+// pipe (72 % of its wavefronts in the density pass): the scattered neighbour
+// records and table records.
+
+template <typename T> struct Vec4;
+template <> struct Vec4<float> {
+    typedef float4 type;
+    static __device__ __forceinline__ float4 ld(const float4 *p) { return __ldg(p); }
+    static __device__ __forceinline__ float4 make(double a, double b, double c, double d) {
+        return make_float4((float)a, (float)b, (float)c, (float)d);
+    }
+};
+template <> struct Vec4<double> {
+    typedef double4 type;
+    static __device__ __forceinline__ double4 ld(const double4 *p) {
+        const double2 *q = reinterpret_cast<const double2 *>(p);
+        const double2 a = __ldg(q), b = __ldg(q + 1);
+        return make_double4(a.x, a.y, b.x, b.y);
+    }
+    static __device__ __forceinline__ double4 make(double a, double b, double c, double d) {
+        return make_double4(a, b, c, d);
+    }
+};
+
+// Coefficient columns (4, nX) -> one record per interval, in T.
+template <typename T>
+__global__ void eam_pack_splines(int nX, const double *__restrict__ C, typename Vec4<T>::type *__restrict__ out) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k < nX) out[k] = Vec4<T>::make(C[k], C[nX + k], C[2 * (size_t)nX + k], C[3 * (size_t)nX + k]);
+}
+
+// Distance of a pair inside the cutoff and its inverse.  Float32: the root in
+// float64 by one Newton step on the float32 inverse root (about 2e-14
+// relative, far inside a float32 offset within an interval), the inverse by
+// one in float32.
+__device__ __forceinline__ void spline_dist(double r2, double &r, float &ir) {
+    const float q2 = (float)r2, q = rsqrtf(q2);
+    const double r0 = r2 * (double)q;
+    r = fma(0.5 * (double)q, fma(-r0, r0, r2), r0);
+    ir = q * fmaf(-0.5f * q2 * q, q, 1.5f);
+}
+__device__ __forceinline__ void spline_dist(double r2, double &r, double &ir) {
+    r = sqrt(r2);
+    ir = 1.0 / r;
+}
+
+constexpr int SPL_MAXSP = 8;
+
+// First packed record and knot count of each function, and whether the
+// pair tables hold r * phi.
+struct SplTab {
+    int rho_o[SPL_MAXSP], rho_n[SPL_MAXSP];
+    int phi_o[SPL_MAXSP * SPL_MAXSP], phi_n[SPL_MAXSP * SPL_MAXSP];
+    int over_r[SPL_MAXSP * SPL_MAXSP];
+    int rho_over[SPL_MAXSP];
+};
+
+// Resident blocks in float32 (density / force us at 256k: 8 / 5 blocks 117 /
+// 166, 10 / 6 121 / 161, 12 / 7 119 / 162 with spills).
+struct SplineBounds {
+    static constexpr int dens(int size, int) { return size == 4 ? 10 : 1; }
+    static constexpr int force(int size, int) { return size == 4 ? 6 : 1; }
+};
+
+template <typename T>
+struct PolSpline {
+    typedef SplTab Shared;
+    typedef SplineBounds Bounds;
+    typedef typename Vec4<T>::type T4;
+    static constexpr bool species_addresses = true;
+    static constexpr bool boxed = sizeof(T) == 4;
+    EamDev E;
+    const T4 *tab;
+    double x0, ih, h;  // the common grid: first knot, 1 / spacing, spacing
+
+    __device__ __forceinline__ void setup(SplTab &Z) const {
+        for (int k = threadIdx.x; k < E.ns * E.ns; k += blockDim.x) {
+            const int f = E.phi_f[k];
+            Z.phi_o[k] = E.xo[f];
+            Z.phi_n[k] = max(E.nx[f], 2);
+            Z.over_r[k] = E.codes[f] == F_SPLINE_R;
+            if (k < E.ns) {
+                const int g = E.rho_f[k];
+                Z.rho_o[k] = E.xo[g];
+                Z.rho_n[k] = max(E.nx[g], 2);
+                Z.rho_over[k] = E.codes[g] == F_SPLINE_R;
+            }
+        }
+        __syncthreads();
+    }
+    // The interval of r by rounding (r - x0) / h - 1/2 to the nearest integer
+    // with the 1.5 * 2^52 shift, whose low word is the integer; a distance at
+    // a knot (a tie) belongs to the interval above it, as the search gives.
+    struct At {
+        int k;
+        T dx;
+        double d;
+    };
+    __device__ __forceinline__ At locate(double r) const {
+        const double M = 6755399441055744.0;
+        At a;
+        a.d = r - x0;
+        const double u = __dadd_rn(fma(a.d, ih, -0.5), M);
+        a.k = __double2loint(u);
+        double q = fma(-__dsub_rn(u, M), h, a.d);
+        if (q >= h) {
+            ++a.k;
+            q -= h;
+        }
+        a.dx = (T)q;
+        return a;
+    }
+    __device__ __forceinline__ T4 record(At a, int o, int n, T &dx) const {
+        int k = a.k;
+        dx = a.dx;
+        if ((unsigned)k > (unsigned)(n - 2)) {  // extrapolated from the end intervals
+            k = k < 0 ? 0 : n - 2;
+            dx = (T)fma(-(double)k, h, a.d);
+        }
+        return Vec4<T>::ld(tab + o + k);
+    }
+    __device__ __forceinline__ T dens1(const SplTab &Z, int sj, double r2) const {
+        double r;
+        T ir;
+        spline_dist(r2, r, ir);
+        T dx;
+        const T4 c = record(locate(r), Z.rho_o[sj], Z.rho_n[sj], dx);
+        const T v = ((c.x * dx + c.y) * dx + c.z) * dx + c.w;
+        return Z.rho_over[sj] ? v * ir : v;
+    }
+    static __device__ __forceinline__ T slope(const T4 &c, T dx) {
+        return (T(3) * c.x * dx + T(2) * c.y) * dx + c.z;
+    }
+    static __device__ __forceinline__ T value(const T4 &c, T dx) { return ((c.x * dx + c.y) * dx + c.z) * dx + c.w; }
+    __device__ __forceinline__ void pair(const SplTab &Z, int si, int sj, double r2, T &phi, T &dphi, T &drj, T &dri,
+                                         T &ir) const {
+        double r;
+        spline_dist(r2, r, ir);
+        const At a = locate(r);
+        const int f = si * E.ns + sj;
+        T xp, xj, xi;
+        const T4 cp = record(a, Z.phi_o[f], Z.phi_n[f], xp);
+        const T4 cj = record(a, Z.rho_o[sj], Z.rho_n[sj], xj);
+        const T4 ci = record(a, Z.rho_o[si], Z.rho_n[si], xi);
+        phi = value(cp, xp);
+        dphi = slope(cp, xp);
+        drj = slope(cj, xj);
+        dri = slope(ci, xi);
+        if (Z.over_r[f]) {
+            phi *= ir;
+            dphi = (dphi - phi) * ir;
+        }
+        if (Z.rho_over[sj]) drj = (drj - value(cj, xj) * ir) * ir;
+        if (Z.rho_over[si]) dri = (dri - value(ci, xi) * ir) * ir;
+    }
+};
+
 template <typename T>
 __device__ __forceinline__ T pair_dist(double r2);
 template <> __device__ __forceinline__ double pair_dist<double>(double r2) { return sqrt(r2); }
@@ -463,7 +624,10 @@ template <> __device__ __forceinline__ float pair_dist<float>(double r2) { retur
 
 template <typename T>
 struct PolZSmem {
+    typedef ZTab<T> Shared;
+    typedef ZhouBounds Bounds;
     static constexpr bool species_addresses = true;  // species index the tables
+    static constexpr bool boxed = false;
     EamDev E;
     __device__ __forceinline__ void setup(ZTab<T> &Z) const { load_ztab<T>(E, Z); }
     __device__ __forceinline__ T dens1(const ZTab<T> &Z, int sj, double r2) const {
@@ -501,6 +665,9 @@ __device__ __forceinline__ float zdens_f32(const ZK<float> &K, int sj, double r2
 
 template <typename T, int NS>
 struct PolZ2 {
+    typedef ZTab<T> Shared;
+    typedef ZhouBounds Bounds;
+    static constexpr bool boxed = sizeof(T) == 4;
     static constexpr bool species_addresses = false;  // species only compared, never an index
     ZK<T> K;
     __device__ __forceinline__ void setup(ZTab<T> &) const {}
@@ -637,6 +804,9 @@ __device__ __forceinline__ void zdec2(f2x r2, f2x dre, f2x ire, f2x nshift, f2x 
 }
 
 struct PolZ2x {
+    typedef ZTab<float> Shared;
+    typedef ZhouBounds Bounds;
+    static constexpr bool boxed = true;
     static constexpr bool species_addresses = false;  // species only compared, never an index
     ZK<float> K;
     ZK2x X;
@@ -781,10 +951,10 @@ __device__ __forceinline__ double3 ld_pos(const double *__restrict__ pos, int j)
 // aux[2 i].  Slot indices are loaded two iterations ahead, the neighbour's
 // position and species one ahead.
 template <typename T, int LPA, class Pol, int CM>
-__global__ void __launch_bounds__(EAM_BLOCK, sizeof(T) == 4 ? (CM == 2 ? MBF_EAM_DENS_MINB_BOX : MBF_EAM_DENS_MINB) : 1)
+__global__ void __launch_bounds__(EAM_BLOCK, Pol::Bounds::dens(sizeof(T), CM))
     eam_density(SysView S, const int *__restrict__ row_off, const int *__restrict__ nbr, Pol P, double rc2,
                 double *__restrict__ aux, Chk ck) {
-    __shared__ ZTab<T> Z;
+    __shared__ typename Pol::Shared Z;
     P.setup(Z);
     const int sub = threadIdx.x & (LPA - 1);
     const int gpb = EAM_BLOCK / LPA;
@@ -874,13 +1044,13 @@ template <> struct SlotVec<float> {
 // of the row, at most about 20 terms; float64 across lanes and in the
 // gather) and double in the float64 path.
 template <typename T, int LPA, class Pol, int CM>
-__global__ void __launch_bounds__(EAM_BLOCK, sizeof(T) == 4 ? (CM == 2 ? MBF_EAM_MINB_BOX : MBF_EAM_MINB) : 1)
+__global__ void __launch_bounds__(EAM_BLOCK, Pol::Bounds::force(sizeof(T), CM))
     eam_force(SysView S, const int *__restrict__ row_off, const int *__restrict__ upper,
               const int *__restrict__ nbr, const int *__restrict__ rev, Pol P, double rc2,
               const double4 *__restrict__ pk, const double *__restrict__ aux,
               typename SlotVec<T>::type *__restrict__ slot_f, double *__restrict__ f_local,
               double *__restrict__ per_atom, Chk ck) {
-    __shared__ ZTab<T> Z;
+    __shared__ typename Pol::Shared Z;
     P.setup(Z);
     const int sub = threadIdx.x & (LPA - 1);
     const int gpb = EAM_BLOCK / LPA;
@@ -1084,7 +1254,7 @@ __global__ void __launch_bounds__(EAM_BLOCK) eam_site(SysView S, const int *__re
                                                       const double4 *__restrict__ pk,
                                                       const double *__restrict__ aux, SiteOut so, Chk ck) {
     constexpr int LPA = 8;
-    __shared__ ZTab<T> Z;
+    __shared__ typename Pol::Shared Z;
     P.setup(Z);
     const int sub = threadIdx.x & (LPA - 1);
     const int gpb = EAM_BLOCK / LPA;
@@ -1137,7 +1307,8 @@ __global__ void __launch_bounds__(EAM_BLOCK) eam_site(SysView S, const int *__re
 struct EamBufs {
     double4 *pk;
     double *aux;
-    void *slot;  // per-slot pair forces (SlotVec<T>)
+    void *slot;    // per-slot pair forces (SlotVec<T>)
+    void *slot_b;  // 16 bytes per slot: the packed spline tables
     double *f_local;
     double *forces;
     double *per_atom;
@@ -1225,8 +1396,8 @@ template <typename T, class Pol>
 static int eam_dispatch(const Pol &P, int lpa, const SysView &S, const mbf_nlist *nl, const EamDev &E, double rc2,
                         const EamBufs &B, Chk ck, const SiteOut &so, const ChunkSums &cs, int n_chunks,
                         int phases, cudaStream_t st) {
-    // the launch-argument box for the float32 one- and two-element Zhou path
-    if constexpr (sizeof(T) == 4 && !Pol::species_addresses)
+    // the launch-argument box for the policies that have such kernels
+    if constexpr (Pol::boxed)
         if (S.boxed) return eam_dispatch_lpa<T, Pol, 2>(lpa, S, nl, P, E, rc2, B, ck, so, cs, n_chunks, phases, st);
     return S.ortho ? eam_dispatch_lpa<T, Pol, 1>(lpa, S, nl, P, E, rc2, B, ck, so, cs, n_chunks, phases, st)
                    : eam_dispatch_lpa<T, Pol, 0>(lpa, S, nl, P, E, rc2, B, ck, so, cs, n_chunks, phases, st);
@@ -1273,10 +1444,46 @@ static bool make_zk(const mbf_eam_tables *tab, ZK<T> &K) {
     return true;
 }
 
+// The common grid of the pair and density tables, from the host copy of the
+// parameter rows: every one a spline on uniform knots (a row [1, x0, 1 / h, 0
+// ...]) with the same x0 and h; false otherwise.
+static bool spline_grid(const mbf_eam_tables *tab, double &x0, double &ih) {
+    if (tab->zhou_fused || tab->ns < 1 || tab->ns > SPL_MAXSP || !tab->P_host || !tab->rho_f_host || !tab->phi_f_host)
+        return false;
+    const int ns = tab->ns;
+    for (int k = 0; k < ns + ns * ns; ++k) {
+        const int f = k < ns ? tab->rho_f_host[k] : tab->phi_f_host[k - ns];
+        const double *p = tab->P_host + (size_t)f * EAM_NCOL;
+        if (p[0] != 1.0 || !(p[2] > 0.0)) return false;
+        for (int c = 3; c < EAM_NCOL; ++c)
+            if (p[c] != 0.0) return false;
+        if (k == 0) {
+            x0 = p[1];
+            ih = p[2];
+        } else if (p[1] != x0 || p[2] != ih) {
+            return false;
+        }
+    }
+    return true;
+}
+
 template <typename T>
 static int eam_select(const mbf_eam_tables *tab, int lpa, const SysView &S, const mbf_nlist *nl, const EamDev &E,
                       double rc2, const EamBufs &B, Chk ck, const SiteOut &so, const ChunkSums &cs, int n_chunks,
                       int ph, cudaStream_t st) {
+    PolSpline<T> spl;
+    // the packed tables live in the slot_b region, 16 bytes per list slot: a
+    // list too short for them (a few hundred atoms) keeps the generic path
+    if (spline_grid(tab, spl.x0, spl.ih) &&
+        (size_t)tab->nX * sizeof(typename PolSpline<T>::T4) <= 16 * (size_t)ck.n_slots) {
+        spl.E = E;
+        spl.h = 1.0 / spl.ih;
+        auto *packed = static_cast<typename PolSpline<T>::T4 *>(B.slot_b);
+        spl.tab = packed;
+        eam_pack_splines<T><<<(tab->nX + 255) / 256, 256, 0, st>>>(tab->nX, E.C, packed);
+        MBF_CHECK_LAUNCH();
+        return eam_dispatch<T>(spl, lpa, S, nl, E, rc2, B, ck, so, cs, n_chunks, ph, st);
+    }
     ZK<T> K;
     if (make_zk<T>(tab, K)) {
         if (tab->ns == 1)
@@ -1364,6 +1571,7 @@ static int eam_eval(const mbf_system *sys, const mbf_nlist *nl, const mbf_eam_ta
     B.pk = ws_at<double4>(workspace, L.pack);
     B.aux = ws_at<double>(workspace, L.atom_aux);
     B.slot = ws_at<char>(workspace, L.slot);
+    B.slot_b = ws_at<char>(workspace, L.slot_b);
     B.f_local = ws_at<double>(workspace, L.f_local);
     B.forces = forces;
     B.per_atom = ws_at<double>(workspace, L.per_atom);

@@ -141,10 +141,10 @@ constexpr int ERR_CLEAR_BYTES = 16;
 //   err      device error words (ints; see ERR_CLEAR_BYTES)
 //   per_atom (n_atoms, ATOM_ACC) doubles
 //   f_local  (n_atoms, 3) doubles (three-body potentials: centre-local force)
-//   atom_aux (n_atoms, 2) doubles (EAM F'(rho), F(rho))
+//   atom_aux (n_atoms, 2) doubles (EAM F'(rho), F(rho); three-body: live mask)
 //   pack     (n_atoms, 4) doubles (position + F'(rho), one record per atom)
 //   slot     (n_slots, 3) doubles (three-body force left on each neighbour)
-//   slot_b   (n_slots, 2) doubles (Tersoff bond order and its derivative)
+//   slot_b   (n_slots, 2) doubles (EAM: the packed spline tables)
 //   partial  (n_chunks, ATOM_ACC) doubles
 //   sdone    (n_chunks,) completion counters of the per-structure sums
 struct EvalLayout {
