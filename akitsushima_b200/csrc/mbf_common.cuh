@@ -102,6 +102,69 @@ __device__ __forceinline__ const double *cell_of(const SysView &S, int atom) {
     return S.cells + 18 * (size_t)s;
 }
 
+// One centre's cell in registers, for a loop over its row: a diagonal cell
+// (the same branch for the whole launch) by its three lengths, any other by
+// the 3x3 pair, with fused multiply-add.  Every operation is odd in the
+// displacement, so both atoms of a pair see the same vector up to its sign.
+struct RowCell {
+    double c[18];
+    bool ortho;
+    __device__ __forceinline__ void load(const SysView &S, int atom) {
+        const double *p = cell_of(S, atom);
+        ortho = S.ortho != 0;
+        if (ortho) {
+#pragma unroll
+            for (int k = 0; k < 18; ++k) c[k] = 0.0;
+            c[0] = __ldg(p); c[4] = __ldg(p + 4); c[8] = __ldg(p + 8);
+            c[9] = __ldg(p + 9); c[13] = __ldg(p + 13); c[17] = __ldg(p + 17);
+        } else {
+#pragma unroll
+            for (int k = 0; k < 18; ++k) c[k] = __ldg(p + k);
+        }
+    }
+    __device__ __forceinline__ void mic(double rx, double ry, double rz, double &dx, double &dy, double &dz) const {
+        if (ortho) {
+            dx = rx - c[0] * rint_shift(rx * c[9]);
+            dy = ry - c[4] * rint_shift(ry * c[13]);
+            dz = rz - c[8] * rint_shift(rz * c[17]);
+        } else {
+            double sx = rx * c[9] + ry * c[12] + rz * c[15];
+            double sy = rx * c[10] + ry * c[13] + rz * c[16];
+            double sz = rx * c[11] + ry * c[14] + rz * c[17];
+            sx -= rint_shift(sx);
+            sy -= rint_shift(sy);
+            sz -= rint_shift(sz);
+            dx = sx * c[0] + sy * c[3] + sz * c[6];
+            dy = sx * c[1] + sy * c[4] + sz * c[7];
+            dz = sx * c[2] + sy * c[5] + sz * c[8];
+        }
+    }
+};
+
+// sqrt(r2) in float64 for a float32 evaluation: one Newton step on the
+// float32 inverse root (about 1e-14 relative), a fifth of sqrt()'s
+// instructions.  r2 within float32's range.
+__device__ __forceinline__ double root_near(double r2) {
+    const double q = (double)rsqrtf((float)r2), r0 = r2 * q;
+    return fma(0.5 * q, fma(-r0, r0, r2), r0);
+}
+template <typename T> __device__ __forceinline__ double leg_root(double r2);
+template <> __device__ __forceinline__ double leg_root<double>(double r2) { return sqrt(r2); }
+template <> __device__ __forceinline__ double leg_root<float>(double r2) { return root_near(r2); }
+
+// r and 1 / r of a leg in float64: the inverse root by one Newton step on the
+// float32 one for a float32 evaluation.
+template <typename T> __device__ __forceinline__ void leg_dist(double r2, double &r, double &ir);
+template <> __device__ __forceinline__ void leg_dist<double>(double r2, double &r, double &ir) {
+    r = sqrt(r2);
+    ir = 1.0 / r;
+}
+template <> __device__ __forceinline__ void leg_dist<float>(double r2, double &r, double &ir) {
+    const double q = (double)rsqrtf((float)r2);
+    ir = q * fma(-0.5 * r2 * q, q, 1.5);
+    r = r2 * ir;
+}
+
 // Sum over the LPA lanes of a lane group (all 32 lanes must call it).
 template <int LPA, typename T>
 __device__ __forceinline__ T group_sum(T v) {

@@ -7,15 +7,21 @@
 // (:1165-1451, both orders with lambda/2 of their own (i, j, k) record, legs
 // from the pair records (i, j, j)).  The two-body term of a pair reads the
 // record of the lower-indexed atom (:714-762).
-#include "mbf_util.cuh"
+#include "mbf_rows.cuh"
 
 namespace mbf {
 
 // Lanes per atom (LPA) is a template parameter chosen by the host (the
-// autotuner); lane groups per block keep the staged rows under 48 KB.
+// autotuner); GPB lane groups per block keep the staged rows near 15 KB, so
+// that registers and not shared memory bound the resident warps.
 template <int MAXN, int LPA> struct SwGeom {
-    static constexpr int GPB = 512 / MAXN;
+    static constexpr int WIDE = 512 / MAXN < 32 / LPA ? 512 / MAXN : 32 / LPA;  // a whole warp, if 48 KB hold it
+    static constexpr int GPB = 256 / MAXN > WIDE ? 256 / MAXN : WIDE;
     static constexpr int BLOCK = GPB * LPA;
+    // Resident threads per SM the kernel is compiled for (its registers):
+    // with the gather, 64,000-atom Ge-Sn mixed at 640 / 768 / 896 threads 103 /
+    // 98 / 96 us, 32,768-atom Ge-Sn float64 at 512 / 640 78 / 83.
+    static constexpr int min_blocks(int size) { return (size == 8 ? 512 : 896) / (BLOCK < 32 ? 32 : BLOCK); }
 };
 
 struct SwDev {
@@ -26,6 +32,62 @@ struct SwDev {
     double rc;
 };
 
+// Records as the kernel reads them, in T.
+template <typename T> struct SwPair { T valid, eps, sig, a, A, B, p, q; };
+template <typename T> struct SwLeg { T sig, a, gam, pad; };
+template <typename T> struct SwTri { T c, cos0; };  // c = 0: no such angle
+
+template <typename T>
+__device__ __forceinline__ SwPair<T> sw_pair_row(const double *__restrict__ t) {
+    return {(T)__ldg(t), (T)__ldg(t + 1), (T)__ldg(t + 2), (T)__ldg(t + 3),
+            (T)__ldg(t + 4), (T)__ldg(t + 5), (T)__ldg(t + 6), (T)__ldg(t + 7)};
+}
+template <typename T>
+__device__ __forceinline__ SwLeg<T> sw_leg_row(const double *__restrict__ t) {
+    return {(T)__ldg(t), (T)__ldg(t + 1), (T)__ldg(t + 2), T(0)};
+}
+template <typename T>
+__device__ __forceinline__ SwTri<T> sw_tri_row(const double *__restrict__ t) {
+    return {__ldg(t) != 0.0 ? (T)__ldg(t + 1) : T(0), (T)__ldg(t + 2)};
+}
+
+// The square of the distance beyond which the pair (a, b) takes part in no
+// term, from either atom (a little beyond: the terms test their own cutoff).
+// Both atoms of a pair agree on it.
+__device__ __forceinline__ double sw_reach2(const SwDev &P, int a, int b) {
+    double r = 0.0;
+    for (int o = 0; o < 2; ++o) {
+        const int ab = o == 0 ? a * P.ns + b : b * P.ns + a;
+        const double *t = P.tb + 8 * ab, *l = P.leg + 4 * ab;
+        if (__ldg(t) != 0.0) r = fmax(r, __ldg(t + 2) * __ldg(t + 3));
+        r = fmax(r, __ldg(l) * __ldg(l + 1));
+    }
+    return r * r * (1.0 + 1e-6);
+}
+
+// The tables of up to SW_SH species in shared memory.
+constexpr int SW_SH = 3;
+template <typename T>
+struct SwTab {
+    SwPair<T> pair[SW_SH * SW_SH];
+    SwLeg<T> leg[SW_SH * SW_SH];
+    SwTri<T> tri[SW_SH * SW_SH * SW_SH];
+    double reach2[SW_SH * SW_SH];
+};
+
+template <typename T>
+__device__ __forceinline__ void sw_load_tab(const SwDev &P, SwTab<T> &B) {
+    const int ns = P.ns;
+    if (ns > SW_SH) return;
+    for (int q = threadIdx.x; q < ns * ns; q += blockDim.x) {
+        B.pair[q] = sw_pair_row<T>(P.tb + 8 * q);
+        B.leg[q] = sw_leg_row<T>(P.leg + 4 * q);
+        B.reach2[q] = sw_reach2(P, q / ns, q % ns);
+    }
+    for (int q = threadIdx.x; q < ns * ns * ns; q += blockDim.x) B.tri[q] = sw_tri_row<T>(P.tri + 4 * q);
+    __syncthreads();
+}
+
 // Per-leg factors of the three-body term (engine/stillinger_weber.py:96-154):
 // h(i, j, k) = c3 E_j E_k (cos theta_jik - cos0)^2 with E_x = exp(gamma_x /
 // (r_ix / sigma_x - a_x)) and dE_x/dr_ix = E_x D_x, D_x = -gamma_x /
@@ -34,267 +96,261 @@ struct SwDev {
 // early return).  The legs depend only on (centre, neighbour), so they are
 // evaluated once per slot, not once per angle.
 template <typename T>
-__device__ __forceinline__ void sw_leg(T r, T sig, T a, T gam, T &E, T &D) {
-    T x = r / sig;
-    if (!(x < a)) {
-        E = T(0);
-        D = T(0);
-        return;
-    }
-    T d = x - a;
-    E = clamped_exp<T>(gam / d);
-    D = -gam / (sig * d * d);
+__device__ __forceinline__ void sw_leg(T r, const SwLeg<T> &l, T &E, T &D) {
+    E = T(0);
+    D = T(0);
+    const T x = r / l.sig;
+    if (!(x < l.a)) return;
+    const T d = x - l.a;
+    E = clamped_exp<T>(l.gam / d);
+    if (E != T(0)) D = -l.gam / (l.sig * d * d);
 }
 
-// One centre's row staged in shared memory: displacements, 1/r, leg
-// factors, species, and the slots inside the cutoff compacted into `list`.
+// Two-body energy and its r-derivative (engine/stillinger_weber.py:23-52).
+template <typename T>
+__device__ __forceinline__ void sw_two(T r, const SwPair<T> &t, T &V2, T &dV2) {
+    V2 = T(0);
+    dV2 = T(0);
+    const T x = r / t.sig;
+    if (t.valid == T(0) || !(x < t.a)) return;
+    const T tt = T(1) / (x - t.a), ex = clamped_exp<T>(tt), ix = T(1) / x;
+    T xp, xq;
+    if (t.p == T(4)) {  // the published silicon exponents need no pow
+        const T i2 = ix * ix;
+        xp = i2 * i2;
+    } else {
+        xp = RT<T>::pw(x, -t.p);
+    }
+    xq = t.q == T(0) ? T(1) : RT<T>::pw(x, -t.q);
+    const T w = t.eps * t.A * ex, u = t.B * xp - xq;
+    V2 = w * u;
+    dV2 = w * ((-t.p * t.B * xp + t.q * xq) * ix - u * (tt * tt)) / t.sig;
+}
+
+// One centre's legs in shared memory, compacted in slot order: displacement
+// and unit vector, length and leg factors.  Groups of a warp lie 32 bytes
+// apart modulo the banks' 128.
 template <typename T, int MAXN>
 struct SwRow {
-    T x[MAXN], y[MAXN], z[MAXN], r[MAXN], ir[MAXN], E[MAXN], D[MAXN];
-    int sp[MAXN];
-    int list[MAXN];
+    T ux[MAXN], uy[MAXN], uz[MAXN], E[MAXN], D[MAXN], x[MAXN], y[MAXN], z[MAXN], r[MAXN];
+    int sp[MAXN], rev[MAXN];
+    int meta[MAXN];  // slot in the row | (i < j) << 8
+    char pad[32];
 };
 
-// SYM: every (i, j, k) record equals its (i, k, j) twin (one species): one
-// coefficient and cos0 for every angle.  Otherwise both orders, each with
-// its own record (lambda/2 of (i, j, k) and of (i, k, j)).
+// SYM: one species, so every angle has one coefficient and cos0.  Otherwise
+// both orders of an angle, each with its own record (lambda/2 of (i, j, k)
+// and of (i, k, j)).
 //
-// For slot s and partner k (both inside the cutoff, k != s) with
-// P = E_s E_k, cos = u_s . u_k, dc_o = cos - cos0_o over the orders o:
-//   energy booked on slot s:  c_1 P dc_1^2        (order (i, s, k))
+// For leg s and partner k with P = E_s E_k, cos = u_s . u_k, dc_o = cos -
+// cos0_o over the orders o:
+//   energy booked on leg s:  c_1 P dc_1^2        (order (i, s, k))
 //   dh/dr_s = P [D_s A u_s + (B / r_s)(u_k - cos u_s)],
 //   A = sum_o c_o dc_o^2,  B = 2 sum_o c_o dc_o,
-// so each ordered triple's energy is booked once and each slot collects the
-// whole gradient of every angle on its own leg.
+// so each ordered triple's energy is booked once and each leg collects the
+// whole gradient of every angle on it; the sums over k are a vector
+// (P B u_k) and two scalars (P A and P B cos).  With half of the leg's pair
+// term that is D_s = dU_i/dr_s, kept on i and left negated in the neighbour's
+// own slot.
+//
+// Bound by instruction issue and latency: 16 legs and 240 ordered angles a
+// centre in 64,000-atom Ge-Sn.  The record tables are staged in T (an angle's
+// records were six float64 loads and conversions), legs beyond their own
+// pair's reach are dropped before the angle loop, and the sums over k are in
+// unit vectors: 136 -> 96 us there with the gather, mixed.  (The legs of a
+// block as one list, as the Tersoff kernel has them, took 104: its 23 KB of
+// staged legs leave fewer warps resident than the fuller lanes gain.)
 template <typename T, int MAXN, bool SYM, int LPA>
-__global__ void sw_force(SysView S, const int *__restrict__ row_off, const int *__restrict__ nbr,
-                         const int *__restrict__ rev, SwDev P, double *__restrict__ slot_G, double *__restrict__ f_local,
-                         double *__restrict__ per_atom, int *__restrict__ err, SiteOut so) {
+__global__ void __launch_bounds__(SwGeom<MAXN, LPA>::BLOCK, SwGeom<MAXN, LPA>::min_blocks(sizeof(T)))
+    sw_center(SysView S, const int *__restrict__ row_off, const int *__restrict__ nbr, const int *__restrict__ rev,
+              SwDev P, double *__restrict__ slot_G, double *__restrict__ f_local, double *__restrict__ per_atom,
+              unsigned *__restrict__ live_mask, int n_slots, ClearWords clr, SiteOut so) {
     constexpr int GPB = SwGeom<MAXN, LPA>::GPB;
+    constexpr int NB = LPA < 8 ? LPA : 8, KS = LPA / NB;
     __shared__ SwRow<T, MAXN> rows[GPB];
-    const int sub = threadIdx.x & (LPA - 1);
-    const int lane = threadIdx.x & 31;
-    const unsigned gmask = (LPA == 32) ? 0xffffffffu : (((1u << LPA) - 1u) << (lane & ~(LPA - 1)));
+    __shared__ SwTab<T> B;
+    const int i = blockIdx.x * GPB + threadIdx.x / LPA;
+    RowHead head;
+    head.load(S, row_off, i);
+    clr.run();
+    sw_load_tab<T>(P, B);
+    const int sub = threadIdx.x & (LPA - 1), gl = threadIdx.x & 31 & ~(LPA - 1);
+    const unsigned gmask = ((1u << LPA) - 1u) << gl;
+    const int lt = sub & (NB - 1), ks = sub / NB;
     SwRow<T, MAXN> &R = rows[threadIdx.x / LPA];
     const int ns = P.ns;
-    for (int base = blockIdx.x * GPB; base < S.n_atoms; base += gridDim.x * GPB) {
-        int i = base + threadIdx.x / LPA;
-        int beg = 0, n = 0, nok = 0, si = 0;
-        bool live = i < S.n_atoms;
-        if (live) {
-            beg = row_off[i];
-            n = row_off[i + 1] - beg;
-            if (n > MAXN) {
-                if (sub == 0) atomicOr(err, MBF_DEV_ROW_TOO_LONG);
-                live = false;
-            }
-        }
-        if (live) {
-            si = S.types[i];
-            const double *cell = cell_of(S, i);
-            double xi = S.pos[3 * (size_t)i], yi = S.pos[3 * (size_t)i + 1], zi = S.pos[3 * (size_t)i + 2];
-            // n is uniform over the lane group, so every lane of the group
-            // takes the same number of trips and the ballot is complete
-            for (int s0 = 0; s0 < n; s0 += LPA) {
-                int s = s0 + sub;
-                bool ok = false;
-                if (s < n) {
-                    int j = nbr[beg + s];
-                    double dx, dy, dz;
-                    mic_exact(cell, S.pos[3 * (size_t)j] - xi, S.pos[3 * (size_t)j + 1] - yi,
-                              S.pos[3 * (size_t)j + 2] - zi, dx, dy, dz);
-                    double r = sqrt(dx * dx + dy * dy + dz * dz);
-                    ok = r < P.rc && r > 1e-12;
-                    if (so.vec) {
-                        size_t os = 3 * (size_t)(beg + s);
-                        so.vec[os] = dx;
-                        so.vec[os + 1] = dy;
-                        so.vec[os + 2] = dz;
-                    }
-                    if (ok) {
-                        int sj = S.types[j];
-                        const double *ls = P.leg + 4 * (si * ns + sj);
-                        T E, D;
-                        sw_leg<T>((T)r, (T)ls[0], (T)ls[1], (T)ls[2], E, D);
-                        R.x[s] = (T)dx;
-                        R.y[s] = (T)dy;
-                        R.z[s] = (T)dz;
-                        R.r[s] = (T)r;
-                        R.ir[s] = T(1) / (T)r;
-                        R.E[s] = E;
-                        R.D[s] = D;
-                        R.sp[s] = sj;
-                    } else {
-                        size_t o = 3 * (size_t)rev[beg + s];
-                        slot_G[o] = 0.0;
-                        slot_G[o + 1] = 0.0;
-                        slot_G[o + 2] = 0.0;
-                    }
-                }
-                unsigned b = __ballot_sync(gmask, ok) >> (lane & ~(LPA - 1));
-                if (LPA < 32) b &= (1u << LPA) - 1u;
-                if (ok) R.list[nok + __popc(b & ((1u << sub) - 1u))] = s;
-                nok += __popc(b);
-            }
-        }
-        __syncwarp();
-        double fx = 0, fy = 0, fz = 0, e = 0;
-        double v[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-        if (live) {
-            T c_sym = T(0), cos0_sym = T(0);
-            if (SYM) {
-                c_sym = (T)P.tri[1];
-                cos0_sym = (T)P.tri[2];
-                if (P.tri[0] == 0.0) c_sym = T(0);
-            }
-            for (int t = sub; t < nok; t += LPA) {
-                int s = R.list[t];
-                int j = nbr[beg + s];
-                int sj = R.sp[s];
-                T xs = R.x[s], ys = R.y[s], zs = R.z[s], r = R.r[s], irs = R.ir[s];
-                T Es = R.E[s], Ds = R.D[s];
-                double dx = (double)xs, dy = (double)ys, dz = (double)zs;
-                double cx = 0.0;
-                // two-body (engine/stillinger_weber.py:23-52), record of the
-                // lower-indexed atom's species order
-                int lo = i < j ? si : sj, hi = i < j ? sj : si;
-                const double *t2 = P.tb + 8 * (lo * ns + hi);
-                if (t2[0] != 0.0) {
-                    T sig = (T)t2[2], a = (T)t2[3];
-                    T xi_ = r / sig;
-                    if (xi_ < a) {
-                        T eps = (T)t2[1], A = (T)t2[4], B = (T)t2[5], pp = (T)t2[6], qq = (T)t2[7];
-                        T tt = T(1) / (xi_ - a);
-                        T ex = clamped_exp<T>(tt);
-                        T xp = RT<T>::pw(xi_, -pp), xq = RT<T>::pw(xi_, -qq);
-                        T V2 = eps * A * (B * xp - xq) * ex;
-                        T dV2 = eps * A * ex * ((-pp * B * xp / xi_ + qq * xq / xi_) + (B * xp - xq) * (-tt * tt));
-                        e += 0.5 * (double)V2;
-                        cx = (double)(dV2 / sig / r);
-                    }
-                }
-                // three-body angles with slot s as one leg
-                T gx = T(0), gy = T(0), gz = T(0);
-                double e3 = 0.0;
-                if (Es != T(0)) {
-                    for (int u = 0; u < nok; ++u) {
-                        if (u == t) continue;
-                        int k = R.list[u];
-                        T Ek = R.E[k];
-                        if (Ek == T(0)) continue;
-                        T xk = R.x[k], yk = R.y[k], zk = R.z[k], irk = R.ir[k];
-                        T cs = (xs * xk + ys * yk + zs * zk) * (irs * irk);
-                        T Pp = Es * Ek;
-                        T A, B, eh;
-                        if (SYM) {
-                            T dc = cs - cos0_sym;
-                            eh = c_sym * dc * dc;
-                            A = T(2) * eh;
-                            B = T(4) * c_sym * dc;
-                        } else {
-                            int sk = R.sp[k];
-                            const double *t3 = P.tri + 4 * ((si * ns + sj) * ns + sk);
-                            const double *t3r = P.tri + 4 * ((si * ns + sk) * ns + sj);
-                            T c1 = t3[0] != 0.0 ? (T)t3[1] : T(0);
-                            T c2 = t3r[0] != 0.0 ? (T)t3r[1] : T(0);
-                            T dc1 = cs - (T)t3[2], dc2 = cs - (T)t3r[2];
-                            eh = c1 * dc1 * dc1;
-                            A = eh + c2 * dc2 * dc2;
-                            B = T(2) * (c1 * dc1 + c2 * dc2);
-                        }
-                        e3 += (double)(Pp * eh);
-                        // dh/dr_s = P [(D_s A - B cos / r_s) u_s + (B / r_k) ... ] in
-                        // displacement form: u_s = d_s / r_s, u_k = d_k / r_k
-                        T as = Pp * (Ds * A - B * cs * irs) * irs;
-                        T ak = Pp * B * irs * irk;
-                        gx += as * xs + ak * xk;
-                        gy += as * ys + ak * yk;
-                        gz += as * zs + ak * zk;
-                    }
-                }
-                e += e3;
-                double Gx = -(double)gx, Gy = -(double)gy, Gz = -(double)gz;
-                fx += cx * dx - Gx;
-                fy += cx * dy - Gy;
-                fz += cx * dz - Gz;
-                double hx = 0.5 * cx * dx, hy = 0.5 * cx * dy, hz = 0.5 * cx * dz;
-                v[0] += -hx * dx + Gx * dx;
-                v[1] += -hx * dy + Gx * dy;
-                v[2] += -hx * dz + Gx * dz;
-                v[3] += -hy * dx + Gy * dx;
-                v[4] += -hy * dy + Gy * dy;
-                v[5] += -hy * dz + Gy * dz;
-                v[6] += -hz * dx + Gz * dx;
-                v[7] += -hz * dy + Gz * dy;
-                v[8] += -hz * dz + Gz * dz;
-                if (so.dudv) {  // U_i = 1/2 sum V2 + angles at i (engine/site_terms.py:179-300)
-                    size_t os = 3 * (size_t)(beg + s);
-                    so.dudv[os] = 0.5 * cx * dx - Gx;
-                    so.dudv[os + 1] = 0.5 * cx * dy - Gy;
-                    so.dudv[os + 2] = 0.5 * cx * dz - Gz;
-                }
-                // the force on neighbour j goes to j's own slot (j -> i)
-                size_t o = 3 * (size_t)rev[beg + s];
-                slot_G[o] = Gx;
-                slot_G[o + 1] = Gy;
-                slot_G[o + 2] = Gz;
-            }
-        }
-        fx = group_sum<LPA>(fx);
-        fy = group_sum<LPA>(fy);
-        fz = group_sum<LPA>(fz);
-        e = group_sum<LPA>(e);
-#pragma unroll
-        for (int q = 0; q < 9; ++q) v[q] = group_sum<LPA>(v[q]);
-        if (sub == 0 && i < S.n_atoms && so.e) so.e[i] = e;
-        if (sub == 0 && i < S.n_atoms) {
-            f_local[3 * (size_t)i] = fx;
-            f_local[3 * (size_t)i + 1] = fy;
-            f_local[3 * (size_t)i + 2] = fz;
-            double *pa = per_atom + (size_t)i * ATOM_ACC;
-            pa[0] = e;
-#pragma unroll
-            for (int q = 0; q < 9; ++q) pa[1 + q] = v[q];
-            pa[10] = (double)nok;
-        }
-        __syncwarp();
+    const bool small = ns <= SW_SH;
+    double fx = 0, fy = 0, fz = 0, e = 0;
+    double v[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+    head.slots<LPA>(nbr, rev, n_slots, ns, MAXN);
+    const RowStage st = stage_row<LPA>(
+        S, head, nbr, rev, n_slots, ns, P.rc, i, live_mask, so.vec,
+        [&](int a, int b) { return small ? B.reach2[a * ns + b] : sw_reach2(P, a, b); },
+        [&](int q, int s, int j, int sj, int rs, double dx, double dy, double dz, double r2) {
+            R.x[q] = (T)dx;
+            R.y[q] = (T)dy;
+            R.z[q] = (T)dz;
+            // unit vector and length rounded once, from float64
+            double r, ir;
+            leg_dist<T>(r2, r, ir);
+            R.r[q] = (T)r;
+            R.ux[q] = (T)(dx * ir);
+            R.uy[q] = (T)(dy * ir);
+            R.uz[q] = (T)(dz * ir);
+            R.sp[q] = sj;
+            R.rev[q] = rs;
+            R.meta[q] = s | (i < j ? 1 << 8 : 0);
+        });
+    const int nl = st.nl, beg = st.beg, si = st.si;
+    __syncwarp(gmask);
+    for (int q = sub; q < nl; q += LPA) {
+        const int ij = si * ns + R.sp[q];
+        T E, D;
+        sw_leg<T>(R.r[q], small ? B.leg[ij] : sw_leg_row<T>(P.leg + 4 * ij), E, D);
+        R.E[q] = E;
+        R.D[q] = D;
     }
+    __syncwarp(gmask);
+    SwTri<T> own = {T(0), T(0)};
+    if (SYM) own = B.tri[0];
+    for (int t0 = 0; t0 < nl; t0 += NB) {
+        const int t = t0 + lt;
+        const bool act = t < nl;
+        // sums over k: P B u_k, P A, P B cos, and the energy
+        T wx = T(0), wy = T(0), wz = T(0), sA = T(0), sB = T(0);
+        double e3 = 0.0;
+        T uxs = T(0), uys = T(0), uzs = T(0);
+        if (act) {
+            uxs = R.ux[t];
+            uys = R.uy[t];
+            uzs = R.uz[t];
+            const T Es = R.E[t];
+            const int rowj = (si * ns + R.sp[t]) * ns;
+            if (Es != T(0)) {
+                for (int k = ks; k < nl; k += KS) {
+                    if (k == t) continue;
+                    const T uxk = R.ux[k], uyk = R.uy[k], uzk = R.uz[k];
+                    const T cs = uxs * uxk + uys * uyk + uzs * uzk, Pp = Es * R.E[k];
+                    T A, Bc, eh;
+                    if (SYM) {
+                        const T dc = cs - own.cos0;
+                        eh = own.c * dc * dc;
+                        A = T(2) * eh;
+                        Bc = T(4) * own.c * dc;
+                    } else {
+                        const int sk = R.sp[k], ra = rowj + sk, rb = (si * ns + sk) * ns + R.sp[t];
+                        const SwTri<T> q1 = small ? B.tri[ra] : sw_tri_row<T>(P.tri + 4 * ra);
+                        const SwTri<T> q2 = small ? B.tri[rb] : sw_tri_row<T>(P.tri + 4 * rb);
+                        const T dc1 = cs - q1.cos0, dc2 = cs - q2.cos0;
+                        const T b1 = q1.c * dc1, b2 = q2.c * dc2;
+                        eh = b1 * dc1;
+                        A = eh + b2 * dc2;
+                        Bc = T(2) * (b1 + b2);
+                    }
+                    const T w = Pp * Bc;
+                    wx += w * uxk;
+                    wy += w * uyk;
+                    wz += w * uzk;
+                    sA += Pp * A;
+                    sB += w * cs;
+                    e3 += (double)(Pp * eh);
+                }
+            }
+        }
+#pragma unroll
+        for (int o = NB; o < LPA; o <<= 1) {
+            wx += __shfl_xor_sync(gmask, wx, o, LPA);
+            wy += __shfl_xor_sync(gmask, wy, o, LPA);
+            wz += __shfl_xor_sync(gmask, wz, o, LPA);
+            sA += __shfl_xor_sync(gmask, sA, o, LPA);
+            sB += __shfl_xor_sync(gmask, sB, o, LPA);
+        }
+        e += e3;
+        if (act && ks == 0) {
+            const T r = R.r[t], ir = T(1) / r;
+            const int mt = R.meta[t], sj = R.sp[t];
+            // the pair record of the lower-indexed atom's species order
+            const int pr = mt & 256 ? si * ns + sj : sj * ns + si;
+            T V2, dV2;
+            sw_two<T>(r, small ? B.pair[pr] : sw_pair_row<T>(P.tb + 8 * pr), V2, dV2);
+            e += 0.5 * (double)V2;
+            const double hx = 0.5 * (double)(dV2 * ir);
+            const T su = R.D[t] * sA - sB * ir;
+            const double dx = (double)R.x[t], dy = (double)R.y[t], dz = (double)R.z[t];
+            const double Dx = hx * dx + (double)(su * uxs + wx * ir), Dy = hx * dy + (double)(su * uys + wy * ir),
+                         Dz = hx * dz + (double)(su * uzs + wz * ir);
+            fx += Dx;
+            fy += Dy;
+            fz += Dz;
+            v[0] -= Dx * dx;
+            v[1] -= Dx * dy;
+            v[2] -= Dx * dz;
+            v[3] -= Dy * dx;
+            v[4] -= Dy * dy;
+            v[5] -= Dy * dz;
+            v[6] -= Dz * dx;
+            v[7] -= Dz * dy;
+            v[8] -= Dz * dz;
+            if (so.dudv) {  // U_i = 1/2 sum V2 + angles at i (engine/site_terms.py:179-300)
+                const size_t os = 3 * (size_t)(beg + (mt & 255));
+                so.dudv[os] = Dx;
+                so.dudv[os + 1] = Dy;
+                so.dudv[os + 2] = Dz;
+            }
+            // the force on neighbour j goes to j's own slot (j -> i)
+            const size_t o = 3 * (size_t)R.rev[t];
+            slot_G[o] = -Dx;
+            slot_G[o + 1] = -Dy;
+            slot_G[o + 2] = -Dz;
+        }
+    }
+    __syncwarp();
+    put_atom<LPA>(per_atom, f_local, so.e, i < S.n_atoms ? i : -1, e, v, fx, fy, fz, st.nok, st.bad);
 }
 
+// Everything one launch needs besides the shape.
+struct SwArgs {
+    SysView S;
+    const mbf_nlist *nl;
+    SwDev P;
+    double *slot_G, *f_local, *per_atom;
+    unsigned *live_mask;
+    ClearWords clr;
+    SiteOut so;
+};
+
 template <typename T, int MAXN, bool SYM, int LPA>
-static int sw_launch(const SysView &S, const mbf_nlist *nl, const SwDev &P, double *slot_G, double *f_local,
-                     double *per_atom, double *forces, int *err, const SiteOut &so, cudaStream_t st) {
+static int sw_launch(const SwArgs &A, cudaStream_t st) {
     constexpr int GPB = SwGeom<MAXN, LPA>::GPB, BLOCK = SwGeom<MAXN, LPA>::BLOCK;
-    int blocks = (S.n_atoms + GPB - 1) / GPB;
-    int g = persistent_grid(blocks, BLOCK, (const void *)sw_force<T, MAXN, SYM, LPA>);
-    PROF_BEGIN("sw_force", st);
-    sw_force<T, MAXN, SYM, LPA><<<g, BLOCK, 0, st>>>(S, nl->row_off, nl->nbr, nl->rev, P, slot_G, f_local, per_atom, err,
-                                                     so);
-    PROF_END("sw_force", st);
+    const int blocks = (A.S.n_atoms + GPB - 1) / GPB;
+    PROF_BEGIN("sw_center", st);
+    sw_center<T, MAXN, SYM, LPA><<<blocks, BLOCK, 0, st>>>(A.S, A.nl->row_off, A.nl->nbr, A.nl->rev, A.P, A.slot_G,
+                                                           A.f_local, A.per_atom, A.live_mask,
+                                                      (int)A.nl->n_slots, A.clr, A.so);
+    PROF_END("sw_center", st);
     MBF_CHECK_LAUNCH();
-    return MBF_OK;   // the eval's gather_reduce adds the slot forces
+    return MBF_OK;   // the eval's gather_live adds the slot forces
 }
 
 template <typename T, int MAXN, bool SYM>
-static int sw_lpa(int lpa, const SysView &S, const mbf_nlist *nl, const SwDev &P, double *slot_G, double *f_local,
-                  double *per_atom, double *forces, int *err, const SiteOut &so, cudaStream_t st) {
+static int sw_lpa(int lpa, const SwArgs &A, cudaStream_t st) {
     switch (lpa) {
-        case 4: return sw_launch<T, MAXN, SYM, 4>(S, nl, P, slot_G, f_local, per_atom, forces, err, so, st);
-        case 8: return sw_launch<T, MAXN, SYM, 8>(S, nl, P, slot_G, f_local, per_atom, forces, err, so, st);
-        case 16: return sw_launch<T, MAXN, SYM, 16>(S, nl, P, slot_G, f_local, per_atom, forces, err, so, st);
+        case 4: return sw_launch<T, MAXN, SYM, 4>(A, st);
+        case 8: return sw_launch<T, MAXN, SYM, 8>(A, st);
+        case 16: return sw_launch<T, MAXN, SYM, 16>(A, st);
         default: return MBF_ERR_ARGUMENT;
     }
 }
 
 template <typename T, bool SYM>
-static int sw_dispatch(int mr, int lpa, const SysView &S, const mbf_nlist *nl, const SwDev &P, double *slot_G,
-                       double *f_local, double *per_atom, double *forces, int *err, const SiteOut &so,
-                       cudaStream_t st) {
-    if (lpa <= 0) lpa = 8;
-    if (mr <= 32) return sw_lpa<T, 32, SYM>(lpa, S, nl, P, slot_G, f_local, per_atom, forces, err, so, st);
-    if (mr <= 64) return sw_lpa<T, 64, SYM>(lpa, S, nl, P, slot_G, f_local, per_atom, forces, err, so, st);
-    return sw_lpa<T, 128, SYM>(lpa, S, nl, P, slot_G, f_local, per_atom, forces, err, so, st);
+static int sw_dispatch(int mr, int lpa, const SwArgs &A, cudaStream_t st) {
+    if (mr <= 32) return sw_lpa<T, 32, SYM>(lpa, A, st);
+    if (mr <= 64) return sw_lpa<T, 64, SYM>(lpa, A, st);
+    return sw_lpa<T, 128, SYM>(lpa, A, st);
 }
+
+// The longest row sw_dispatch's choice for `mr` stages.
+static int sw_row_limit(int mr) { return mr <= 32 ? 32 : (mr <= 64 ? 64 : 128); }
 
 }  // namespace mbf
 
@@ -315,32 +371,37 @@ static int sw_eval(const mbf_system *sys, const mbf_nlist *nl, const mbf_sw_tabl
         if (cudaMemsetAsync(virial, 0, sizeof(double) * 9 * sys->n_struct, st) != cudaSuccess) return MBF_ERR_CUDA;
         return MBF_OK;
     }
+    if (nl->n_slots < 0 || nl->n_slots > 0x7fffff00LL) return MBF_ERR_ARGUMENT;
     if (nl->max_row > 128) return MBF_ERR_ROW_TOO_LONG;
-    SysView S = make_view(sys);
-    SwDev P;
-    P.ns = tab->ns;
-    P.tb = tab->tb;
-    P.leg = tab->leg;
-    P.tri = tab->tri;
-    P.rc = tab->r_cut;
+    // the per-structure completion counters live in a region of n_chunks
+    // words; every structure owns at least one chunk
+    if (plan->n_chunks <= 0 || sys->n_struct <= 0 || plan->n_chunks < sys->n_struct) return MBF_ERR_ARGUMENT;
+    SwArgs A;
+    A.S = make_view(sys);
+    A.nl = nl;
+    A.P.ns = tab->ns;
+    A.P.tb = tab->tb;
+    A.P.leg = tab->leg;
+    A.P.tri = tab->tri;
+    A.P.rc = tab->r_cut;
+    A.slot_G = ws_at<double>(workspace, L.slot);
+    A.f_local = ws_at<double>(workspace, L.f_local);
+    A.per_atom = ws_at<double>(workspace, L.per_atom);
+    A.live_mask = ws_at<unsigned>(workspace, L.atom_aux);
+    unsigned *sdone = ws_at<unsigned>(workspace, L.sdone);
     int *err = ws_at<int>(workspace, L.err);
-    if (cudaMemsetAsync(err, 0, ERR_CLEAR_BYTES, st) != cudaSuccess) return MBF_ERR_CUDA;
-    double *per_atom = ws_at<double>(workspace, L.per_atom);
-    double *f_local = ws_at<double>(workspace, L.f_local);
-    double *slot_G = ws_at<double>(workspace, L.slot);
-    double *partial = ws_at<double>(workspace, L.partial);
-    int mr = nl->max_row;
-    bool sym = tab->ns == 1;
+    A.clr = {(unsigned *)err, ERR_CLEAR_BYTES / 4, sdone, sys->n_struct};
+    A.so = so;
+    const int lpa = lanes_per_atom > 0 ? lanes_per_atom : 8, mr = nl->max_row;
     int rc;
     if (precision == MBF_FP64)
-        rc = sym ? sw_dispatch<double, true>(mr, lanes_per_atom, S, nl, P, slot_G, f_local, per_atom, forces, err, so, st)
-                 : sw_dispatch<double, false>(mr, lanes_per_atom, S, nl, P, slot_G, f_local, per_atom, forces, err, so, st);
+        rc = tab->ns == 1 ? sw_dispatch<double, true>(mr, lpa, A, st) : sw_dispatch<double, false>(mr, lpa, A, st);
     else
-        rc = sym ? sw_dispatch<float, true>(mr, lanes_per_atom, S, nl, P, slot_G, f_local, per_atom, forces, err, so, st)
-                 : sw_dispatch<float, false>(mr, lanes_per_atom, S, nl, P, slot_G, f_local, per_atom, forces, err, so, st);
+        rc = tab->ns == 1 ? sw_dispatch<float, true>(mr, lpa, A, st) : sw_dispatch<float, false>(mr, lpa, A, st);
     if (rc != MBF_OK) return rc;
-    return gather_reduce(sys->n_struct, sys->n_atoms, nl->row_off, slot_G, f_local, forces, per_atom, plan, partial,
-                         energy, virial, ws_at<unsigned>(workspace, L.sdone), st);
+    return gather_live(sys->n_struct, sys->n_atoms, nl->row_off, A.slot_G, A.live_mask, sw_row_limit(mr), err,
+                       A.f_local, forces, A.per_atom, plan, ws_at<double>(workspace, L.partial), energy, virial, sdone,
+                       st);
 }
 
 extern "C" int mbf_sw_eval(const mbf_system *sys, const mbf_nlist *nl, const mbf_sw_tables *tab,

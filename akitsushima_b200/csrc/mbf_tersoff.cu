@@ -12,25 +12,22 @@
 // Owner computes, no atomics: the lane group of centre i evaluates every
 // term of U_i, keeps the force on i and writes -dU_i/dr_x into x's own slot
 // (x -> i); atom a later sums its own row of slots (gather_reduce).
-#include "mbf_util.cuh"
+#include "mbf_rows.cuh"
 
 namespace mbf {
 
 // Lanes per atom (LPA) is a template parameter chosen by the host (the
-// autotuner); GPB lane groups per block keep the staged rows near 20 KB, so
-// the blocks of one SM end at different times and its last wave is short
-// (eight groups against sixteen, 32,768-atom SiC: 89 against 92 us).
+// autotuner): LPA lanes stage a centre's row, and LPA / 4 lanes share the
+// angle loops of a leg.  A block takes GPB centres (about 30 KB of staged legs
+// in float64) with at least two warps for the leg passes.
 template <int MAXN, int LPA> struct TeGeom {
     static constexpr int GPB = 256 / MAXN;
-    static constexpr int BLOCK = GPB * LPA;
-    // Resident threads per SM the kernel is compiled for, its register
-    // budget: 128 in float64, 96 in mixed precision.  SiC, 8 lanes, us at 384
-    // / 512 / 640 / 768 threads: 86 / 80 / 82 / 97 in float64; in mixed, at
-    // 512 / 640 / 768 / 1024: 72 / 64 / 64 / 70.
-    static constexpr int min_blocks(int size) {
-        const int b = (size == 8 ? 512 : 640) / BLOCK;
-        return b < 32 ? b : 32;
-    }
+    static constexpr int BLOCK = GPB * LPA < 64 ? 64 : GPB * LPA;
+    static constexpr int KS = LPA / 4;
+    // Resident threads per SM the kernel is compiled for (its registers):
+    // with the gather, 32,768-atom SiC float64 at 384 / 512 threads 66 / 62 us,
+    // 64,000-atom Si mixed at 512 / 640 55 / 53.
+    static constexpr int min_blocks(int size) { return (size == 8 ? 512 : 640) / BLOCK; }
 };
 
 struct TeDev {
@@ -109,7 +106,7 @@ __device__ __forceinline__ TeTri<T> te_tri_row(const double *__restrict__ t) {
 // species whether its records are all the same, valid and without lambda3
 // (one element, or the Tersoff-1989 mixing rules): then one record serves
 // every angle of the centre.
-constexpr int TE_SH = 4;
+constexpr int TE_SH = 3;
 template <typename T>
 struct TeTab {
     double tb[TE_SH * TE_SH * 10];
@@ -157,17 +154,18 @@ template <int MAXN> struct TeDist<double, MAXN> {};
 // One centre's legs (neighbours inside their pair's cutoff) in shared
 // memory, compacted in slot order: displacement, length and its inverse, the
 // cutoff function of the leg as a zeta term's third atom (record (i, k)) and
-// its derivative, the bond's zeta-gradient coefficient and pair part.
-// Groups of a warp lie 32 bytes apart modulo the banks' 128, so the lanes'
-// broadcast reads of different groups do not meet in a bank.
+// its derivative, the bond's zeta, then zeta-gradient coefficient, its pair
+// part and energy, and the leg's gradient dU_i/dr.  Rows lie 32 bytes apart
+// modulo the banks' 128.
 template <typename T, int MAXN>
 struct TeRow {
+    double gx[MAXN], gy[MAXN], gz[MAXN];
+    double e[MAXN];  // r^2, then the pair part's slope, at last the energy (in gx until then)
     T x[MAXN], y[MAXN], z[MAXN], r[MAXN], ir[MAXN], fk[MAXN], dfk[MAXN], coef[MAXN];
     TeDist<T, MAXN> dist;
-    double cx[MAXN];  // r^2 while staging
     int rev[MAXN];    // the leg's reverse slot
     int meta[MAXN];   // slot in the row | (i < j) << 8 | species << 9
-    char pad[32];
+    int beg, nl, si, pad[5];
 };
 
 template <int MAXN> __device__ __forceinline__ void te_put_r(TeRow<double, MAXN> &R, int q, double r) { R.r[q] = r; }
@@ -191,151 +189,124 @@ __device__ __forceinline__ void te_expo(T l3, T m, T u, T &ex, T &dex) {
     else dex = ex * m * RT<T>::pw(l3, m) * RT<T>::pw(u, m - T(1));
 }
 
-// Every term of a centre.  A group of LPA lanes takes one centre; in the
-// angle loops four legs at a time, each by LPA / 4 lanes that share the loop
-// over the third atom.  The bound is instruction issue and latency, not
-// memory (32,768-atom SiC, float64: 0.6 % of DRAM bandwidth), so the work is
-// cut to what the terms need: legs beyond their own pair's cutoff are dropped
-// before any loop, the cutoff functions are evaluated once per leg and not
-// per angle, one angle gives zeta_j's term k and zeta_k's term j one common
-// geometry, and g and g' take one reciprocal.  With the gather: 80 us (SiC
-// above), against 415 us for a zeta and a force kernel of a lane per bond
-// that evaluated the cutoff functions per angle, each gradient from both of
-// its bonds, and a bond order for the partner atom to read.
+// Every term of a block's centres.  The bound is instruction issue and
+// latency, not memory (32,768-atom SiC, float64: 0.6 % of DRAM bandwidth), so
+// the work is cut to what the terms need: legs beyond their own pair's cutoff
+// are dropped before any loop, the passes over legs run over the block's legs
+// as one list, the cutoff functions are evaluated once per leg and not per
+// angle, one angle gives zeta_j's term k and zeta_k's term j one common
+// geometry, and g and g' take one reciprocal.  Blocks are persistent: the
+// tables are loaded once, and the next row's loads are in flight during the
+// current one.  With the gather, SiC above: 62 us (80 with a lane group per
+// centre in every pass and one-shot blocks), against 415 us for a zeta and a
+// force kernel of a lane per bond that evaluated the cutoff functions per
+// angle, each gradient from both of its bonds, and a bond order for the
+// partner atom to read.
 template <typename T, int MAXN, int LPA>
 __global__ void __launch_bounds__(TeGeom<MAXN, LPA>::BLOCK, TeGeom<MAXN, LPA>::min_blocks(sizeof(T)))
     te_center(SysView S, const int *__restrict__ row_off, const int *__restrict__ nbr, const int *__restrict__ rev,
               TeDev P, double *__restrict__ slot_G, double *__restrict__ f_local, double *__restrict__ per_atom,
-              unsigned *__restrict__ live_mask, ClearWords clr, SiteOut so) {
-    constexpr int GPB = TeGeom<MAXN, LPA>::GPB;
-    constexpr int NB = 4, KS = LPA / NB;
-    static_assert(LPA >= NB && LPA < 32, "te_center: 4 to 16 lanes per centre");
+              unsigned *__restrict__ live_mask, int n_slots, ClearWords clr, SiteOut so) {
+    typedef TeGeom<MAXN, LPA> G;
+    constexpr int GPB = G::GPB, BLOCK = G::BLOCK, KS = G::KS;
     __shared__ TeRow<T, MAXN> rows[GPB];
     __shared__ TeTab<T> B;
+    __shared__ BlockLegs<GPB, MAXN> F;
+    const int g = threadIdx.x / LPA, sub = threadIdx.x & (LPA - 1);
+    RowHead next;
+    next.load(S, row_off, g < GPB ? blockIdx.x * GPB + g : S.n_atoms);
     clr.run();
     te_load_tab<T>(P, B);
-    const int sub = threadIdx.x & (LPA - 1), gl = threadIdx.x & 31 & ~(LPA - 1);
-    const unsigned gones = (1u << LPA) - 1u, gmask = gones << gl;
-    const int lt = sub & (NB - 1), ks = sub / NB;
-    TeRow<T, MAXN> &R = rows[threadIdx.x / LPA];
     const int ns = P.ns;
     const bool small = ns <= TE_SH;
     const double *const tb = small ? B.tb : P.tb;
     auto tri_row = [&](int q) { return small ? B.tri[q] : te_tri_row<T>(P.tri + 8 * (size_t)q); };
-    const int i = blockIdx.x * GPB + threadIdx.x / LPA;
-    double fx = 0, fy = 0, fz = 0, e = 0;
-    double v[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-    int nl = 0, nok = 0, beg = 0, n = 0, si = 0;
-    if (i < S.n_atoms) {
-        beg = row_off[i];
-        n = row_off[i + 1] - beg;
-        if (n > MAXN) n = 0;  // reported by the gather, which sees every row
-        si = S.types[i];
+    TeRow<T, MAXN> &mine = rows[g < GPB ? g : 0];
+    next.slots<LPA>(nbr, rev, n_slots, ns, MAXN);
+    for (int base = blockIdx.x * GPB; base < S.n_atoms; base += gridDim.x * GPB) {  // uniform over the block
+    const int i = g < GPB ? base + g : S.n_atoms;
+    const RowHead head = next;
+    const int i_next = g < GPB ? i + gridDim.x * GPB : S.n_atoms;
+    next.load(S, row_off, i_next);
+    const RowStage st = stage_row<LPA>(
+        S, head, nbr, rev, n_slots, ns, P.rc, i, live_mask, so.vec,
+        [&](int a, int b) { return small ? B.reach2[a * ns + b] : te_reach2(P, a, b); },
+        [&](int q, int s, int j, int sj, int rs, double dx, double dy, double dz, double r2) {
+            mine.x[q] = (T)dx;
+            mine.y[q] = (T)dy;
+            mine.z[q] = (T)dz;
+            mine.e[q] = r2;
+            mine.rev[q] = rs;
+            mine.meta[q] = s | (i < j ? 1 << 8 : 0) | sj << 9;
+        });
+    if (sub == 0 && g < GPB) {
+        mine.beg = st.beg;
+        mine.nl = st.nl;
+        mine.si = st.si;
     }
-    // the legs, compacted in slot order; every loop has the same trip count
-    // over a group
-    if (n > 0) {
-        const double *cell = cell_of(S, i);
-        const double xi = S.pos[3 * (size_t)i], yi = S.pos[3 * (size_t)i + 1], zi = S.pos[3 * (size_t)i + 2];
-        const double rc2 = P.rc * P.rc;
-        unsigned word = 0;
-        for (int s0 = 0; s0 < n; s0 += LPA) {
-            const int s = s0 + sub;
-            bool ok = false, lv = false;
-            int j = 0, sj = 0, rs = 0;
-            double dx = 0, dy = 0, dz = 0, r2 = 0;
-            if (s < n) {
-                j = nbr[beg + s];
-                rs = rev[beg + s];
-                sj = S.types[j];
-                mic_exact(cell, S.pos[3 * (size_t)j] - xi, S.pos[3 * (size_t)j + 1] - yi, S.pos[3 * (size_t)j + 2] - zi,
-                          dx, dy, dz);
-                r2 = dx * dx + dy * dy + dz * dz;
-                ok = r2 < rc2 && r2 > 1e-24;
-                lv = ok && r2 <= (small ? B.reach2[si * ns + sj] : te_reach2(P, si, sj));
-                if (so.vec) {
-                    const size_t os = 3 * (size_t)(beg + s);
-                    so.vec[os] = dx;
-                    so.vec[os + 1] = dy;
-                    so.vec[os + 2] = dz;
-                }
-            }
-            const unsigned b = (__ballot_sync(gmask, lv) >> gl) & gones;
-            nok += __popc((__ballot_sync(gmask, ok) >> gl) & gones);
-            if (lv) {
-                const int q = nl + __popc(b & ((1u << sub) - 1u));
-                R.x[q] = (T)dx;
-                R.y[q] = (T)dy;
-                R.z[q] = (T)dz;
-                R.cx[q] = r2;
-                R.rev[q] = rs;
-                R.meta[q] = s | (i < j ? 1 << 8 : 0) | sj << 9;
-            }
-            nl += __popc(b);
-            word |= b << (s0 & 31);
-            if (((s0 + LPA) & 31) == 0 || s0 + LPA >= n) {
-                if (sub == 0) live_mask[4 * (size_t)i + (s0 >> 5)] = word;
-                word = 0;
-            }
-        }
-    }
-    __syncwarp(gmask);
-    for (int q = sub; q < nl; q += LPA) {
-        const double r = sqrt(R.cx[q]);
-        const double *tk = tb + 10 * (si * ns + (R.meta[q] >> 9));
+    const int total = flatten_legs<GPB, MAXN, LPA>(F, g, sub, st.nl);
+    // a lane per leg: length and cutoff function
+    for (int q = threadIdx.x; q < total; q += BLOCK) {
+        const int m = F.map[q], t = m & (MAXN - 1);
+        TeRow<T, MAXN> &R = rows[m / MAXN];
+        const double r = leg_root<T>(R.e[t]);
+        const double *tk = tb + 10 * (R.si * ns + (R.meta[t] >> 9));
         T fk = T(0), dfk = T(0);
         if (tk[0] != 0.0) te_cut<T>((T)r, (T)tk[5], (T)tk[6], fk, dfk);
-        te_put_r(R, q, r);
-        R.ir[q] = T(1) / (T)r;
-        R.fk[q] = fk;
-        R.dfk[q] = dfk;
+        te_put_r(R, t, r);
+        R.ir[t] = T(1) / (T)r;
+        R.fk[t] = fk;
+        R.dfk[t] = dfk;
     }
-    __syncwarp(gmask);
-    const bool plain = small && B.plain[si];
-    const TeTri<T> own = plain ? B.tri[si * ns * ns] : TeTri<T>();
-    // zeta of every bond
-    for (int t0 = 0; t0 < nl; t0 += NB) {
-        const int t = t0 + lt;
+    __syncthreads();
+    next.slots<LPA>(nbr, rev, n_slots, ns, MAXN);
+    // KS lanes per leg: zeta of the bond
+    const int ks = threadIdx.x & (KS - 1);
+    const unsigned share = ((1u << KS) - 1u) << (threadIdx.x & 31 & ~(KS - 1));
+    for (int q = threadIdx.x / KS; q < total; q += BLOCK / KS) {
+        const int m = F.map[q], t = m & (MAXN - 1);
+        TeRow<T, MAXN> &R = rows[m / MAXN];
+        const int nl = R.nl, si = R.si;
         T zeta = T(0);
-        if (t < nl) {
-            const T xs = R.x[t], ys = R.y[t], zs = R.z[t], irs = R.ir[t];
-            if (plain) {
-                for (int k = ks; k < nl; k += KS) {
-                    const T fk = R.fk[k];
-                    if (k == t || fk == T(0)) continue;
-                    const T cs = (xs * R.x[k] + ys * R.y[k] + zs * R.z[k]) * (irs * R.ir[k]);
-                    zeta += own.gam * fk * te_g<T>(own.c2, own.d2, own.h - cs);
-                }
-            } else {
-                const T rs = R.r[t];
-                const int row = (si * ns + (R.meta[t] >> 9)) * ns;
-                for (int k = ks; k < nl; k += KS) {
-                    const T fk = R.fk[k];
-                    if (k == t || fk == T(0)) continue;
-                    const TeTri<T> q = tri_row(row + (R.meta[k] >> 9));
-                    if (q.valid == T(0)) continue;
-                    const T cs = (xs * R.x[k] + ys * R.y[k] + zs * R.z[k]) * (irs * R.ir[k]);
-                    T ex, dex;
-                    te_expo<T>(q.l3, q.m, rs - R.r[k], ex, dex);
-                    zeta += q.gam * fk * te_g<T>(q.c2, q.d2, q.h - cs) * ex;
-                }
+        const T xs = R.x[t], ys = R.y[t], zs = R.z[t], irs = R.ir[t];
+        if (small && B.plain[si]) {
+            const TeTri<T> own = B.tri[si * ns * ns];
+            for (int k = ks; k < nl; k += KS) {
+                const T fk = R.fk[k];
+                if (k == t || fk == T(0)) continue;
+                const T cs = (xs * R.x[k] + ys * R.y[k] + zs * R.z[k]) * (irs * R.ir[k]);
+                zeta += own.gam * fk * te_g<T>(own.c2, own.d2, own.h - cs);
+            }
+        } else {
+            const T rs = R.r[t];
+            const int row = (si * ns + (R.meta[t] >> 9)) * ns;
+            for (int k = ks; k < nl; k += KS) {
+                const T fk = R.fk[k];
+                if (k == t || fk == T(0)) continue;
+                const TeTri<T> w = tri_row(row + (R.meta[k] >> 9));
+                if (w.valid == T(0)) continue;
+                const T cs = (xs * R.x[k] + ys * R.y[k] + zs * R.z[k]) * (irs * R.ir[k]);
+                T ex, dex;
+                te_expo<T>(w.l3, w.m, rs - R.r[k], ex, dex);
+                zeta += w.gam * fk * te_g<T>(w.c2, w.d2, w.h - cs) * ex;
             }
         }
-#pragma unroll
-        for (int o = NB; o < LPA; o <<= 1) zeta += __shfl_xor_sync(gmask, zeta, o, LPA);
-        if (t < nl && ks == 0) R.coef[t] = zeta;
+        zeta = share_sum<KS>(share, zeta);
+        if (ks == 0) R.coef[t] = zeta;
     }
-    __syncwarp(gmask);
-    // the bonds, one lane each: bond order, energy, pair part and the
-    // coefficient of zeta's gradient; the two-body part is per bond, not per
-    // angle, and float64 in both precisions
-    for (int t = sub; t < nl; t += LPA) {
-        const int mt = R.meta[t], sj = mt >> 9;
+    __syncthreads();
+    // a lane per bond: bond order, energy, pair part and the coefficient of
+    // zeta's gradient; the two-body part is per bond, not per angle, and
+    // float64 in both precisions
+    for (int q = threadIdx.x; q < total; q += BLOCK) {
+        const int m = F.map[q], t = m & (MAXN - 1);
+        TeRow<T, MAXN> &R = rows[m / MAXN];
+        const int mt = R.meta[t], sj = mt >> 9, si = R.si;
         const double *tij = tb + 10 * (si * ns + sj);
         const double *tp = mt & 256 ? tij : tb + 10 * (sj * ns + si);
         const double z = (double)R.coef[t];
         T coef = T(0);
-        double cx = 0.0;
+        double cx = 0.0, e = 0.0;
         if (tp[0] != 0.0) {
             const double r = te_get_r(R, t);
             double fc, dfc;
@@ -359,106 +330,92 @@ __global__ void __launch_bounds__(TeGeom<MAXN, LPA>::BLOCK, TeGeom<MAXN, LPA>::m
                 const double l1 = tp[3], l2 = tp[4];
                 const double fr = tp[1] * clamped_exp<double>(-l1 * r);
                 const double fa = -tp[2] * clamped_exp<double>(-l2 * r);
-                e += 0.5 * (fc * (fr + b * fa));
+                e = 0.5 * (fc * (fr + b * fa));
                 cx = 0.5 * (dfc * (fr + b * fa) + fc * (-l1 * fr - l2 * b * fa)) / r;
                 if (fabs(db) > 1e-30) coef = (T)(0.5 * fc * fa * db);
             }
         }
         R.coef[t] = coef;
-        R.cx[t] = cx;
+        R.e[t] = cx;
+        R.gx[t] = e;
     }
-    __syncwarp(gmask);
-    // dU_i / dr of every leg: t as the bond partner of zeta_t's terms and as
-    // the third atom of the other bonds' terms.  With c = cos(t, k), both
-    // parts point along d_k and d_t:
+    __syncthreads();
+    // dU_i / dr of every leg, KS lanes each: t as the bond partner of zeta_t's
+    // terms and as the third atom of the other bonds' terms.  With c =
+    // cos(t, k), both parts point along d_k and d_t:
     //   d = A (d_k / (r_t r_k) - c d_t / r_t^2) + B d_t
-    for (int t0 = 0; t0 < nl; t0 += NB) {
-        const int t = t0 + lt;
-        const bool act = t < nl;
+    for (int q = threadIdx.x / KS; q < total; q += BLOCK / KS) {
+        const int m = F.map[q], t = m & (MAXN - 1);
+        TeRow<T, MAXN> &R = rows[m / MAXN];
+        const int nl = R.nl, si = R.si;
         double gx = 0, gy = 0, gz = 0, gs = 0;
-        T xs = T(0), ys = T(0), zs = T(0);
-        if (act) {
-            xs = R.x[t];
-            ys = R.y[t];
-            zs = R.z[t];
-            const T irs = R.ir[t], ct = R.coef[t], ft = R.fk[t], dft = R.dfk[t], ir2 = irs * irs;
-            auto add = [&](T A, T B_, T c, T ii, T xk, T yk, T zk) {
-                const T Ai = A * ii;
-                gx += (double)(Ai * xk);
-                gy += (double)(Ai * yk);
-                gz += (double)(Ai * zk);
-                gs += (double)(B_ - A * c * ir2);
-            };
-            if (plain) {
-                for (int k = ks; k < nl; k += KS) {
-                    const T ck = R.coef[k], w = ct * R.fk[k] + ck * ft;
-                    if (k == t || (w == T(0) && ck == T(0))) continue;
-                    const T xk = R.x[k], yk = R.y[k], zk = R.z[k], ii = irs * R.ir[k];
-                    const T c = (xs * xk + ys * yk + zs * zk) * ii;
-                    T g, dg;
-                    te_gdg<T>(own.c2, own.d2, own.h - c, g, dg);
-                    add(own.gam * w * dg, own.gam * ck * dft * g * irs, c, ii, xk, yk, zk);
-                }
-            } else {
-                const T rs = R.r[t];
-                const int st = R.meta[t] >> 9;
-                for (int k = ks; k < nl; k += KS) {
-                    const T fk = R.fk[k], ck = R.coef[k];
-                    const bool as_j = ct != T(0) && fk != T(0), as_k = ck != T(0) && ft != T(0);
-                    if (k == t || !(as_j || as_k)) continue;
-                    const int sk = R.meta[k] >> 9;
-                    const T xk = R.x[k], yk = R.y[k], zk = R.z[k], ii = irs * R.ir[k];
-                    const T c = (xs * xk + ys * yk + zs * zk) * ii;
-                    T A = T(0), B_ = T(0), g, dg, ex, dex;
-                    if (as_j) {
-                        const TeTri<T> q = tri_row((si * ns + st) * ns + sk);
-                        if (q.valid != T(0)) {
-                            te_gdg<T>(q.c2, q.d2, q.h - c, g, dg);
-                            te_expo<T>(q.l3, q.m, rs - R.r[k], ex, dex);
-                            const T w = ct * q.gam * fk;
-                            A += w * dg * ex;
-                            B_ += w * g * dex * irs;
-                        }
+        const T xs = R.x[t], ys = R.y[t], zs = R.z[t];
+        const T irs = R.ir[t], ct = R.coef[t], ft = R.fk[t], dft = R.dfk[t], ir2 = irs * irs;
+        auto add = [&](T A, T B_, T c, T ii, T xk, T yk, T zk) {
+            const T Ai = A * ii;
+            gx += (double)(Ai * xk);
+            gy += (double)(Ai * yk);
+            gz += (double)(Ai * zk);
+            gs += (double)(B_ - A * c * ir2);
+        };
+        if (small && B.plain[si]) {
+            const TeTri<T> own = B.tri[si * ns * ns];
+            for (int k = ks; k < nl; k += KS) {
+                const T ck = R.coef[k], w = ct * R.fk[k] + ck * ft;
+                if (k == t || (w == T(0) && ck == T(0))) continue;
+                const T xk = R.x[k], yk = R.y[k], zk = R.z[k], ii = irs * R.ir[k];
+                const T c = (xs * xk + ys * yk + zs * zk) * ii;
+                T gg, dg;
+                te_gdg<T>(own.c2, own.d2, own.h - c, gg, dg);
+                add(own.gam * w * dg, own.gam * ck * dft * gg * irs, c, ii, xk, yk, zk);
+            }
+        } else {
+            const T rs = R.r[t];
+            const int s_t = R.meta[t] >> 9;
+            for (int k = ks; k < nl; k += KS) {
+                const T fk = R.fk[k], ck = R.coef[k];
+                const bool as_j = ct != T(0) && fk != T(0), as_k = ck != T(0) && ft != T(0);
+                if (k == t || !(as_j || as_k)) continue;
+                const int s_k = R.meta[k] >> 9;
+                const T xk = R.x[k], yk = R.y[k], zk = R.z[k], ii = irs * R.ir[k];
+                const T c = (xs * xk + ys * yk + zs * zk) * ii;
+                T A = T(0), B_ = T(0), gg, dg, ex, dex;
+                if (as_j) {
+                    const TeTri<T> u = tri_row((si * ns + s_t) * ns + s_k);
+                    if (u.valid != T(0)) {
+                        te_gdg<T>(u.c2, u.d2, u.h - c, gg, dg);
+                        te_expo<T>(u.l3, u.m, rs - R.r[k], ex, dex);
+                        const T w = ct * u.gam * fk;
+                        A += w * dg * ex;
+                        B_ += w * gg * dex * irs;
                     }
-                    if (as_k) {
-                        const TeTri<T> q = tri_row((si * ns + sk) * ns + st);
-                        if (q.valid != T(0)) {
-                            te_gdg<T>(q.c2, q.d2, q.h - c, g, dg);
-                            te_expo<T>(q.l3, q.m, R.r[k] - rs, ex, dex);
-                            const T w = ck * q.gam;
-                            A += w * ft * dg * ex;
-                            B_ += w * g * (dft * ex - ft * dex) * irs;
-                        }
-                    }
-                    add(A, B_, c, ii, xk, yk, zk);
                 }
+                if (as_k) {
+                    const TeTri<T> u = tri_row((si * ns + s_k) * ns + s_t);
+                    if (u.valid != T(0)) {
+                        te_gdg<T>(u.c2, u.d2, u.h - c, gg, dg);
+                        te_expo<T>(u.l3, u.m, R.r[k] - rs, ex, dex);
+                        const T w = ck * u.gam;
+                        A += w * ft * dg * ex;
+                        B_ += w * gg * (dft * ex - ft * dex) * irs;
+                    }
+                }
+                add(A, B_, c, ii, xk, yk, zk);
             }
         }
-#pragma unroll
-        for (int o = NB; o < LPA; o <<= 1) {
-            gx += __shfl_xor_sync(gmask, gx, o, LPA);
-            gy += __shfl_xor_sync(gmask, gy, o, LPA);
-            gz += __shfl_xor_sync(gmask, gz, o, LPA);
-            gs += __shfl_xor_sync(gmask, gs, o, LPA);
-        }
-        if (act && ks == 0) {
-            const double dx = (double)xs, dy = (double)ys, dz = (double)zs;
-            gs += R.cx[t];
-            const double Dx = gx + gs * dx, Dy = gy + gs * dy, Dz = gz + gs * dz;
-            fx += Dx;
-            fy += Dy;
-            fz += Dz;
-            v[0] -= Dx * dx;
-            v[1] -= Dx * dy;
-            v[2] -= Dx * dz;
-            v[3] -= Dy * dx;
-            v[4] -= Dy * dy;
-            v[5] -= Dy * dz;
-            v[6] -= Dz * dx;
-            v[7] -= Dz * dy;
-            v[8] -= Dz * dz;
+        gx = share_sum<KS>(share, gx);
+        gy = share_sum<KS>(share, gy);
+        gz = share_sum<KS>(share, gz);
+        gs = share_sum<KS>(share, gs);
+        if (ks == 0) {
+            gs += R.e[t];
+            R.e[t] = R.gx[t];
+            const double Dx = gx + gs * (double)xs, Dy = gy + gs * (double)ys, Dz = gz + gs * (double)zs;
+            R.gx[t] = Dx;
+            R.gy[t] = Dy;
+            R.gz[t] = Dz;
             if (so.dudv) {  // engine/site_terms.py:312-437: own bond order
-                const size_t os = 3 * (size_t)(beg + (R.meta[t] & 255));
+                const size_t os = 3 * (size_t)(R.beg + (R.meta[t] & 255));
                 so.dudv[os] = Dx;
                 so.dudv[os + 1] = Dy;
                 so.dudv[os + 2] = Dz;
@@ -470,24 +427,8 @@ __global__ void __launch_bounds__(TeGeom<MAXN, LPA>::BLOCK, TeGeom<MAXN, LPA>::m
             slot_G[o + 2] = -Dz;
         }
     }
-    __syncwarp();
-    // f and v: only the first lane of each leg holds sums
-    fx = group_sum<NB>(fx);
-    fy = group_sum<NB>(fy);
-    fz = group_sum<NB>(fz);
-    e = group_sum<LPA>(e);
-#pragma unroll
-    for (int q = 0; q < 9; ++q) v[q] = group_sum<NB>(v[q]);
-    if (sub == 0 && i < S.n_atoms) {
-        if (so.e) so.e[i] = e;
-        f_local[3 * (size_t)i] = fx;
-        f_local[3 * (size_t)i + 1] = fy;
-        f_local[3 * (size_t)i + 2] = fz;
-        double *pa = per_atom + (size_t)i * ATOM_ACC;
-        pa[0] = e;
-#pragma unroll
-        for (int q = 0; q < 9; ++q) pa[1 + q] = v[q];
-        pa[10] = (double)nok;
+    __syncthreads();
+    sum_legs<LPA>(mine, st, g < GPB && i < S.n_atoms ? i : -1, per_atom, f_local, so.e);
     }
 }
 
@@ -505,10 +446,11 @@ struct TeArgs {
 template <typename T, int MAXN, int LPA>
 static int te_launch(const TeArgs &A, cudaStream_t st) {
     constexpr int GPB = TeGeom<MAXN, LPA>::GPB, BLOCK = TeGeom<MAXN, LPA>::BLOCK;
-    const int blocks = (A.S.n_atoms + GPB - 1) / GPB;
+    const int blocks = persistent_grid((A.S.n_atoms + GPB - 1) / GPB, BLOCK, (const void *)te_center<T, MAXN, LPA>);
     PROF_BEGIN("te_center", st);
     te_center<T, MAXN, LPA><<<blocks, BLOCK, 0, st>>>(A.S, A.nl->row_off, A.nl->nbr, A.nl->rev, A.P, A.slot_G, A.f_local,
-                                                      A.per_atom, A.live_mask, A.clr, A.so);
+                                                      A.per_atom, A.live_mask,
+                                                      (int)A.nl->n_slots, A.clr, A.so);
     PROF_END("te_center", st);
     MBF_CHECK_LAUNCH();
     return MBF_OK;   // the eval's gather_reduce adds the slot forces
@@ -553,6 +495,7 @@ static int tersoff_eval(const mbf_system *sys, const mbf_nlist *nl, const mbf_te
         if (cudaMemsetAsync(virial, 0, sizeof(double) * 9 * sys->n_struct, st) != cudaSuccess) return MBF_ERR_CUDA;
         return MBF_OK;
     }
+    if (nl->n_slots < 0 || nl->n_slots > 0x7fffff00LL) return MBF_ERR_ARGUMENT;
     if (nl->max_row > 128) return MBF_ERR_ROW_TOO_LONG;
     // the per-structure completion counters live in a region of n_chunks
     // words; every structure owns at least one chunk

@@ -121,82 +121,14 @@ int exclusive_scan(const int *in, int *out, int n, int *ws, cudaStream_t st) {
 // ---- force gather and per-structure sums -----------------------------------
 
 // Gather the three-body forces the centres left on atom a: every centre x
-// wrote the force its angles put on a into a's own slot (a -> x), so the
-// row is read contiguously, 8 lanes per atom; fused with the per-structure
-// sums (ChunkSums): a block per chunk of the reduction plan, each group also
-// adding its atom's record (entries sub and sub + 8), the next atom's row
-// bounds loaded one iteration ahead.
-template <int NT>
-__global__ void __launch_bounds__(NT) gather_reduce_rows(const int *__restrict__ row_off,
-                                                         const double *__restrict__ G,
-                                                         const double *__restrict__ f_local,
-                                                         double *__restrict__ forces, ChunkSums cs) {
-    constexpr int LPA = 8, NG = NT / LPA;
-    const int c = blockIdx.x;
-    const int s = cs.chunk[3 * c], a0 = cs.chunk[3 * c + 1], a1 = cs.chunk[3 * c + 2];
-    const int sub = threadIdx.x & (LPA - 1), grp = threadIdx.x / LPA;
-    double r0 = 0.0, r1 = 0.0;
-    int nb = 0, ne = 0;
-    if (a0 + grp < a1) {
-        nb = row_off[a0 + grp];
-        ne = row_off[a0 + grp + 1];
-    }
-    for (int base = a0; base < a1; base += NG) {  // uniform over the block
-        const int a = base + grp, beg = nb, end = ne;
-        if (a + NG < a1) {
-            nb = row_off[a + NG];
-            ne = row_off[a + NG + 1];
-        }
-        double fx = 0, fy = 0, fz = 0;
-        if (a < a1) {
-            // each slot force is read once: streaming (evict-first) loads
-#pragma unroll 4
-            for (int q = beg + sub; q < end; q += LPA) {
-                fx += __ldcs(G + 3 * (size_t)q);
-                fy += __ldcs(G + 3 * (size_t)q + 1);
-                fz += __ldcs(G + 3 * (size_t)q + 2);
-            }
-            const double *pa = cs.per_atom + (size_t)a * ATOM_ACC;
-            r0 += pa[sub];
-            if (sub < ATOM_ACC - LPA) r1 += pa[LPA + sub];
-        }
-        fx = group_sum<LPA>(fx);
-        fy = group_sum<LPA>(fy);
-        fz = group_sum<LPA>(fz);
-        if (sub == 0 && a < a1) {
-            forces[3 * (size_t)a] = f_local[3 * (size_t)a] + fx;
-            forces[3 * (size_t)a + 1] = f_local[3 * (size_t)a + 1] + fy;
-            forces[3 * (size_t)a + 2] = f_local[3 * (size_t)a + 2] + fz;
-        }
-    }
-    chunk_sums_finish<NT>(cs, c, s, r0, r1);
-}
-
-int gather_reduce(int n_struct, int n_atoms, const int *row_off, const double *G, const double *f_local,
-                  double *forces, const double *per_atom, const mbf_reduce_plan *plan, double *partial,
-                  double *energy, double *virial, unsigned *sdone, cudaStream_t st) {
-    // the completion counters live in a region of n_chunks words; every
-    // structure owns at least one chunk
-    if (plan->n_chunks <= 0 || n_struct <= 0 || plan->n_chunks < n_struct || !sdone) return MBF_ERR_ARGUMENT;
-    if (cudaMemsetAsync(sdone, 0, sizeof(unsigned) * (size_t)n_struct, st) != cudaSuccess) return MBF_ERR_CUDA;
-    ChunkSums cs = {plan->chunk, plan->chunk_first, per_atom, partial, energy, virial, sdone};
-    PROF_BEGIN("gather_reduce", st);
-    int nt = chunk_block(n_atoms, plan->n_chunks);
-    if (nt == 128)
-        gather_reduce_rows<128><<<plan->n_chunks, 128, 0, st>>>(row_off, G, f_local, forces, cs);
-    else if (nt == 256)
-        gather_reduce_rows<256><<<plan->n_chunks, 256, 0, st>>>(row_off, G, f_local, forces, cs);
-    else
-        gather_reduce_rows<512><<<plan->n_chunks, 512, 0, st>>>(row_off, G, f_local, forces, cs);
-    PROF_END("gather_reduce", st);
-    MBF_CHECK_LAUNCH();
-    return MBF_OK;
-}
-
-// gather_reduce_rows over the slots whose live bit is set: a list radius of
-// cutoff + skin holds two to three times the slots that carry a force
-// (32,768-atom SiC: 15.5 listed, 4 live), and the others are neither
-// written nor read.  Up to four slots a lane are in flight at once.
+// wrote the force its terms put on a into a's own slot (a -> x), so the row
+// is read contiguously, 8 lanes per atom; fused with the per-structure sums
+// (ChunkSums): a block per chunk of the reduction plan, each group also
+// adding its atom's record (entries sub and sub + 8).  Only the slots whose
+// live bit is set are read: a list radius of cutoff + skin holds two to three
+// times the slots that carry a force (32,768-atom SiC: 15.5 listed, 6 live),
+// and the others are never written.  Bound by latency: up to four slots a
+// lane are in flight at once.
 template <int NT>
 __global__ void __launch_bounds__(NT) gather_live_rows(const int *__restrict__ row_off, const double *__restrict__ G,
                                                        const uint4 *__restrict__ live_mask, int row_limit,
@@ -207,24 +139,33 @@ __global__ void __launch_bounds__(NT) gather_live_rows(const int *__restrict__ r
     const int s = cs.chunk[3 * c], a0 = cs.chunk[3 * c + 1], a1 = cs.chunk[3 * c + 2];
     const int sub = threadIdx.x & (LPA - 1), grp = threadIdx.x / LPA;
     double r0 = 0.0, r1 = 0.0;
+    // the next atom's bounds and mask one iteration ahead: a slot's load then
+    // waits on nothing
     int nb = 0, ne = 0;
+    uint4 nm = make_uint4(0u, 0u, 0u, 0u);
     if (a0 + grp < a1) {
         nb = row_off[a0 + grp];
         ne = row_off[a0 + grp + 1];
+        nm = live_mask[a0 + grp];
     }
     for (int base = a0; base < a1; base += NG) {  // uniform over the block
         const int a = base + grp, beg = nb, n = ne - nb;
+        const uint4 m4 = nm;
         if (a + NG < a1) {
             nb = row_off[a + NG];
             ne = row_off[a + NG + 1];
+            nm = live_mask[a + NG];
         }
         double fx = 0, fy = 0, fz = 0, fl = 0;
         if (a < a1) {
-            const uint4 m4 = live_mask[a];
             const double *pa = cs.per_atom + (size_t)a * ATOM_ACC;
             const double ra = pa[sub];
-            const double rb = sub < ATOM_ACC - LPA ? pa[LPA + sub] : 0.0;
+            double rb = sub < ATOM_ACC - LPA ? pa[LPA + sub] : 0.0;
             if (sub < 3) fl = f_local[3 * (size_t)a + sub];
+            if (sub == 10 - LPA && rb < 0.0) {  // a bad index in the row (put_atom)
+                atomicOr(err, MBF_DEV_BAD_INDEX);
+                rb = 0.0;
+            }
             if (n > row_limit) {
                 if (sub == 0) atomicOr(err, MBF_DEV_ROW_TOO_LONG);
             } else {
