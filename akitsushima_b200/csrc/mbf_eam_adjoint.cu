@@ -20,24 +20,31 @@
 // one evaluation of F; with c1 = gE F' + F'' D_t rho-bar and c2 = F', a
 // density parameter's site value is c1 d(rho)/dtheta + c2 d(D_t rho)/dtheta.
 // Density and pair functions are built from decays
-// g(r; r_e, exponent, shift), each differentiated in its own three
-// parameters only; an element's eight parameters and the cross pair's
+// g(r; r_e, exponent, shift), whose parameter derivatives and tangents are
+// written out from d ln g; an element's eight parameters and the cross pair's
 // (f_a, u_a, f_b, u_b) dependence are chained by hand from those.
 //
-// Sites of atom i (W = 12 + 21 ns):
-//   0..11               rho_e, rho_s, Fn0..Fn3, F0..F3, eta, F_e of row F_f[s_i]
-//                       (columns 2, 3, 10..19)
-//   12 + 4 s + 0..3     r_e, f_e, beta, lambda of row rho_f[s] (columns 0, 1, 5, 9)
-//   12 + 4 ns + 17 s    the pair row phi_f[s_i, s]: 0..7 the earlier species'
-//                       r_e, f_e, alpha, beta, A, B, kappa, lambda (columns 0,
-//                       1, 4..9), 8..15 the later species' (columns 20, 21,
-//                       24..29, cross rows only), 16 the factor k (column 42)
-// Columns 40, 41 (switch radius and width) are not differentiated: the
-// cutoff is fixed during a fit.  The gradient is with respect to the rows
-// the generic Zhou evaluation reads (rho_f, F_f, phi_f); the fused path
-// reads the same element parameters from the density rows, which the table
-// builders fill identically.  Sites are reduced onto the entries in a fixed
-// order: deterministic.
+// Passes: rho-bar and its tangent (8 lanes per atom), which also marks and
+// counts the live pairs above the diagonal by unordered species pair; the
+// embedding sites (a thread per atom); a scan and a compaction into one list
+// per species pair; one pass over each list with the site sums in registers;
+// a final reduction onto the table entries.
+//
+// Sites of a species pair (a, b), a <= b (PAIR_SITES values):
+//   0..7    the pair row phi_f[a, b]: the earlier species' r_e, f_e, alpha,
+//           beta, A, B, kappa, lambda (columns 0, 1, 4..9)
+//   8..15   the later species' (columns 20, 21, 24..29; a < b only)
+//   16      the factor k (column 42; a < b only)
+//   17..20  r_e, f_e, beta, lambda of row rho_f[b] (columns 0, 1, 5, 9), from
+//           the a atom's density; for a = b, from both atoms'
+//   21..24  the same of row rho_f[a], from the b atom's density (a < b only)
+// and 12 per centre species: rho_e, rho_s, Fn0..Fn3, F0..F3, eta, F_e of row
+// F_f[s] (columns 2, 3, 10..19).  Columns 40, 41 (switch radius and width) are
+// not differentiated: the cutoff is fixed during a fit.  The gradient is with
+// respect to the rows the generic Zhou evaluation reads (rho_f, F_f, phi_f);
+// the fused path reads the same element parameters from the density rows,
+// which the table builders fill identically.  Sites are reduced onto the
+// entries in a fixed order: deterministic.
 #include "mbf_hd.cuh"
 
 namespace mbf {
@@ -52,33 +59,47 @@ struct EamAdjTab {
     double rc;
 };
 
-// g = exp(-expo (x - 1)) / (1 + (x - shift)^20), x = r / re, the decay
-// every Zhou function is built from (engine/eam_zhou.py:20-45), with r's
-// tangent rt; as HD<3> its directions are (re, expo, shift).
-template <int K>
-__device__ __forceinline__ HD<K> hz_decay(double r, double rt, const HD<K> &re, const HD<K> &expo,
-                                          const HD<K> &shift) {
-    HD<K> R = hd_const<K>(r);
-    R.t = rt;
-    HD<K> x = R / re;
-    HD<K> e = hd_exp<K>((-1.0) * (expo * (x + (-1.0))));
-    HD<K> u = x - shift;
-    double u2 = u.v * u.v, u4 = u2 * u2, u8 = u4 * u4, u16 = u8 * u8, u18 = u16 * u2;
-    HD<K> den = 1.0 + hd_apply<K>(u, u18 * u2, 20.0 * u18 * u.v, 380.0 * u18);
-    return e / den;
+// g = exp(-expo (x - 1)) / (1 + (x - shift)^20), x = r / re, the decay every
+// Zhou function is built from (engine/eam_zhou.py:20-45; ire = 1 / re): value,
+// tangent (r's is rt), and for (re, expo, shift) the derivatives p and their tangents q.
+// With w = 20 u^19 / (1 + u^20), u = x - shift: d ln g / dx = -(expo + w),
+// / d expo = -(x - 1), / d shift = w, and w' = 380 u^18 / (1 + u^20) - w^2;
+// p_k = g l_k and q_k = g_t l_k + g (l_k)_t.
+struct Decay {
+    double v, t, p[3], q[3];
+};
+
+__device__ __forceinline__ Decay zdecay3(double r, double rt, double ire, double expo, double shift) {
+    const double x = r * ire, xt = rt * ire, u = x - shift;
+    const double u2 = u * u, u4 = u2 * u2, u8 = u4 * u4, u16 = u8 * u8, u18 = u16 * u2;
+    const double id = 1.0 / fma(u18, u2, 1.0);
+    const double w = 20.0 * u18 * u * id, wx = 380.0 * u18 * id - w * w, lx = -(expo + w);
+    Decay g;
+    g.v = exp(-expo * (x - 1.0)) * id;
+    g.t = g.v * lx * xt;
+    const double l0 = -lx * x * ire, l0t = (wx * x - lx) * ire * xt;
+    g.p[0] = g.v * l0;
+    g.p[1] = -g.v * (x - 1.0);
+    g.p[2] = g.v * w;
+    g.q[0] = fma(g.t, l0, g.v * l0t);
+    g.q[1] = -fma(g.t, x - 1.0, g.v * xt);
+    g.q[2] = fma(g.t, w, g.v * wx * xt);
+    return g;
 }
 
-__device__ __forceinline__ HD<3> hz_g3(double r, double rt, double re, double expo, double shift) {
-    return hz_decay<3>(r, rt, hd_param<3>(re, 0, 0), hd_param<3>(expo, 1, 0), hd_param<3>(shift, 2, 0));
+// The quintic switch (columns 40, 41 of a row) at r, from its start r0 = rc -
+// width and iw = 1 / width: value and tangent.
+struct Switch {
+    double r0, iw;
+};
+__device__ __forceinline__ Switch switch_of(const double *row) {
+    return {row[2 * EADJ_NZ] - row[2 * EADJ_NZ + 1], 1.0 / row[2 * EADJ_NZ + 1]};
 }
-
-// The quintic switch of a row (columns 40, 41) at r: value and tangent.
-__device__ __forceinline__ void hz_switch(const double *row, double r, double rt, double &S, double &St) {
-    double rc = row[2 * EADJ_NZ], w = row[2 * EADJ_NZ + 1];
-    double s = (r - (rc - w)) / w;
+__device__ __forceinline__ void hz_switch(const Switch &w, double r, double rt, double &S, double &St) {
+    double s = (r - w.r0) * w.iw;
     s = s < 0.0 ? 0.0 : (s > 1.0 ? 1.0 : s);
     S = 1.0 - s * s * s * (10.0 - 15.0 * s + 6.0 * s * s);
-    St = -30.0 * s * s * (1.0 - s) * (1.0 - s) / w * rt;
+    St = -30.0 * s * s * (1.0 - s) * (1.0 - s) * w.iw * rt;
 }
 
 // One element's density f = f_e gB and pair u = A gA - B gB (unswitched),
@@ -87,7 +108,7 @@ __device__ __forceinline__ void hz_switch(const double *row, double r, double rt
 // (q): site_k += af f.p_k + bf f.q_k + au u.p_k + bu u.q_k, for the 8
 // element parameters r_e, f_e, alpha, beta, A, B, kappa, lambda (columns 0,
 // 1, 4..9 of p).
-__device__ __forceinline__ void hz_species_sites(double *o, const HD<3> &gA, const HD<3> &gB, const double *p,
+__device__ __forceinline__ void hz_species_sites(double *o, const Decay &gA, const Decay &gB, const double *p,
                                                  double af, double bf, double au, double bu) {
     double fe = p[1], A = p[6], B = p[7];
     o[0] += fe * (af * gB.p[0] + bf * gB.q[0]) + au * (A * gA.p[0] - B * gB.p[0]) + bu * (A * gA.q[0] - B * gB.q[0]);
@@ -126,284 +147,381 @@ __device__ __forceinline__ HD<13> hz_embed(const double *p, double rho, double r
 
 __device__ __forceinline__ const double *row_of(const EamAdjTab &T, int f) { return T.P + (size_t)f * EADJ_NCOL; }
 
-// Value and r-tangent of f_e g(r; r_e, beta, lambda) S(r) for pass 1.
-__device__ __forceinline__ void dens_value(const double *row, double r, double rt, double &v, double &vt) {
-    double x = r / row[0];
-    double e = exp(-row[5] * (x - 1.0));
-    double u = x - row[9];
-    double u2 = u * u, u4 = u2 * u2, u8 = u4 * u4, u16 = u8 * u8, u19 = u16 * u2 * u;
-    double id = 1.0 / (1.0 + u19 * u);
-    double g = e * id;
-    double dg = g * (-row[5] - 20.0 * u19 * id) / row[0];
+// A density row's constants for pass 1, and value and r-tangent of
+// f_e g(r; r_e, beta, lambda) S(r).
+struct DensRow {
+    double ire, fe, beta, lam;
+    Switch sw;
+};
+__device__ __forceinline__ void dens_value(const DensRow &p, double r, double rt, double &v, double &vt) {
+    const double x = r * p.ire, u = x - p.lam;
+    const double u2 = u * u, u4 = u2 * u2, u8 = u4 * u4, u16 = u8 * u8, u19 = u16 * u2 * u;
+    const double id = 1.0 / fma(u19, u, 1.0);
+    const double g = p.fe * exp(-p.beta * (x - 1.0)) * id;
     double Sw, St;
-    hz_switch(row, r, 1.0, Sw, St);  // St = dS/dr here
-    v = row[1] * g * Sw;
-    vt = row[1] * (dg * Sw + g * St) * rt;
+    hz_switch(p.sw, r, rt, Sw, St);
+    v = g * Sw;
+    vt = g * (St - (p.beta + 20.0 * u19 * id) * p.ire * rt * Sw);
 }
 
-// Tiles: EADJ_TA atoms (embedding pass) or EADJ_TP pairs (pair pass) per
-// iteration of a block; blocks stride over tiles in a fixed order and keep
-// their own sums, so every reduction below is in a fixed order.
-constexpr int EADJ_TA = 128;
-constexpr int EADJ_TP = 64;
-constexpr int EADJ_GRID = 148 * 16;  // pair-kernel blocks at most (16 per SM of a B200)
-constexpr int EADJ_PS = 25;          // staged values of one pair
-constexpr int EADJ_STRIDE = 25;      // odd: conflict-free 8-byte shared accesses
+constexpr int EADJ_TA = 128;         // atoms per block of the embedding pass
+constexpr int EADJ_LPA = 8;          // lanes per atom of the row passes
+constexpr int EADJ_PS = 25;          // sites of a species pair
+constexpr int EADJ_PB = 128;         // threads of a pair block
+constexpr int EADJ_PG = 148 * 4;     // pair blocks per species pair at most
 
-// Pass 1, a thread per atom: rho-bar and its tangent over the full row, the
-// embedding sites (12; summed per species of the centre into the block's
-// partialF row) and the coefficients c1 = gE F' + F'' D_t rho-bar, c2 = F'
-// through which every density parameter acts on this atom's site term.
-// Also counts the live pairs above the diagonal (j > i, inside the cutoff):
-// cnt[i] like-species pairs, cnt[n_atoms + i] cross pairs.
-__global__ void __launch_bounds__(EADJ_TA) eam_adjoint_embed(SysView S, const int *__restrict__ row_off,
-                                                             const int *__restrict__ upper,
-                                                             const int *__restrict__ nbr, EamAdjTab T, AdjIn G,
-                                                             double2 *__restrict__ cc, int *__restrict__ cnt,
-                                                             double *__restrict__ partialF) {
-    __shared__ double sf[EADJ_TA * 13];  // 12 sites per atom, odd stride
-    __shared__ int scode[EADJ_TA];
-    extern __shared__ double accF[];     // ns * 12
-    const int ns = T.ns, nf = 12 * ns;
-    for (int k = threadIdx.x; k < nf; k += blockDim.x) accF[k] = 0.0;
+// Index of the unordered species pair (a, b).
+__device__ __forceinline__ int pair_code(int a, int b, int ns) {
+    const int lo = min(a, b), hi = max(a, b);
+    return lo * ns - lo * (lo - 1) / 2 + hi - lo;
+}
+
+// Position and upstream force gradient of an atom.
+struct PairAtom {
+    double x[3], f[3];
+    __device__ __forceinline__ void load(const SysView &S, const AdjIn &G, int a) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            x[k] = __ldg(S.pos + 3 * (size_t)a + k);
+            f[k] = G.gF ? __ldg(G.gF + 3 * (size_t)a + k) : 0.0;
+        }
+    }
+};
+
+// What a structure contributes to its pairs' geometry: the cell, and the
+// upstream virial gradient's symmetric part (only d . gW d enters).
+struct PairCell {
+    RowCell cell;
+    double w[6];  // xx yy zz 2xy 2xz 2yz of the symmetric part
+    __device__ __forceinline__ void load(const SysView &S, const AdjIn &G, int atom, int sst) {
+        cell.load(S, atom);
+        if (G.gW) {
+            const double *g = G.gW + 9 * (size_t)sst;
+            w[0] = __ldg(g);
+            w[1] = __ldg(g + 4);
+            w[2] = __ldg(g + 8);
+            w[3] = __ldg(g + 1) + __ldg(g + 3);
+            w[4] = __ldg(g + 2) + __ldg(g + 6);
+            w[5] = __ldg(g + 5) + __ldg(g + 7);
+        } else {
+#pragma unroll
+            for (int k = 0; k < 6; ++k) w[k] = 0.0;
+        }
+    }
+    // r^2, r and the tangent of r of the pair (i, j): t_ij = gF_i - gF_j - gW d
+    // enters only through d . t / r.
+    __device__ __forceinline__ void pair(const PairAtom &i, const PairAtom &j, double &r2, double &r, double &rt) const {
+        double x, y, z;
+        cell.mic(j.x[0] - i.x[0], j.x[1] - i.x[1], j.x[2] - i.x[2], x, y, z);
+        r2 = x * x + y * y + z * z;
+        const double ir = rsqrt(r2);
+        r = r2 * ir;
+        rt = ir * (x * (i.f[0] - j.f[0]) + y * (i.f[1] - j.f[1]) + z * (i.f[2] - j.f[2]) -
+                   (x * (w[0] * x + w[3] * y + w[4] * z) + y * (w[1] * y + w[5] * z) + z * (w[2] * z)));
+    }
+};
+
+// Pass 1, EADJ_LPA lanes per atom over its full row: rho-bar and its tangent
+// into rr.  Slots above the diagonal get a mark (1 + the neighbour's species
+// where the pair is inside the cutoff, else 0), and cnt[c * n_atoms + i]
+// counts them by species pair.  Bound by FP64 issue and the scattered loads
+// of the neighbours: 170 us for 101,000 atoms of 134 slots (a thread per atom,
+// with the embedding at its end, took 340).
+__global__ void __launch_bounds__(128) eam_adjoint_density(SysView S, const int *__restrict__ row_off,
+                                                           const int *__restrict__ upper, const int *__restrict__ nbr,
+                                                           EamAdjTab T, AdjIn G, double2 *__restrict__ rr,
+                                                           unsigned char *__restrict__ mark, int *__restrict__ cnt) {
+    constexpr int LPA = EADJ_LPA;
+    __shared__ DensRow dens[8];
+    const int i = (blockIdx.x * blockDim.x + threadIdx.x) / LPA, sub = threadIdx.x & (LPA - 1);
+    const bool in = i < S.n_atoms;
+    const int ns = T.ns;
+    for (int k = threadIdx.x; k < ns; k += blockDim.x) {
+        const double *p = row_of(T, T.rho_f[k]);
+        dens[k] = {1.0 / p[0], p[1], p[5], p[9], switch_of(p)};
+    }
+    __syncthreads();
     const double rc2 = T.rc * T.rc;
-    int n_tiles = (S.n_atoms + EADJ_TA - 1) / EADJ_TA;
-    for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
-        int i = tile * EADJ_TA + threadIdx.x;
-        int code = -1;
-        double *o = sf + 13 * threadIdx.x;
-        if (i < S.n_atoms) {
-            int si = S.types[i];
-            int sst = S.n_struct > 1 ? S.atom_struct[i] : 0;
-            double gE = G.gE ? G.gE[sst] : 0.0;
-            const double *cell = cell_of(S, i);
-            double rho = 0.0, rho_t = 0.0;
-            int up = upper[i], n_like = 0, n_cross = 0;
-            for (int s = row_off[i]; s < row_off[i + 1]; ++s) {
-                int j = nbr[s];
-                double d[3], r, tg[3];
-                adj_leg(S, G, cell, i, j, sst, d, r, tg);
-                if (!(r * r < rc2 && r * r > 1e-24)) continue;
-                int sj = S.types[j];
-                if (s >= up) {
-                    if (si == sj) ++n_like;
-                    else ++n_cross;
-                }
-                double rt = (d[0] * tg[0] + d[1] * tg[1] + d[2] * tg[2]) / r;
+    double rho = 0.0, rho_t = 0.0;
+    unsigned long long c0 = 0ull, c1 = 0ull;  // marked slots by species, 16 bits each (species 0-3, 4-7)
+    int si = 0;
+    if (in) {
+        si = S.types[i];
+        const int sst = S.n_struct > 1 ? S.atom_struct[i] : 0, up = upper[i], end = row_off[i + 1];
+        PairCell pc;
+        pc.load(S, G, i, sst);
+        // slot indices two iterations ahead, the neighbour's data one ahead
+        int s = row_off[i] + sub, j1 = s + LPA < end ? nbr[s + LPA] : i, tn = 0;
+        PairAtom me, nx;
+        me.load(S, G, i);
+        if (s < end) {
+            const int j0 = nbr[s];
+            nx.load(S, G, j0);
+            tn = S.types[j0];
+        }
+        for (; s < end; s += LPA) {
+            const PairAtom at = nx;
+            const int sj = tn;
+            if (s + LPA < end) {
+                nx.load(S, G, j1);
+                tn = S.types[j1];
+            }
+            if (s + 2 * LPA < end) j1 = nbr[s + 2 * LPA];
+            double r2, r, rt;
+            pc.pair(me, at, r2, r, rt);
+            const bool live = r2 < rc2 && r2 > 1e-24;
+            if (live) {
                 double v, vt;
-                dens_value(row_of(T, T.rho_f[sj]), r, rt, v, vt);
+                dens_value(dens[sj], r, rt, v, vt);
                 rho += v;
                 rho_t += vt;
             }
-            // the embedding, rho-bar clamped at 0 as the evaluation does
-            double rb = rho > 0.0 ? rho : 0.0;
-            HD<13> F = hz_embed(row_of(T, T.F_f[si]), rb, rho_t);
+            if (s >= up) {
+                mark[s] = live ? (unsigned char)(1 + sj) : 0;
+                if (live) (sj < 4 ? c0 : c1) += 1ull << (16 * (sj & 3));
+            }
+        }
+    }
+    rho = group_sum<LPA>(rho);
+    rho_t = group_sum<LPA>(rho_t);
+    c0 = group_sum<LPA>(c0);
+    c1 = group_sum<LPA>(c1);
+    if (!in) return;
+    if (sub == 0) rr[i] = make_double2(rho, rho_t);
+    for (int c = sub, a = 0, first = 0; c < ns * (ns + 1) / 2; c += LPA) {
+        while (c >= first + ns - a) first += ns - a++;  // c = pair_code(a, b)
+        const int b = a + c - first, o = a == si ? b : (b == si ? a : -1);
+        cnt[(size_t)c * S.n_atoms + i] = o < 0 ? 0 : (int)((o < 4 ? c0 : c1) >> (16 * (o & 3)) & 0xffffull);
+    }
+}
+
+// Pass 2, a thread per atom: the embedding sites (12; summed per species of
+// the centre into the block's partialF row) and the coefficients c1 = gE F' +
+// F'' D_t rho-bar, c2 = F' through which every density parameter acts on this
+// atom's site term (cc, in place of rr).
+__global__ void __launch_bounds__(EADJ_TA) eam_adjoint_embed(SysView S, EamAdjTab T, AdjIn G, double2 *__restrict__ cc,
+                                                             double *__restrict__ partialF) {
+    __shared__ double sf[EADJ_TA * 13];  // 12 sites per atom, odd stride
+    __shared__ int scode[EADJ_TA];
+    const int nf = 12 * T.ns;
+    const int i = blockIdx.x * EADJ_TA + threadIdx.x;
+    int code = -1;
+    double *o = sf + 13 * threadIdx.x;
+    if (i < S.n_atoms) {
+        const int si = S.types[i];
+        const int sst = S.n_struct > 1 ? S.atom_struct[i] : 0;
+        const double gE = G.gE ? G.gE[sst] : 0.0;
+        const double2 rr = cc[i];
+        // the embedding, rho-bar clamped at 0 as the evaluation does
+        const double rb = rr.x > 0.0 ? rr.x : 0.0;
+        HD<13> F = hz_embed(row_of(T, T.F_f[si]), rb, rr.y);
 #pragma unroll
-            for (int k = 0; k < 12; ++k) o[k] = gE * F.p[k] + F.q[k];
-            cc[i] = make_double2(rho > 0.0 ? gE * F.p[12] + F.q[12] : 0.0, F.p[12]);
-            cnt[i] = n_like;
-            cnt[S.n_atoms + i] = n_cross;
-            code = si;
+        for (int k = 0; k < 12; ++k) o[k] = gE * F.p[k] + F.q[k];
+        cc[i] = make_double2(rr.x > 0.0 ? gE * F.p[12] + F.q[12] : 0.0, F.p[12]);
+        code = si;
+    }
+    scode[threadIdx.x] = code;
+    __syncthreads();
+    const int cnt = min(EADJ_TA, S.n_atoms - (int)blockIdx.x * EADJ_TA);
+    for (int item = threadIdx.x; item < nf; item += blockDim.x) {
+        const int sp = item / 12, k = item % 12;
+        double a = 0.0;
+        for (int q = 0; q < cnt; ++q)
+            if (scode[q] == sp) a += sf[13 * q + k];
+        partialF[(size_t)item * gridDim.x + blockIdx.x] = a;  // (site, block)
+    }
+}
+
+// Compaction, EADJ_LPA lanes per atom: the marked slots of its upper half as
+// pairs (atom of the earlier species, atom of the later) at the scanned
+// offsets, each list in atom then slot order.
+__global__ void __launch_bounds__(128) eam_adjoint_compact(int n_atoms, int ns, const int *__restrict__ types,
+                                                           const int *__restrict__ row_off,
+                                                           const int *__restrict__ upper, const int *__restrict__ nbr,
+                                                           const unsigned char *__restrict__ mark,
+                                                           const int *__restrict__ pos, int2 *__restrict__ pairs) {
+    constexpr int LPA = EADJ_LPA;
+    const int i = (blockIdx.x * blockDim.x + threadIdx.x) / LPA, sub = threadIdx.x & (LPA - 1);
+    if (i >= n_atoms) return;  // whole groups leave together
+    const int gl = threadIdx.x & 31 & ~(LPA - 1);
+    const unsigned gones = (1u << LPA) - 1u, gmask = gones << gl;
+    const int si = types[i], beg = upper[i], end = row_off[i + 1];
+    // lane b of the group keeps the next position in species b's list
+    int next = sub < ns ? pos[(size_t)pair_code(si, sub, ns) * n_atoms + i] : 0;
+    int mn = 0, jn = 0;
+    if (beg + sub < end) {
+        mn = mark[beg + sub];
+        jn = nbr[beg + sub];
+    }
+    for (int s0 = beg; s0 < end; s0 += LPA) {
+        const int m = mn, j = jn, s1 = s0 + LPA + sub;
+        mn = 0;
+        if (s1 < end) {
+            mn = mark[s1];
+            jn = nbr[s1];
         }
-        scode[threadIdx.x] = code;
-        __syncthreads();
-        int cnt = min(EADJ_TA, S.n_atoms - tile * EADJ_TA);
-        for (int item = threadIdx.x; item < nf; item += blockDim.x) {
-            int sp = item / 12, k = item % 12;
-            double a = 0.0;
-            for (int q = 0; q < cnt; ++q)
-                if (scode[q] == sp) a += sf[13 * q + k];
-            accF[item] += a;
+        int o = -1;
+        for (int b = 0; b < ns; ++b) {
+            const unsigned hit = (__ballot_sync(gmask, m == 1 + b) >> gl) & gones;
+            const int base = __shfl_sync(gmask, next, b, LPA);
+            if (m == 1 + b) o = base + __popc(hit & ((1u << sub) - 1u));
+            if (sub == b) next += __popc(hit);
         }
-        __syncthreads();
-    }
-    for (int k = threadIdx.x; k < nf; k += blockDim.x) partialF[(size_t)blockIdx.x * nf + k] = accF[k];
-}
-
-// Compacted pair list, a thread per atom: its live upper slots (the same
-// test as eam_adjoint_embed's, so the same count) at its scanned offsets,
-// like pairs in [pos[0], pos[N]), cross pairs in [pos[N], pos[2N]), each in
-// atom then slot order.
-__global__ void eam_adjoint_compact(SysView S, const int *__restrict__ row_off, const int *__restrict__ upper,
-                                    const int *__restrict__ nbr, EamAdjTab T, AdjIn G,
-                                    const int *__restrict__ pos, int *__restrict__ pairs) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= S.n_atoms) return;
-    int si = S.types[i];
-    int sst = S.n_struct > 1 ? S.atom_struct[i] : 0;
-    const double *cell = cell_of(S, i);
-    const double rc2 = T.rc * T.rc;
-    int ol = pos[i], oc = pos[S.n_atoms + i];
-    for (int s = upper[i]; s < row_off[i + 1]; ++s) {
-        int j = nbr[s];
-        double d[3], r, tg[3];
-        adj_leg(S, G, cell, i, j, sst, d, r, tg);
-        if (!(r * r < rc2 && r * r > 1e-24)) continue;
-        if (S.types[j] == si) pairs[ol++] = s;
-        else pairs[oc++] = s;
+        if (o >= 0) pairs[o] = si <= m - 1 ? make_int2(i, j) : make_int2(j, i);
     }
 }
 
-// The slot's owning atom: rows are sorted, so a binary search in row_off.
-__device__ __forceinline__ int eadj_owner(const int *__restrict__ row_off, int n_atoms, int s) {
-    int lo = 0, hi = n_atoms - 1;
-    while (lo < hi) {
-        int mid = (lo + hi + 1) >> 1;
-        if (row_off[mid] <= s) lo = mid; else hi = mid - 1;
-    }
-    return lo;
-}
-
-// Density sites of one centre's view of a neighbour of species s at r:
-// rho_s = f_e gB S, contributing c1 d(rho)/dtheta + c2 d(D_t rho)/dtheta to
-// r_e, f_e, beta, lambda (o[0..3]).
-__device__ __forceinline__ void dens_sites(double *o, const HD<3> &gB, const double *row, double Sw, double St,
+// Density sites of a neighbour species' row at r: f_e gB S, contributing
+// c1 d(rho)/dtheta + c2 d(D_t rho)/dtheta to r_e, f_e, beta, lambda (o[0..3]).
+__device__ __forceinline__ void dens_sites(double *o, const Decay &gB, const double *row, double Sw, double St,
                                            double c1, double c2) {
-    double a = c1 * Sw + c2 * St, bq = c2 * Sw;
-    double af = a * row[1], bf = bq * row[1];
+    const double a = c1 * Sw + c2 * St, bq = c2 * Sw, af = a * row[1], bf = bq * row[1];
     o[0] += af * gB.p[0] + bf * gB.q[0];
     o[1] += a * gB.v + bq * gB.t;
     o[2] += af * gB.p[1] + bf * gB.q[1];
     o[3] += af * gB.p[2] + bf * gB.q[2];
 }
 
-// The density decay of species row `dr` at r: the pair's decay of the same
-// element when the density row holds the same (r_e, beta, lambda), else its
-// own.
-__device__ __forceinline__ HD<3> dens_decay(const double *dr, const double *blk, const HD<3> &gB_blk, double r,
-                                            double rt) {
-    if (dr[0] == blk[0] && dr[5] == blk[5] && dr[9] == blk[9]) return gB_blk;
-    return hz_g3(r, rt, dr[0], dr[5], dr[9]);
+// A block's constants of its species pair: 1 / r_e and the switches of the
+// pair row and of the density rows, and whether a density row's decay and
+// switch are those of the pair row's element (they are in a table built from
+// one set of element parameters, and are then evaluated once).
+struct PairConst {
+    double ire_a, ire_b, ire_da, ire_db;
+    Switch sw, sw_a, sw_b;
+    int same_a, same_b;
+};
+__device__ __forceinline__ bool same_decay(const double *dr, const double *blk) {
+    return dr[0] == blk[0] && dr[5] == blk[5] && dr[9] == blk[9];
 }
 
-// The 25 staged values of the live pair at slot s (i < j): 0..16 the pair
-// sites of row phi_f[s_i, s_j] (weight 1: the two halves 1/2 phi of the
-// site terms of i and j), 17..20 the density sites of i's view of rho_{s_j}
-// (coefficients of i), 21..24 those of j's view of rho_{s_i}.  Returns the
-// code s_i ns + s_j.
+// Pass 3, one species pair per blockIdx.y: a thread takes every
+// EADJ_PB-th pair of its block's contiguous share of the list and keeps the
+// site sums in registers; the block's sums go to its row of `partial`.  Sites
+// staged in shared memory per tile of pairs and summed there by entry, with
+// the decays in generic hyper-dual arithmetic, took 714 us for the 4.9 M
+// pairs of 101,000 Ni3Al atoms; this pass takes 228.  Bound by FP64 issue and
+// its latency (36-40 % of the FP64 pipe).
+// Resident blocks: 4 of 128 registers for the like pairs, 2 of 202 for the
+// cross pairs (101,000 atoms, both: 228 us; 5 spills: 259; 3 cross blocks: 241).
 template <bool LIKE>
-__device__ int eam_pair_sites(const SysView &S, const int *__restrict__ row_off, const int *__restrict__ nbr,
-                              const EamAdjTab &T, const AdjIn &G, const double2 *__restrict__ cc, int s, double *o) {
-    const int ns = T.ns;
-    int i = eadj_owner(row_off, S.n_atoms, s);
-    int j = nbr[s];
-    int si = S.types[i], sj = S.types[j];
-    int sst = S.n_struct > 1 ? S.atom_struct[i] : 0;
-    double gE = G.gE ? G.gE[sst] : 0.0;
-    double d[3], r, tg[3];
-    adj_leg(S, G, cell_of(S, i), i, j, sst, d, r, tg);
-    double rt = (d[0] * tg[0] + d[1] * tg[1] + d[2] * tg[2]) / r;
-    for (int k = 0; k < EADJ_PS; ++k) o[k] = 0.0;
-    const double *row = row_of(T, T.phi_f[si * ns + sj]);
-    const double *rho_i = row_of(T, T.rho_f[si]), *rho_j = row_of(T, T.rho_f[sj]);
-    const double2 ci = cc[i], cj = cc[j];
-    double Sw, St, Dw, Dt;
-    hz_switch(row, r, rt, Sw, St);
-    HD<3> gAa = hz_g3(r, rt, row[0], row[4], row[8]);
-    HD<3> gBa = hz_g3(r, rt, row[0], row[5], row[9]);
-    if (LIKE) {
-        // phi = u S
-        hz_species_sites(o, gAa, gBa, row, 0.0, 0.0, gE * Sw + St, Sw);
-        HD<3> gD = dens_decay(rho_j, row, gBa, r, rt);
-        hz_switch(rho_j, r, rt, Dw, Dt);
-        dens_sites(o + 17, gD, rho_j, Dw, Dt, ci.x, ci.y);
-        dens_sites(o + 21, gD, rho_i, Dw, Dt, cj.x, cj.y);
-    } else {
-        // phi = k psi, psi = 1/2 S (q u_a + u_b / q), q = f_b / f_a, a the
-        // earlier species: psi's derivatives in (f_a, u_a, f_b, u_b), then
-        // each element's chain
-        const double *pb = row + EADJ_NZ;
-        HD<3> gAb = hz_g3(r, rt, pb[0], pb[4], pb[8]);
-        HD<3> gBb = hz_g3(r, rt, pb[0], pb[5], pb[9]);
-        HD<4> fa = hd_param<4>(row[1] * gBa.v, 0, 0), ua = hd_param<4>(row[6] * gAa.v - row[7] * gBa.v, 1, 0);
-        HD<4> fb = hd_param<4>(pb[1] * gBb.v, 2, 0), ub = hd_param<4>(pb[6] * gAb.v - pb[7] * gBb.v, 3, 0);
-        fa.t = row[1] * gBa.t;
-        ua.t = row[6] * gAa.t - row[7] * gBa.t;
-        fb.t = pb[1] * gBb.t;
-        ub.t = pb[6] * gAb.t - pb[7] * gBb.t;
-        HD<4> Sh = hd_const<4>(Sw);
-        Sh.t = St;
-        HD<4> q = fb / fa;
-        HD<4> psi = 0.5 * (Sh * (q * ua + ub / q));
-        double h = row[2 * EADJ_NZ + 2];
-        hz_species_sites(o, gAa, gBa, row, h * (gE * psi.p[0] + psi.q[0]), h * psi.p[0],
-                         h * (gE * psi.p[1] + psi.q[1]), h * psi.p[1]);
-        hz_species_sites(o + 8, gAb, gBb, pb, h * (gE * psi.p[2] + psi.q[2]), h * psi.p[2],
-                         h * (gE * psi.p[3] + psi.q[3]), h * psi.p[3]);
-        o[16] = gE * psi.v + psi.t;
-        // the element blocks of s_i and s_j in the cross row
-        bool i_first = si < sj;
-        const double *bi = i_first ? row : pb, *bj = i_first ? pb : row;
-        HD<3> gDj = dens_decay(rho_j, bj, i_first ? gBb : gBa, r, rt);
-        hz_switch(rho_j, r, rt, Dw, Dt);
-        dens_sites(o + 17, gDj, rho_j, Dw, Dt, ci.x, ci.y);
-        HD<3> gDi = dens_decay(rho_i, bi, i_first ? gBa : gBb, r, rt);
-        hz_switch(rho_i, r, rt, Dw, Dt);
-        dens_sites(o + 21, gDi, rho_i, Dw, Dt, cj.x, cj.y);
-    }
-    return si * ns + sj;
-}
-
-// Pass 2, a thread per live pair of one segment of the compacted list
-// (like pairs [0, pos[N]) or cross pairs [pos[N], pos[2 N])), EADJ_TP
-// pairs per tile: the staged values are sorted by code
-// inside the tile (a counting sort, ranks from warp matches, so the order
-// is fixed), then each (code, value) item is summed over its segment into
-// the block's partialP row (ns^2 * 25).  The two segments are separate
-// instantiations: the like pairs' kernel keeps a smaller register budget.
-// Resident blocks per SM the cross-pair instantiation is compiled for (its
-// register budget: 65536 / (EADJ_TP * MBF_EADJ_CROSS_MINB)).
-#ifndef MBF_EADJ_CROSS_MINB
-#define MBF_EADJ_CROSS_MINB 8
-#endif
-
-template <bool LIKE>
-__global__ void __launch_bounds__(EADJ_TP, LIKE ? 1 : MBF_EADJ_CROSS_MINB) eam_adjoint_pairs(SysView S, const int *__restrict__ row_off,
-                                                             const int *__restrict__ nbr, EamAdjTab T, AdjIn G,
+__global__ void __launch_bounds__(EADJ_PB, LIKE ? 4 : 2) eam_adjoint_pairs(SysView S, EamAdjTab T, AdjIn G,
                                                              const double2 *__restrict__ cc,
-                                                             const int *__restrict__ pairs,
-                                                             const int *__restrict__ seg_begin,
-                                                             const int *__restrict__ seg_end,
-                                                             double *__restrict__ partialP) {
-    __shared__ double st[EADJ_TP * EADJ_STRIDE];
-    __shared__ int order[EADJ_TP];
-    __shared__ int wcnt[2][65], start[66];
-    extern __shared__ double accP[];     // ns^2 * 25
-    const int ns = T.ns, nc = ns * ns, ni = nc * EADJ_PS;
-    for (int k = threadIdx.x; k < ni; k += blockDim.x) accP[k] = 0.0;
-    const int p0 = *seg_begin, np = *seg_end - p0;
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    for (int tile = blockIdx.x; tile * EADJ_TP < np; tile += gridDim.x) {
-        int m = tile * EADJ_TP + threadIdx.x;
-        int code = nc;  // past the last code: not summed
-        if (m < np)
-            code = eam_pair_sites<LIKE>(S, row_off, nbr, T, G, cc, pairs[p0 + m], st + EADJ_STRIDE * threadIdx.x);
-        for (int k = threadIdx.x; k < 2 * 65; k += blockDim.x) (&wcnt[0][0])[k] = 0;
-        __syncthreads();
-        unsigned same = __match_any_sync(MBF_FULL, code);
-        int rank = __popc(same & ((1u << lane) - 1u));
-        if (rank == 0) wcnt[w][code] = __popc(same);
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            int a = 0;
-            for (int c = 0; c <= nc; ++c) {
-                start[c] = a;
-                a += wcnt[0][c] + wcnt[1][c];
-            }
-            start[nc + 1] = a;
-        }
-        __syncthreads();
-        order[start[code] + (w ? wcnt[0][code] : 0) + rank] = threadIdx.x;
-        __syncthreads();
-        for (int item = threadIdx.x; item < ni; item += blockDim.x) {
-            int c = item / EADJ_PS, k = item % EADJ_PS;
-            double a = 0.0;
-            for (int q = start[c]; q < start[c + 1]; ++q) a += st[EADJ_STRIDE * order[q] + k];
-            accP[item] += a;
-        }
-        __syncthreads();
+                                                             const int2 *__restrict__ pairs,
+                                                             const int *__restrict__ pos,
+                                                             double *__restrict__ partial) {
+    constexpr int NV = LIKE ? 12 : EADJ_PS;
+    __shared__ double rows[4][EADJ_NCOL];   // pair row, the two density rows
+    __shared__ double sums[EADJ_PB / 32][NV];
+    __shared__ PairConst K;
+    const int ns = T.ns;
+    int a = blockIdx.y, b = blockIdx.y;
+    if (!LIKE) {  // the blockIdx.y-th pair a < b
+        a = 0;
+        int q = blockIdx.y;
+        while (q >= ns - 1 - a) q -= ns - 1 - a++;
+        b = a + 1 + q;
     }
-    for (int k = threadIdx.x; k < ni; k += blockDim.x) partialP[(size_t)blockIdx.x * ni + k] = accP[k];
+    const int c = pair_code(a, b, ns);
+    for (int k = threadIdx.x; k < EADJ_NCOL; k += blockDim.x) {
+        rows[0][k] = row_of(T, T.phi_f[a * ns + b])[k];
+        rows[1][k] = row_of(T, T.rho_f[a])[k];
+        rows[2][k] = row_of(T, T.rho_f[b])[k];
+    }
+    __syncthreads();
+    const double *row = rows[0], *rho_a = rows[1], *rho_b = rows[2], *pb = LIKE ? row : row + EADJ_NZ;
+    if (threadIdx.x == 0) {
+        K.ire_a = 1.0 / row[0];
+        K.ire_b = 1.0 / pb[0];
+        K.ire_da = 1.0 / rho_a[0];
+        K.ire_db = 1.0 / rho_b[0];
+        K.sw = switch_of(row);
+        K.sw_a = switch_of(rho_a);
+        K.sw_b = switch_of(rho_b);
+        const bool w_a = row[40] == rho_a[40] && row[41] == rho_a[41], w_b = row[40] == rho_b[40] && row[41] == rho_b[41];
+        K.same_a = same_decay(rho_a, row) && w_a;
+        K.same_b = same_decay(rho_b, pb) && w_b;
+    }
+    __syncthreads();
+    double o[NV];
+#pragma unroll
+    for (int k = 0; k < NV; ++k) o[k] = 0.0;
+    const int p0 = pos[(size_t)c * S.n_atoms], np = pos[(size_t)(c + 1) * S.n_atoms] - p0;
+    const int per = (np + gridDim.x - 1) / gridDim.x;
+    const int m1 = min(np, ((int)blockIdx.x + 1) * per);
+    for (int m = (int)blockIdx.x * per + threadIdx.x; m < m1; m += EADJ_PB) {
+        const int2 pq = pairs[p0 + m];
+        const int sst = S.n_struct > 1 ? __ldg(S.atom_struct + pq.x) : 0;
+        const double gE = G.gE ? __ldg(G.gE + sst) : 0.0;
+        const double2 cp = cc[pq.x], cq = cc[pq.y];
+        double r2, r, rt;
+        PairCell pc;
+        pc.load(S, G, pq.x, sst);
+        PairAtom ap, aq;
+        ap.load(S, G, pq.x);
+        aq.load(S, G, pq.y);
+        pc.pair(ap, aq, r2, r, rt);
+        double Sw, St;
+        hz_switch(K.sw, r, rt, Sw, St);
+        const Decay gA = zdecay3(r, rt, K.ire_a, row[4], row[8]);
+        const Decay gB = zdecay3(r, rt, K.ire_a, row[5], row[9]);
+        // the density sites of row rho (decay gD, or its own) with the
+        // coefficients c of the atom that sees it
+        auto density = [&](double *od, int same, const Decay &gD, const double *rho, double ire, const Switch &sw,
+                           double cx, double cy) {
+            if (same) {
+                dens_sites(od, gD, rho, Sw, St, cx, cy);
+            } else {
+                double Dw, Dt;
+                hz_switch(sw, r, rt, Dw, Dt);
+                dens_sites(od, zdecay3(r, rt, ire, rho[5], rho[9]), rho, Dw, Dt, cx, cy);
+            }
+        };
+        if constexpr (LIKE) {
+            // phi = u S; the two atoms' densities are of the same row
+            hz_species_sites(o, gA, gB, row, 0.0, 0.0, gE * Sw + St, Sw);
+            density(o + 8, K.same_b, gB, rho_b, K.ire_db, K.sw_b, cp.x + cq.x, cp.y + cq.y);
+        } else {
+            // phi = k psi, psi = 1/2 S (A + B), A = q u_a, B = u_b / q, q =
+            // f_b / f_a: psi's derivatives in (f_a, u_a, f_b, u_b) and their
+            // tangents, then each element's chain
+            const Decay hA = zdecay3(r, rt, K.ire_b, pb[4], pb[8]);
+            const Decay hB = zdecay3(r, rt, K.ire_b, pb[5], pb[9]);
+            const double fa = row[1] * gB.v, fat = row[1] * gB.t, fb = pb[1] * hB.v, fbt = pb[1] * hB.t;
+            const double ua = row[6] * gA.v - row[7] * gB.v, uat = row[6] * gA.t - row[7] * gB.t;
+            const double ub = pb[6] * hA.v - pb[7] * hB.v, ubt = pb[6] * hA.t - pb[7] * hB.t;
+            const double inv = 1.0 / (fa * fb), ifa = fb * inv, ifb = fa * inv, q = fb * ifa, iq = fa * ifb;
+            const double mt = fbt * ifb - fat * ifa;  // (ln q)_t
+            const double A = q * ua, B = ub * iq, At = A * mt + q * uat, Bt = ubt * iq - B * mt;
+            const double h = row[2 * EADJ_NZ + 2], hS = 0.5 * h * Sw, hSt = 0.5 * h * St;
+            const double E = A - B, Et = At - Bt;
+            const double wq = hS * q, wqt = q * (hSt + hS * mt), wi = hS * iq, wit = iq * (hSt - hS * mt);
+            const double eb = hS * E * ifb, ebt = (hSt * E + hS * Et) * ifb - eb * (fbt * ifb);
+            const double ea = -hS * E * ifa, eat = -(hSt * E + hS * Et) * ifa - ea * (fat * ifa);
+            o[16] += 0.5 * (gE * Sw * (A + B) + St * (A + B) + Sw * (At + Bt));
+            hz_species_sites(o, gA, gB, row, gE * ea + eat, ea, gE * wq + wqt, wq);
+            density(o + 21, K.same_a, gB, rho_a, K.ire_da, K.sw_a, cq.x, cq.y);
+            hz_species_sites(o + 8, hA, hB, pb, gE * eb + ebt, eb, gE * wi + wit, wi);
+            density(o + 17, K.same_b, hB, rho_b, K.ire_db, K.sw_b, cp.x, cp.y);
+        }
+    }
+    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+        double x = o[k];
+#pragma unroll
+        for (int d = 16; d > 0; d >>= 1) x += __shfl_xor_sync(MBF_FULL, x, d);
+        if (l == 0) sums[w][k] = x;
+    }
+    __syncthreads();
+    double *out = partial + (size_t)c * EADJ_PS * gridDim.x + blockIdx.x;  // (list, site, block)
+    for (int k = threadIdx.x; k < EADJ_PS; k += blockDim.x) {
+        const int v = !LIKE ? k : (k < 8 ? k : (k >= 17 && k < 21 ? k - 9 : -1));
+        double x = 0.0;
+        if (v >= 0)
+            for (int q = 0; q < EADJ_PB / 32; ++q) x += sums[q][v];
+        out[(size_t)k * gridDim.x] = x;
+    }
 }
 
 // Column -> site of a role (-1: not differentiated).
@@ -418,40 +536,36 @@ __device__ __forceinline__ int p_site(int c) {
 }
 
 // One warp per entry (row f, column c) of d_P: the block partials that feed
-// it -- the embedding sums of the row's species, the density values of
-// every code with that neighbour (i's view) or centre (j's view) species,
-// the pair values of the row's code(s) -- summed over blocks by lanes, then
-// a fixed shuffle tree.
+// it -- the embedding sums of the row's species, the density sites of every
+// pair with that species, the pair sites of the row's pair -- summed over
+// blocks by lanes, then a fixed shuffle tree.
 __global__ void eam_adjoint_final(EamAdjTab T, int gA, const double *__restrict__ partialF, int gP,
-                                  const double *__restrict__ partialP, double *__restrict__ d_P) {
-    const int ns = T.ns, nfs = 12 * ns, ni = ns * ns * EADJ_PS;
+                                  const double *__restrict__ partial, double *__restrict__ d_P) {
+    const int ns = T.ns;
     int e = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, l = threadIdx.x & 31;
     if (e >= T.nf * EADJ_NCOL) return;  // whole warps leave together
     int f = e / EADJ_NCOL, c = e % EADJ_NCOL;
-    int idx[16], n = 0;  // items of partialP feeding this entry (<= 2 ns)
-    int fitem = -1;      // item of partialF
-    for (int s = 0; s < ns; ++s) {
-        if (T.F_f[s] == f && f_site(c) >= 0) fitem = 12 * s + f_site(c);
-        if (T.rho_f[s] == f && d_site(c) >= 0)
-            for (int x = 0; x < ns; ++x) {
-                idx[n++] = (x * ns + s) * EADJ_PS + 17 + d_site(c);  // centre x, neighbour s
-                idx[n++] = (s * ns + x) * EADJ_PS + 21 + d_site(c);  // centre s: j's view
-            }
-    }
+    // one row of n block values: four loads in flight a lane
+    double acc = 0.0;
+    auto add_row = [&](const double *p, int n) {
+        double x[4] = {0.0, 0.0, 0.0, 0.0};
+        for (int b = l; b < n; b += 128) {
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                if (b + 32 * k < n) x[k] += p[b + 32 * k];
+        }
+        acc += (x[0] + x[1]) + (x[2] + x[3]);
+    };
+    for (int s = 0; s < ns; ++s)
+        if (T.F_f[s] == f && f_site(c) >= 0) add_row(partialF + (size_t)(12 * s + f_site(c)) * gA, gA);
+    const int k = p_site(c), d = d_site(c);
     for (int x = 0; x < ns; ++x)
         for (int y = x; y < ns; ++y) {
-            int k = p_site(c);
-            if (T.phi_f[x * ns + y] != f || k < 0 || (x == y && k >= 8)) continue;
-            idx[n++] = (x * ns + y) * EADJ_PS + k;
-            if (x != y) idx[n++] = (y * ns + x) * EADJ_PS + k;
+            const double *pp = partial + (size_t)pair_code(x, y, ns) * gP * EADJ_PS;
+            if (T.phi_f[x * ns + y] == f && k >= 0 && (x != y || k < 8)) add_row(pp + (size_t)k * gP, gP);
+            if (T.rho_f[y] == f && d >= 0) add_row(pp + (size_t)(17 + d) * gP, gP);
+            if (x != y && T.rho_f[x] == f && d >= 0) add_row(pp + (size_t)(21 + d) * gP, gP);
         }
-    double acc = 0.0;
-    if (fitem >= 0)
-        for (int b = l; b < gA; b += 32) acc += partialF[(size_t)b * nfs + fitem];
-    for (int b = l; b < gP; b += 32) {  // the like and the cross kernels' rows
-        const double *pp = partialP + (size_t)b * ni;
-        for (int q = 0; q < n; ++q) acc += pp[idx[q]];
-    }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(MBF_FULL, acc, o);
     if (l == 0) d_P[e] = acc;
@@ -459,34 +573,36 @@ __global__ void eam_adjoint_final(EamAdjTab T, int gA, const double *__restrict_
 
 // Workspace of one call.
 struct EadjLayout {
-    size_t partialF, partialP, cc, cnt, pos, pairs, scan, total;
-    int gA, gP;
+    size_t partialF, partial, cc, cnt, pos, mark, pairs, scan, total;
+    int gA, gP, nc;
 };
 
 static EadjLayout eadj_layout(int n_atoms, long long n_slots, int ns) {
     EadjLayout L;
-    long long ns2 = n_slots > 0 ? n_slots : 1;
-    int tiles_a = (int)((n_atoms + EADJ_TA - 1) / EADJ_TA);
-    long long tiles_p = (ns2 + EADJ_TP - 1) / EADJ_TP;  // the live pairs are at most the slots
-    L.gA = tiles_a < 1 ? 1 : (tiles_a < 65535 ? tiles_a : 65535);
-    L.gP = (int)(tiles_p < EADJ_GRID ? tiles_p : EADJ_GRID);  // rows per pair kernel, at most
-    if (L.gP < 1) L.gP = 1;
+    const long long ns2 = n_slots > 0 ? n_slots : 1;
+    const size_t na = (size_t)(n_atoms > 0 ? n_atoms : 1);
+    L.nc = ns * (ns + 1) / 2;
+    L.gA = (int)((na + EADJ_TA - 1) / EADJ_TA);
+    // pair blocks per list: at least a few hundred pairs each
+    const long long tiles = (ns2 / 2 + 4 * EADJ_PB - 1) / (4 * EADJ_PB);
+    L.gP = (int)(tiles < 1 ? 1 : (tiles < EADJ_PG ? tiles : EADJ_PG));
     size_t o = 0;
     L.partialF = o;
     o = align256(o + sizeof(double) * (size_t)L.gA * 12 * ns);
-    L.partialP = o;
-    o = align256(o + sizeof(double) * (size_t)2 * L.gP * ns * ns * EADJ_PS);
+    L.partial = o;
+    o = align256(o + sizeof(double) * (size_t)L.nc * L.gP * EADJ_PS);
     L.cc = o;
-    o = align256(o + sizeof(double2) * (size_t)(n_atoms > 0 ? n_atoms : 1));
-    size_t na = (size_t)(n_atoms > 0 ? n_atoms : 1);
+    o = align256(o + sizeof(double2) * na);
     L.cnt = o;
-    o = align256(o + sizeof(int) * 2 * na);
+    o = align256(o + sizeof(int) * L.nc * na);
     L.pos = o;
-    o = align256(o + sizeof(int) * (2 * na + 1));
+    o = align256(o + sizeof(int) * (L.nc * na + 1));
+    L.mark = o;
+    o = align256(o + (size_t)ns2);
     L.pairs = o;
-    o = align256(o + sizeof(int) * (size_t)ns2);
+    o = align256(o + sizeof(int2) * (size_t)(ns2 / 2 + 1));
     L.scan = o;
-    o = align256(o + sizeof(int) * scan_workspace_ints((int)(2 * na)));
+    o = align256(o + sizeof(int) * scan_workspace_ints((int)(L.nc * na)));
     L.total = o;
     return L;
 }
@@ -516,6 +632,7 @@ int mbf_eam_adjoint(const mbf_system *sys, const mbf_nlist *nl, const mbf_eam_ta
         if (cudaMemsetAsync(d_P, 0, sizeof(double) * ne, st) != cudaSuccess) return MBF_ERR_CUDA;
         return MBF_OK;
     }
+    if ((long long)L.nc * sys->n_atoms > 0x7fffff00LL) return MBF_ERR_ARGUMENT;  // the scan's integers
     SysView S = make_view(sys);
     EamAdjTab T;
     T.ns = tab->ns;
@@ -530,36 +647,38 @@ int mbf_eam_adjoint(const mbf_system *sys, const mbf_nlist *nl, const mbf_eam_ta
     G.gF = g_forces;
     G.gW = g_virial;
     double *partialF = ws_at<double>(workspace, L.partialF);
-    double *partialP = ws_at<double>(workspace, L.partialP);
+    double *partial = ws_at<double>(workspace, L.partial);
     double2 *cc = ws_at<double2>(workspace, L.cc);
     int *cnt = ws_at<int>(workspace, L.cnt);
     int *pos = ws_at<int>(workspace, L.pos);
-    int *pairs = ws_at<int>(workspace, L.pairs);
-    const int N = sys->n_atoms;
-    PROF_BEGIN("eam_adjoint_embed", st);
-    eam_adjoint_embed<<<L.gA, EADJ_TA, sizeof(double) * 12 * T.ns, st>>>(S, nl->row_off, nl->upper, nl->nbr, T, G,
-                                                                          cc, cnt, partialF);
+    unsigned char *mark = ws_at<unsigned char>(workspace, L.mark);
+    int2 *pairs = ws_at<int2>(workspace, L.pairs);
+    const int N = sys->n_atoms, ns = T.ns;
+    const int rows = (int)(((long long)N * EADJ_LPA + 127) / 128);
+    PROF_BEGIN("eam_adjoint_density", st);
+    eam_adjoint_density<<<rows, 128, 0, st>>>(S, nl->row_off, nl->upper, nl->nbr, T, G, cc, mark, cnt);
+    PROF_END("eam_adjoint_density", st);
     MBF_CHECK_LAUNCH();
-    int rc = exclusive_scan(cnt, pos, 2 * N, ws_at<int>(workspace, L.scan), st);
-    if (rc != MBF_OK) return rc;
-    eam_adjoint_compact<<<(N + 127) / 128, 128, 0, st>>>(S, nl->row_off, nl->upper, nl->nbr, T, G, pos, pairs);
+    PROF_BEGIN("eam_adjoint_embed", st);
+    eam_adjoint_embed<<<L.gA, EADJ_TA, 0, st>>>(S, T, G, cc, partialF);
     PROF_END("eam_adjoint_embed", st);
     MBF_CHECK_LAUNCH();
-    // like pairs [pos[0], pos[N]), cross pairs [pos[N], pos[2 N])
-    size_t psm = sizeof(double) * T.ns * T.ns * EADJ_PS;
-    int gL = persistent_grid(L.gP, EADJ_TP, (const void *)eam_adjoint_pairs<true>, psm);
-    int gC = persistent_grid(L.gP, EADJ_TP, (const void *)eam_adjoint_pairs<false>, psm);
-    size_t ni = (size_t)T.ns * T.ns * EADJ_PS;
+    PROF_BEGIN("eam_adjoint_compact", st);
+    int rc = exclusive_scan(cnt, pos, L.nc * N, ws_at<int>(workspace, L.scan), st);
+    if (rc != MBF_OK) return rc;
+    eam_adjoint_compact<<<rows, 128, 0, st>>>(N, ns, S.types, nl->row_off, nl->upper, nl->nbr, mark, pos, pairs);
+    PROF_END("eam_adjoint_compact", st);
+    MBF_CHECK_LAUNCH();
     PROF_BEGIN("eam_adjoint_pairs", st);
-    eam_adjoint_pairs<true><<<gL, EADJ_TP, psm, st>>>(S, nl->row_off, nl->nbr, T, G, cc, pairs, pos, pos + N,
-                                                       partialP);
+    eam_adjoint_pairs<true><<<dim3(L.gP, ns), EADJ_PB, 0, st>>>(S, T, G, cc, pairs, pos, partial);
     MBF_CHECK_LAUNCH();
-    eam_adjoint_pairs<false><<<gC, EADJ_TP, psm, st>>>(S, nl->row_off, nl->nbr, T, G, cc, pairs, pos + N, pos + 2 * N,
-                                                        partialP + (size_t)gL * ni);
+    if (ns > 1) {
+        eam_adjoint_pairs<false><<<dim3(L.gP, ns * (ns - 1) / 2), EADJ_PB, 0, st>>>(S, T, G, cc, pairs, pos, partial);
+        MBF_CHECK_LAUNCH();
+    }
     PROF_END("eam_adjoint_pairs", st);
-    MBF_CHECK_LAUNCH();
     PROF_BEGIN("eam_adjoint_reduce", st);
-    eam_adjoint_final<<<(ne * 32 + 127) / 128, 128, 0, st>>>(T, L.gA, partialF, gL + gC, partialP, d_P);
+    eam_adjoint_final<<<(ne * 32 + 127) / 128, 128, 0, st>>>(T, L.gA, partialF, L.gP, partial, d_P);
     PROF_END("eam_adjoint_reduce", st);
     MBF_CHECK_LAUNCH();
     return MBF_OK;

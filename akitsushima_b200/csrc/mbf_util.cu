@@ -78,30 +78,34 @@ __global__ void scan_tiles(const int *__restrict__ in, int *__restrict__ out, in
     if (threadIdx.x == 0) tile_sums[blockIdx.x] = total;
 }
 
-// One block: exclusive scan of the tile sums in place; writes the grand
-// total to *total.
-__global__ void scan_tile_sums(int *__restrict__ tile_sums, int n_tiles, int *__restrict__ total) {
-    int carry = 0;
-    for (int base = 0; base < n_tiles; base += blockDim.x) {
-        int i = base + threadIdx.x;
-        int v = i < n_tiles ? tile_sums[i] : 0;
-        int excl;
-        int t = block_excl_scan(v, excl);
-        if (i < n_tiles) tile_sums[i] = excl + carry;
-        carry += t;
+// Adds to each tile the sum of the tiles before it, which every block forms
+// for itself from the tile sums (at most a few thousand, in cache), so the
+// scan is two launches; the last block writes the grand total.
+__global__ void __launch_bounds__(SCAN_BLOCK) scan_add(int *__restrict__ out, int n, const int *__restrict__ tile_sums,
+                                                       int n_tiles) {
+    __shared__ int warp_sum[32];
+    __shared__ int before;
+    int v = 0;
+    for (int k = threadIdx.x; k < blockIdx.x; k += SCAN_BLOCK) v += tile_sums[k];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(MBF_FULL, v, o);
+    if ((threadIdx.x & 31) == 0) warp_sum[threadIdx.x >> 5] = v;
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        int t = warp_sum[threadIdx.x];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(MBF_FULL, t, o);
+        if (threadIdx.x == 0) before = t;
     }
-    if (threadIdx.x == 0) *total = carry;
-}
-
-__global__ void scan_add(int *__restrict__ out, int n, const int *__restrict__ tile_sums,
-                         const int *__restrict__ total) {
-    int base = blockIdx.x * SCAN_TILE;
-    int add = tile_sums[blockIdx.x];
-    for (int k = threadIdx.x; k < SCAN_TILE; k += blockDim.x) {
-        int i = base + k;
+    __syncthreads();
+    const int add = before;
+    const int base = blockIdx.x * SCAN_TILE + threadIdx.x;
+#pragma unroll
+    for (int k = 0; k < SCAN_ITEMS; ++k) {
+        const int i = base + k * SCAN_BLOCK;
         if (i < n) out[i] += add;
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0) out[n] = *total;
+    if ((int)blockIdx.x == n_tiles - 1 && threadIdx.x == 0) out[n] = add + tile_sums[n_tiles - 1];
 }
 
 size_t scan_workspace_ints(int n) { return (size_t)(n + SCAN_TILE - 1) / SCAN_TILE + 2; }
@@ -109,11 +113,8 @@ size_t scan_workspace_ints(int n) { return (size_t)(n + SCAN_TILE - 1) / SCAN_TI
 int exclusive_scan(const int *in, int *out, int n, int *ws, cudaStream_t st) {
     int n_tiles = (n + SCAN_TILE - 1) / SCAN_TILE;
     if (n_tiles == 0) n_tiles = 1;
-    int *tile_sums = ws;
-    int *total = ws + n_tiles;
-    scan_tiles<<<n_tiles, SCAN_BLOCK, 0, st>>>(in, out, n, tile_sums);
-    scan_tile_sums<<<1, SCAN_BLOCK, 0, st>>>(tile_sums, n_tiles, total);
-    scan_add<<<n_tiles, 256, 0, st>>>(out, n, tile_sums, total);
+    scan_tiles<<<n_tiles, SCAN_BLOCK, 0, st>>>(in, out, n, ws);
+    scan_add<<<n_tiles, SCAN_BLOCK, 0, st>>>(out, n, ws, n_tiles);
     MBF_CHECK_LAUNCH();
     return MBF_OK;
 }

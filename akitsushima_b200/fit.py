@@ -813,34 +813,40 @@ class _EamTableEval:
         self.ns = len(skeleton["rho_f"])
         self.nf = len(skeleton["codes"])
         self.fused = 1 if skeleton["fused"] else 0
+        self._fid = {k: np.ascontiguousarray(skeleton[k], dtype=np.int32) for k in ("rho_f", "phi_f")}
         self._ws = None
         self._adj_ws = None
         self.lanes = 2
 
-    def _tab(self, P):
+    def _tab(self, P, P_host=None):
+        """The table's C view; with a host copy of P a one- or two-element
+        set is evaluated with its constants as kernel arguments."""
         k = self.keep
+        host = [None] * 3 if P_host is None else [P_host.ctypes.data] + [self._fid[q].ctypes.data
+                                                                        for q in ("rho_f", "phi_f")]
         return _lib.MbfEamTables(self.ns, self.nf, int(k["X"].shape[0]), _lib.ptr(k["codes"]), _lib.ptr(P),
                                  _lib.ptr(k["xo"]), _lib.ptr(k["nx"]), _lib.ptr(k["X"]), _lib.ptr(k["C"]),
                                  _lib.ptr(k["rho_f"]), _lib.ptr(k["F_f"]), _lib.ptr(k["phi_f"]), self.r_cut,
-                                 self.fused)
+                                 self.fused, *host)
 
-    def autotune(self, P, candidates=(1, 2, 4, 8), reps=3):
+    def autotune(self, P, candidates=(1, 2, 4, 8), reps=3, P_host=None):
         """Keep the fastest lanes-per-atom of the evaluation (CUDA events)."""
         times = {}
         for c in candidates:
             self.lanes = c
-            self.evaluate(P)
+            self.evaluate(P, P_host)
             a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
             a.record()
             for _ in range(reps):
-                self.evaluate(P)
+                self.evaluate(P, P_host)
             b.record()
             b.synchronize()
             times[c] = a.elapsed_time(b) / reps
         self.lanes = min(candidates, key=lambda c: (times[c], c))
         return {"lanes_per_atom": self.lanes, "ms": times}
 
-    def evaluate(self, P):
+    def evaluate(self, P, P_host=None):
+        """``P_host``: the same rows as a C-contiguous float64 numpy array."""
         b, dl = self.batch, self.dlist
         dev = b.device
         L = _lib.lib()
@@ -851,7 +857,7 @@ class _EamTableEval:
         F = torch.empty((b.n_atoms, 3), dtype=torch.float64, device=dev)
         W = torch.empty((b.n_struct, 9), dtype=torch.float64, device=dev)
         st = torch.cuda.current_stream(dev).cuda_stream
-        _lib.check(L.mbf_eam_eval(b.mbf_system(), dl.mbf_nlist(), self._tab(P), b.reduce_plan(), _lib.MBF_FP64,
+        _lib.check(L.mbf_eam_eval(b.mbf_system(), dl.mbf_nlist(), self._tab(P, P_host), b.reduce_plan(), _lib.MBF_FP64,
                                   self.lanes, _lib.ptr(self._ws), self._ws.numel(), _lib.ptr(F), _lib.ptr(E),
                                   _lib.ptr(W), st), "mbf_eam_eval")
         return E, F, W
@@ -962,14 +968,14 @@ class _ZhouModel:
 
     def evaluator(self, batch, skin):
         ev = _EamTableEval(batch, skin, self.ps.potential().function_table(), self.ps.r_cut)
-        P0 = self.ps.table_torch(torch.as_tensor(self.ps.x0)).to(batch.device)
-        return ev, ev.autotune(P0)
+        P0 = self.ps.table_torch(torch.as_tensor(self.ps.x0)).contiguous()
+        return ev, ev.autotune(P0.to(batch.device), P_host=P0.numpy())
 
     def efs(self, x_t, ev):
         return EamEFS.apply(self.ps.table_torch(x_t), ev)
 
     def evaluate(self, ev, dtabs, tabs):
-        return ev.evaluate(dtabs[0])
+        return ev.evaluate(dtabs[0], np.ascontiguousarray(tabs[0]))
 
     def adjoint(self, ev, dtabs, tabs, gE, gF, gW):
         return (ev.adjoint(dtabs[0], gE, gF, gW),)
