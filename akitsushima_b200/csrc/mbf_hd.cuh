@@ -139,46 +139,9 @@ __device__ __forceinline__ HD<K> hd_log(const HD<K> &a) {
     return hd_apply<K>(a, log(a.v), i, -i * i);
 }
 
-template <int K>
-__device__ __forceinline__ HD<K> hd_sin(const HD<K> &a) {
-    double s = sin(a.v), c = cos(a.v);
-    return hd_apply<K>(a, s, c, -s);
-}
-
-// exp clamped as the reference's _nb_exp (engine/_numba_common.py:12-33):
-// constant outside [-500, 500].
-template <int K>
-__device__ __forceinline__ HD<K> hd_cexp(const HD<K> &a) {
-    if (a.v > 500.0) return hd_const<K>(exp(500.0));
-    if (a.v < -500.0) return hd_const<K>(0.0);
-    return hd_exp<K>(a);
-}
-
-template <int K>
-__device__ __forceinline__ HD<K> hd_pow(const HD<K> &x, const HD<K> &y) {
-    return hd_exp<K>(y * hd_log<K>(x));
-}
-
 // Upstream gradients of the adjoint entries.
 struct AdjIn {
     const double *gE, *gF, *gW;  // (S,), (N, 3), (S, 9); null = 0
 };
-
-// Pair vector, its length and its tangent t = gF_i - gF_j - gW d.
-__device__ __forceinline__ void adj_leg(const SysView &S, const AdjIn &G, const double *cell, int i, int j,
-                                        int s_struct, double d[3], double &r, double tg[3]) {
-    mic_exact(cell, S.pos[3 * (size_t)j] - S.pos[3 * (size_t)i], S.pos[3 * (size_t)j + 1] - S.pos[3 * (size_t)i + 1],
-              S.pos[3 * (size_t)j + 2] - S.pos[3 * (size_t)i + 2], d[0], d[1], d[2]);
-    r = sqrt(d[0] * d[0] + d[1] * d[1] + d[2] * d[2]);
-    for (int a = 0; a < 3; ++a) {
-        double t = 0.0;
-        if (G.gF) t = G.gF[3 * (size_t)i + a] - G.gF[3 * (size_t)j + a];
-        if (G.gW) {
-            const double *w = G.gW + 9 * (size_t)s_struct + 3 * a;
-            t -= w[0] * d[0] + w[1] * d[1] + w[2] * d[2];
-        }
-        tg[a] = t;
-    }
-}
 
 }  // namespace mbf
