@@ -44,9 +44,15 @@ static NlLayout nl_layout(int n_atoms, int n_cells) {
     return L;
 }
 
-// The rebuild's staging rows (n_atoms x max_row_limit ints) after the layout.
+// Behind the layout, where the workspace has room: the block search's local
+// coordinates (a float4 per atom), then the staging rows (n_atoms x
+// max_row_limit ints).
+static size_t nl_local_bytes(int n_atoms) { return align256(sizeof(float4) * (size_t)n_atoms); }
+
+static bool nl_local_ok(const void *workspace) { return ((size_t)workspace & (sizeof(float4) - 1)) == 0; }
+
 static size_t nl_staged_bytes(const NlLayout &L, int n_atoms, int max_row_limit) {
-    return L.total + align256(sizeof(int) * (size_t)n_atoms * (size_t)max_row_limit);
+    return L.total + nl_local_bytes(n_atoms) + align256(sizeof(int) * (size_t)n_atoms * (size_t)max_row_limit);
 }
 
 // Bin every atom: fractional coordinate wrapped to [0, 1), sub-cell index
@@ -177,88 +183,434 @@ __device__ __forceinline__ bool pair_hit_diag(double d0, double d1, double d2, d
     return r2 < rl2 && r2 > 1e-20;
 }
 
-// MODE 0 counts each atom's neighbours (row_cnt, max_row); MODE 1 writes
-// them into the CSR rows (row_off, nbr); MODE 2 counts and writes them at a
-// fixed stride into a staging array (`nbr` = stage, row a at a * stride,
-// at most stride entries kept), so one pass serves a list of known row
-// bound.
+// The rows of atoms [q_begin, q_end) of one cell by one warp, with the exact
+// test on every candidate of the stencil.  MODE 0 counts each atom's
+// neighbours (row_cnt); MODE 1 writes them into the CSR rows (row_off, nbr);
+// MODE 2 counts and writes them at a fixed stride into a staging array
+// (`nbr` = stage, row a at a * stride, at most stride entries kept), so one
+// pass serves a list of known row bound.  Returns the longest row it counted
+// (per lane).
+template <int MODE>
+__device__ __forceinline__ int cell_rows_exact(const SysView &S, const double *__restrict__ cell, const Stencil &st,
+                                               int total, const int *__restrict__ cell_atoms, int cs, int q_begin,
+                                               int q_end, double rl2, int *__restrict__ row_cnt,
+                                               const int *__restrict__ row_off, int *__restrict__ nbr, int stride) {
+    constexpr bool FILL = MODE != 0, COUNT = MODE != 1;
+    const int lane = threadIdx.x & 31;
+    const bool diag = cell_is_diagonal(cell);
+    const double d0 = cell[9], d1 = cell[13], d2 = cell[17], l0 = cell[0], l1 = cell[4], l2 = cell[8];
+    int longest = 0;
+    for (int q0 = q_begin; q0 < q_end; q0 += 32) {
+        int nq = min(32, q_end - q0);
+        int a_l = lane < nq ? cell_atoms[cs + q0 + lane] : 0;
+        double xa_l = S.pos[3 * (size_t)a_l], ya_l = S.pos[3 * (size_t)a_l + 1], za_l = S.pos[3 * (size_t)a_l + 2];
+        int cnt = 0;       // lane q: neighbours of atom q found so far
+        int beg_l = 0, len_l = 0;
+        if (FILL && lane < nq) {
+            beg_l = MODE == 1 ? row_off[a_l] : a_l * stride;
+            len_l = MODE == 1 ? row_off[a_l + 1] - beg_l : stride;
+        }
+        for (int t0 = 0; t0 < total; t0 += 32) {
+            int t = t0 + lane;
+            int b = -1;
+            double xb = 0, yb = 0, zb = 0;
+            if (t < total) {
+                b = stencil_atom(st, cell_atoms, t);
+                xb = S.pos[3 * (size_t)b];
+                yb = S.pos[3 * (size_t)b + 1];
+                zb = S.pos[3 * (size_t)b + 2];
+            }
+            // the cell's atoms against this round's candidates, with
+            // the test specialised once per cell (warp-uniform)
+            auto rounds = [&](auto diag_tag) {
+                constexpr bool DIAG = decltype(diag_tag)::value;
+                for (int q = 0; q < nq; ++q) {
+                    int a = __shfl_sync(MBF_FULL, a_l, q);
+                    double xa = __shfl_sync(MBF_FULL, xa_l, q), ya = __shfl_sync(MBF_FULL, ya_l, q),
+                           za = __shfl_sync(MBF_FULL, za_l, q);
+                    bool hit = b >= 0 && b != a &&
+                               (DIAG ? pair_hit_diag(d0, d1, d2, l0, l1, l2, xa, ya, za, xb, yb, zb, rl2)
+                                     : pair_hit(cell, xa, ya, za, xb, yb, zb, rl2));
+                    unsigned m = __ballot_sync(MBF_FULL, hit);
+                    if (FILL) {
+                        int w = __shfl_sync(MBF_FULL, cnt, q);
+                        int beg = __shfl_sync(MBF_FULL, beg_l, q), len = __shfl_sync(MBF_FULL, len_l, q);
+                        if (hit) {
+                            int pos = w + __popc(m & ((1u << lane) - 1u));
+                            if (pos < len) nbr[beg + pos] = b;
+                        }
+                    }
+                    if (lane == q) cnt += __popc(m);
+                }
+            };
+            if (diag)
+                rounds(std::true_type{});
+            else
+                rounds(std::false_type{});
+        }
+        if (COUNT && lane < nq) {
+            row_cnt[a_l] = cnt;
+            longest = max(longest, cnt);
+        }
+    }
+    return longest;
+}
+
+// A warp per cell: cells of few atoms, and those the block search left.
 template <int MODE>
 __global__ void nl_cells(SysView S, const int *__restrict__ grids, const int *__restrict__ cell_start,
                          const int *__restrict__ cell_atoms, int n_cells, double rl2, int *__restrict__ row_cnt,
                          int *__restrict__ max_row, const int *__restrict__ row_off, int *__restrict__ nbr,
-                         int stride) {
-    constexpr bool FILL = MODE != 0, COUNT = MODE != 1;
+                         int stride, const int *__restrict__ done) {
     __shared__ Stencil sst[NL_WARPS];
     int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
     Stencil &st = sst[wid];
+    int longest = 0;
     for (int c = blockIdx.x * NL_WARPS + wid; c < n_cells; c += gridDim.x * NL_WARPS) {
         int cs = cell_start[c], na = cell_start[c + 1] - cs;
-        if (na == 0) continue;  // uniform over the warp
-        int a0 = cell_atoms[cs];
-        int sidx = S.n_struct > 1 ? S.atom_struct[a0] : 0;
+        if (na == 0 || (done && done[c])) continue;  // uniform over the warp
+        int sidx = S.n_struct > 1 ? S.atom_struct[cell_atoms[cs]] : 0;
         int total = build_stencil_of_cell(grids, cell_start, sidx, c, st);
-        const double *cell = S.cells + 18 * (size_t)sidx;
-        const bool diag = cell_is_diagonal(cell);
-        const double d0 = cell[9], d1 = cell[13], d2 = cell[17], l0 = cell[0], l1 = cell[4], l2 = cell[8];
-        for (int q0 = 0; q0 < na; q0 += 32) {
-            int nq = min(32, na - q0);
-            int a_l = lane < nq ? cell_atoms[cs + q0 + lane] : 0;
-            double xa_l = S.pos[3 * (size_t)a_l], ya_l = S.pos[3 * (size_t)a_l + 1], za_l = S.pos[3 * (size_t)a_l + 2];
-            int cnt = 0;       // lane q: neighbours of atom q found so far
-            int beg_l = 0, len_l = 0;
-            if (FILL && lane < nq) {
-                beg_l = MODE == 1 ? row_off[a_l] : a_l * stride;
-                len_l = MODE == 1 ? row_off[a_l + 1] - beg_l : stride;
-            }
-            for (int t0 = 0; t0 < total; t0 += 32) {
-                int t = t0 + lane;
-                int b = -1;
-                double xb = 0, yb = 0, zb = 0;
-                if (t < total) {
-                    b = stencil_atom(st, cell_atoms, t);
-                    xb = S.pos[3 * (size_t)b];
-                    yb = S.pos[3 * (size_t)b + 1];
-                    zb = S.pos[3 * (size_t)b + 2];
-                }
-                // the cell's atoms against this round's candidates, with
-                // the test specialised once per cell (warp-uniform)
-                auto rounds = [&](auto diag_tag) {
-                    constexpr bool DIAG = decltype(diag_tag)::value;
-                    for (int q = 0; q < nq; ++q) {
-                        int a = __shfl_sync(MBF_FULL, a_l, q);
-                        double xa = __shfl_sync(MBF_FULL, xa_l, q), ya = __shfl_sync(MBF_FULL, ya_l, q),
-                               za = __shfl_sync(MBF_FULL, za_l, q);
-                        bool hit = b >= 0 && b != a &&
-                                   (DIAG ? pair_hit_diag(d0, d1, d2, l0, l1, l2, xa, ya, za, xb, yb, zb, rl2)
-                                         : pair_hit(cell, xa, ya, za, xb, yb, zb, rl2));
-                        unsigned m = __ballot_sync(MBF_FULL, hit);
-                        if (FILL) {
-                            int w = __shfl_sync(MBF_FULL, cnt, q);
-                            int beg = __shfl_sync(MBF_FULL, beg_l, q), len = __shfl_sync(MBF_FULL, len_l, q);
-                            if (hit) {
-                                int pos = w + __popc(m & ((1u << lane) - 1u));
-                                if (pos < len) nbr[beg + pos] = b;
-                            }
-                        }
-                        if (lane == q) cnt += __popc(m);
-                    }
-                };
-                if (diag)
-                    rounds(std::true_type{});
-                else
-                    rounds(std::false_type{});
-            }
-            if (COUNT && lane < nq) {
-                row_cnt[a_l] = cnt;
-                atomicMax(max_row, cnt);
-            }
-        }
+        longest = max(longest, cell_rows_exact<MODE>(S, S.cells + 18 * (size_t)sidx, st, total, cell_atoms, cs, 0, na,
+                                                     rl2, row_cnt, row_off, nbr, stride));
+    }
+    if (MODE != 1) {
+        longest = __reduce_max_sync(MBF_FULL, longest);
+        if (lane == 0) atomicMax(max_row, longest);
     }
 }
 
+// A block per cell, for cells of many atoms: counts and stages as MODE 2.
+// The stencil's candidates are put into ascending atom index once per cell, so
+// every row comes out ascending: each sets its bit in a map of the index range
+// that they span, and its rank is the number of bits below its own.  The range
+// is taken around the end of the index (modulo n_atoms), so a stencil over the
+// periodic boundary spans no more of a lattice-ordered structure than one
+// inside it.
+// They are tested in float32 against the cell's atoms, up to NL_NA atoms a
+// warp at a time, in coordinates relative to the cell's middle (`local`, each
+// atom relative to the middle of its own cell, plus the stencil offset).  A
+// squared distance within `margin` of r_list^2 or of 0 is decided by the exact
+// test, so the pair set is the same.  Coordinates are below
+// M = 1.5 sum_k |L_k|_1 / nc_k and off by less than 2^-23 M, so the squared
+// distance of a pair near r = r_list is off by less than
+// 2 sqrt(3) r (2^-22 M + 2^-24 r) + 4 * 2^-24 r^2 < r (M + r) 2^-20; the
+// margin is four times that.  From five cells on each axis two atoms of a
+// stencil are at most 0.4 of the box apart, so the offset's image is the one
+// the minimum image rounds to.  Other cells, cells of more than NL_CAP
+// candidates or a range beyond NL_BITS, and cells near an atom more than 4096
+// boxes away (where the wrap itself loses digits) are left to nl_cells
+// (done = 0).
+//
+// Issue-bound, the rank and the tests about half each: 256,000 Cu-Ni atoms at
+// 80 neighbours (21 atoms a cell, 27 x 21 candidates, 62 % of them kept) take
+// 276 us and leave 66 for the rows' copy into the CSR; a warp per cell with
+// the exact test on every candidate took 463 and left 198 for the rows'
+// sorts.  Merging the 27 runs in shared memory instead of ranking by bits
+// took 240 us alone.  Atoms a warp: 3 as 4 (279), 2 worse (the candidates are
+// read once for all); 128 threads 316, 512 threads 315; at 5 blocks an SM the
+// registers spill (320).
+constexpr int NL_T = 256, NL_NW = NL_T / 32;
+constexpr int NL_CAP = 1024;   // candidates a block ranks
+constexpr int NL_BITS = 1 << 17;   // index range they may span: 32 x 32 groups of 128 bits
+constexpr int NL_NA = 4;       // atoms a warp tests at a time
+
+__device__ __forceinline__ bool grid_is_wide(const int *__restrict__ g) {
+    return g[0] >= 5 && g[1] >= 5 && g[2] >= 5 && g[4] == 3 && g[5] == 3 && g[6] == 3;
+}
+
+// The rows of NA atoms (cand[own[0]], cand[own[NL_NW]], ...) by one warp, every
+// candidate against each; returns the longest.
+template <int NA>
+__device__ __forceinline__ int test_rows(const SysView &S, const double *__restrict__ cell, const float4 *cand,
+                                         const unsigned short *own, int total, float lo2, float hi2, double r_list,
+                                         int *__restrict__ row_cnt, int *__restrict__ stage, int stride) {
+    const int lane = threadIdx.x & 31;
+    const unsigned below = (1u << lane) - 1u;
+    const float tiny = 0.5f * (hi2 - lo2);
+    float ax[NA], ay[NA], az[NA];
+    int a[NA], cnt[NA];
+    int *out[NA];
+#pragma unroll
+    for (int i = 0; i < NA; ++i) {
+        const float4 v = cand[own[i * NL_NW]];
+        ax[i] = v.x;
+        ay[i] = v.y;
+        az[i] = v.z;
+        a[i] = __float_as_int(v.w);
+        cnt[i] = 0;
+        out[i] = stage + (size_t)a[i] * stride;
+    }
+    for (int t = lane; t < total + lane; t += 32) {  // the last round reads padding
+        const float4 v = cand[t];
+        const int b = __float_as_int(v.w);
+        bool hit[NA], near[NA], any = false;
+#pragma unroll
+        for (int i = 0; i < NA; ++i) {
+            const float dx = v.x - ax[i], dy = v.y - ay[i], dz = v.z - az[i];
+            const float r2 = dx * dx + dy * dy + dz * dz;
+            hit[i] = r2 < lo2 && r2 > tiny;
+            near[i] = r2 < hi2 && !hit[i] && b != a[i];
+            any = any || near[i];
+        }
+        if (any) {  // seldom
+            const double *pb = S.pos + 3 * (size_t)b;
+#pragma unroll
+            for (int i = 0; i < NA; ++i)
+                if (near[i]) {
+                    const double *pa = S.pos + 3 * (size_t)a[i];
+                    hit[i] = pair_hit(cell, pa[0], pa[1], pa[2], pb[0], pb[1], pb[2], r_list * r_list);
+                }
+        }
+#pragma unroll
+        for (int i = 0; i < NA; ++i) {
+            const unsigned m = __ballot_sync(MBF_FULL, hit[i]);
+            const int p = cnt[i] + __popc(m & below);
+            if (hit[i] && p < stride) out[i][p] = b;
+            cnt[i] += __popc(m);
+        }
+    }
+    int longest = 0;
+#pragma unroll
+    for (int i = 0; i < NA; ++i) {
+        if (lane == 0) row_cnt[a[i]] = cnt[i];
+        longest = max(longest, cnt[i]);
+    }
+    return longest;
+}
+
+__global__ void __launch_bounds__(NL_T, 4) nl_search(SysView S, const int *__restrict__ grids,
+                                                  const int *__restrict__ cell_start,
+                                                  const float4 *__restrict__ local, int n_cells, double r_list,
+                                                  int *__restrict__ row_cnt, int *__restrict__ max_row,
+                                                  int *__restrict__ stage, int stride, int *__restrict__ done) {
+    __shared__ Stencil st;
+    __shared__ float4 cand[NL_CAP];             // x, y, z, atom; ascending
+    __shared__ uint4 bits[NL_BITS / 128];       // all zero between cells
+    __shared__ ushort4 before[NL_BITS / 128];   // bits set before each word, in its chunk of 128 words
+    __shared__ int chunk[32], ahead_w[NL_NW][32];  // bits set in a chunk, and before it (each warp's copy)
+    __shared__ unsigned short own[NL_CAP];      // place in cand of the cell's atoms
+    __shared__ float3 offset[27];               // of the stencil's cells
+    __shared__ float bound[2];                  // lower and upper squared radius
+    __shared__ float box[6];                    // of the cell's atoms
+    __shared__ int base_sh, range_sh;
+    const int tid = threadIdx.x, wid = tid >> 5, lane = tid & 31;
+    const int N = S.n_atoms;
+    unsigned *word = (unsigned *)bits;
+    const unsigned short *word_before = (const unsigned short *)before;
+    for (int k = tid; k < NL_BITS / 128; k += NL_T) bits[k] = make_uint4(0, 0, 0, 0);
+    int longest = 0;
+    for (int c = blockIdx.x; c < n_cells; c += gridDim.x) {
+        const int cs = cell_start[c], na = cell_start[c + 1] - cs;
+        if (na == 0) continue;  // uniform over the block
+        const int mid = __float_as_int(local[cs + na / 2].w);
+        const int sidx = S.n_struct > 1 ? S.atom_struct[mid] : 0;
+        const double *cell = S.cells + 18 * (size_t)sidx;
+        const int *g = grids + 8 * sidx;
+        __syncthreads();  // the previous cell's readers are done
+        if (wid == 0) {
+            build_stencil_of_cell(grids, cell_start, sidx, c, st);
+            // the range of atom indices, counted from half an index below the
+            // cell's middle atom; in a (sorted) cell the indices from there
+            // to the end of the index come first
+            int base = mid - N / 2;
+            base += base < 0 ? N : 0;
+            const int beg = st.start[lane], len = st.pre[lane + 1] - st.pre[lane];
+            int lo = 0, hi = len;  // entries below base
+            if (len && __float_as_int(local[beg].w) >= base) hi = 0;
+            if (len && __float_as_int(local[beg + len - 1].w) < base) lo = len;
+            while (lo < hi) {
+                const int m = (lo + hi) >> 1;
+                if (__float_as_int(local[beg + m].w) < base) lo = m + 1; else hi = m;
+            }
+            int low = N, high = 0;
+            if (len) {
+                low = __float_as_int(local[beg + (lo < len ? lo : 0)].w) - base;
+                high = __float_as_int(local[beg + (lo > 0 ? lo : len) - 1].w) - base;
+                low += low < 0 ? N : 0;
+                high += high < 0 ? N : 0;
+            }
+            low = __reduce_min_sync(MBF_FULL, low);
+            high = __reduce_max_sync(MBF_FULL, high);
+            if (lane == 0) {
+                base += low;
+                base_sh = base - (base >= N ? N : 0);
+                range_sh = high - low;
+            }
+        }
+        if (wid == 1) {
+            const double s = lane < 9 ? cell[lane] / (double)g[lane / 3] : 0.0;
+            double M = 1.5 * fabs(s);
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) M += __shfl_xor_sync(MBF_FULL, M, o);
+            const float margin = (float)(r_list * (M + r_list) * 0x1p-18);
+            if (lane < 2) bound[lane] = (float)(r_list * r_list) + (lane ? margin : -margin);
+            const float sf = (float)s;
+            float o[3];
+#pragma unroll
+            for (int k = 0; k < 3; ++k)
+                o[k] = (float)(lane / 9 - 1) * __shfl_sync(MBF_FULL, sf, k) +
+                       (float)((lane / 3) % 3 - 1) * __shfl_sync(MBF_FULL, sf, 3 + k) +
+                       (float)(lane % 3 - 1) * __shfl_sync(MBF_FULL, sf, 6 + k);
+            if (lane < 27) offset[lane] = make_float3(o[0], o[1], o[2]);
+        }
+        if (wid == 2) {
+            float lo[3] = {1e30f, 1e30f, 1e30f}, hi[3] = {-1e30f, -1e30f, -1e30f};
+            for (int k = lane; k < na; k += 32) {
+                const float4 q = local[cs + k];
+                lo[0] = fminf(lo[0], q.x), hi[0] = fmaxf(hi[0], q.x);
+                lo[1] = fminf(lo[1], q.y), hi[1] = fmaxf(hi[1], q.y);
+                lo[2] = fminf(lo[2], q.z), hi[2] = fmaxf(hi[2], q.z);
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+                for (int k = 0; k < 3; ++k) {
+                    lo[k] = fminf(lo[k], __shfl_xor_sync(MBF_FULL, lo[k], o));
+                    hi[k] = fmaxf(hi[k], __shfl_xor_sync(MBF_FULL, hi[k], o));
+                }
+            if (lane == 0)
+#pragma unroll
+                for (int k = 0; k < 3; ++k) {
+                    box[k] = lo[k];
+                    box[3 + k] = hi[k];
+                }
+        }
+        __syncthreads();
+        const int base = base_sh, range = range_sh;
+        int total = 0;
+        bool wide = grid_is_wide(g) && na <= NL_CAP && range < NL_BITS && bound[0] > 0.0f && bound[1] < 1e30f;
+        if (wide) {
+            // candidates within r_list of the box of the cell's atoms
+            bool far = false;
+            const float reach = bound[1];
+            for (int run = wid; run < 27; run += NL_NW) {
+                const int beg = st.start[run], len = st.pre[run + 1] - st.pre[run];
+                const float3 o = offset[run];
+                for (int k = lane; k < len; k += 32) {
+                    const float4 q = local[beg + k];
+                    const float x0 = q.x + o.x, x1 = q.y + o.y, x2 = q.z + o.z;
+                    const float e0 = fmaxf(fmaxf(box[0] - x0, x0 - box[3]), 0.0f);
+                    const float e1 = fmaxf(fmaxf(box[1] - x1, x1 - box[4]), 0.0f);
+                    const float e2 = fmaxf(fmaxf(box[2] - x2, x2 - box[5]), 0.0f);
+                    far = far || q.x != q.x;
+                    if (e0 * e0 + e1 * e1 + e2 * e2 >= reach) continue;
+                    const int v = __float_as_int(q.w), x = v - base + (v < base ? N : 0);
+                    atomicOr(word + (x >> 5), 1u << (x & 31));
+                }
+            }
+            wide = !__syncthreads_or(far);
+            for (int k = wid; k < 32; k += NL_NW) {
+                int sum = 0;
+                if (k << 12 <= range) {
+                    const uint4 w = bits[k * 32 + lane];
+                    const int n0 = __popc(w.x), n1 = n0 + __popc(w.y), n2 = n1 + __popc(w.z), n = n2 + __popc(w.w);
+                    sum = n;
+#pragma unroll
+                    for (int o = 1; o < 32; o <<= 1) {
+                        const int t = __shfl_up_sync(MBF_FULL, sum, o);
+                        if (lane >= o) sum += t;
+                    }
+                    const int b = sum - n;
+                    before[k * 32 + lane] = make_ushort4(b, b + n0, b + n1, b + n2);
+                }
+                if (lane == 31) chunk[k] = sum;
+            }
+            __syncthreads();
+            int ahead = chunk[lane];  // lane k: bits set before chunk k
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int t = __shfl_up_sync(MBF_FULL, ahead, o);
+                if (lane >= o) ahead += t;
+            }
+            ahead_w[wid][lane] = ahead - chunk[lane];
+            total = __shfl_sync(MBF_FULL, ahead, 31);
+            wide = wide && total <= NL_CAP;
+        }
+        if (tid == 0) done[c] = wide ? 1 : 0;
+        if (!wide) {  // uniform over the block
+            if (range < NL_BITS)
+                for (int k = tid; k <= range >> 7; k += NL_T) bits[k] = make_uint4(0, 0, 0, 0);
+            continue;
+        }
+        {
+            // bits set below place x of the range
+            auto rank = [&](int x) {
+                return ahead_w[wid][x >> 12] + word_before[x >> 5] + __popc(word[x >> 5] & ((1u << (x & 31)) - 1u));
+            };
+            // the atoms below the base, at the range's far end, come first
+            const int front = N - base <= range ? total - rank(N - base) : 0;
+            for (int run = wid; run < 27; run += NL_NW) {
+                const int beg = st.start[run], len = st.pre[run + 1] - st.pre[run];
+                const float3 o = offset[run];
+                for (int k = lane; k < len; k += 32) {
+                    const float4 q = local[beg + k];
+                    const int v = __float_as_int(q.w), x = v - base + (v < base ? N : 0);
+                    if (!(word[x >> 5] >> (x & 31) & 1u)) continue;
+                    const int at = rank(x) + (v < base ? front - total : front);
+                    cand[at] = make_float4(q.x + o.x, q.y + o.y, q.z + o.z, q.w);
+                    if (run == 13) own[k] = (unsigned short)at;
+                }
+            }
+            if (tid < (-total & 31)) cand[total + tid] = make_float4(1e30f, 1e30f, 1e30f, 0.0f);
+            __syncthreads();
+            for (int k = tid; k < total; k += NL_T) {
+                const int v = __float_as_int(cand[k].w), x = v - base + (v < base ? N : 0);
+                word[x >> 5] = 0;
+            }
+        }
+        const float lo2 = bound[0], hi2 = bound[1];
+        for (int q = wid; q < na; q += NL_NW * NL_NA) {
+            const int n = min(NL_NA, (na - q + NL_NW - 1) / NL_NW);
+            int most = 0;
+            if (n == 4)
+                most = test_rows<4>(S, cell, cand, own + q, total, lo2, hi2, r_list, row_cnt, stage, stride);
+            else if (n == 3)
+                most = test_rows<3>(S, cell, cand, own + q, total, lo2, hi2, r_list, row_cnt, stage, stride);
+            else if (n == 2)
+                most = test_rows<2>(S, cell, cand, own + q, total, lo2, hi2, r_list, row_cnt, stage, stride);
+            else
+                most = test_rows<1>(S, cell, cand, own + q, total, lo2, hi2, r_list, row_cnt, stage, stride);
+            longest = max(longest, most);
+        }
+    }
+    if (lane == 0) atomicMax(max_row, longest);
+}
+
+// The search: with room for the staging rows and the local coordinates a block
+// per cell from NL_BLOCK_ATOMS atoms a cell; the cells that leaves, and all
+// others, a warp each.  A block pays about 12 ns a cell for its ranking, a
+// warp for every candidate again with each atom and for the row sorts later:
+// lists of 64,000 diamond atoms take 374 us by blocks and 102 by warps at 2
+// atoms a cell, 190 and 138 at 7, 167 and 178 at 11, 171 and 256 at 19; of
+// 4,000 atoms the lines cross at 6 a cell.
+constexpr int NL_BLOCK_ATOMS = 10;
+
+static bool nl_blocks(int n_atoms, int n_cells, const float4 *local) {
+    return local && (long long)n_atoms >= (long long)NL_BLOCK_ATOMS * n_cells;
+}
+
+template <int MODE>
+static int nl_rows(const SysView &S, const int *grids, const int *cell_start, const int *cell_atoms,
+                   const float4 *local, int n_cells, double r_list, int *row_cnt, int *max_row, const int *row_off,
+                   int *nbr, int stride, int *done, cudaStream_t st) {
+    if (MODE == 2 && nl_blocks(S.n_atoms, n_cells, local)) {
+        const int g = persistent_grid(n_cells, NL_T, (const void *)nl_search);
+        nl_search<<<g, NL_T, 0, st>>>(S, grids, cell_start, local, n_cells, r_list, row_cnt, max_row, nbr, stride,
+                                      done);
+    } else {
+        done = nullptr;
+    }
+    const int g = persistent_grid((n_cells + NL_WARPS - 1) / NL_WARPS, 32 * NL_WARPS, (const void *)nl_cells<MODE>);
+    nl_cells<MODE><<<g, 32 * NL_WARPS, 0, st>>>(S, grids, cell_start, cell_atoms, n_cells, r_list * r_list, row_cnt,
+                                                max_row, row_off, nbr, stride, done);
+    MBF_CHECK_LAUNCH();
+    return MBF_OK;
+}
+
 // ---- row sorts -----------------------------------------------------------------
-// Rows come out of the search in traversal order; the CSR keeps them
-// ascending.  By length n: up to 32 entries one per lane, ranked by
+// Rows come out of nl_cells in traversal order; the CSR keeps them ascending
+// (nl_search's are).  By length n: up to 32 entries one per lane, ranked by
 // shuffles; up to 64 or 128 a bitonic network in registers over J = 2 or 4
 // entries a lane (entry e = J lane + j, padded with INT_MAX, which sorts
 // last since atom indices are smaller); longer rows by rank in shared
@@ -322,6 +674,30 @@ __device__ __forceinline__ int sort_row_bitonic(const int *src, int n, int *out,
 __device__ __forceinline__ int sort_row(const int *src, int n, int *out, int a, int *row) {
     int lane = threadIdx.x & 31;
     int lower = 0;
+    // a row that is ascending already (the block search's) is only copied;
+    // any other is sorted below, over what was copied
+    bool asc = true;
+    int prev = -1;
+    for (int k0 = 0; k0 < n; k0 += 128) {
+        int v[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int k = k0 + 32 * j + lane;
+            v[j] = k < n ? src[k] : NL_PAD;
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int k = k0 + 32 * j + lane;
+            const int u = __shfl_up_sync(MBF_FULL, v[j], 1);
+            asc = asc && (k >= n || (lane ? u : prev) < v[j]);
+            prev = __shfl_sync(MBF_FULL, v[j], 31);
+            if (k < n && src != out) out[k] = v[j];
+            lower += k < n && v[j] < a ? 1 : 0;
+        }
+    }
+    if (__all_sync(MBF_FULL, asc)) return __reduce_add_sync(MBF_FULL, lower);
+    __syncwarp();
+    lower = 0;
     if (n <= 32) {
         int v = lane < n ? src[lane] : NL_PAD, rank = 0;
         for (int q = 0; q < n; ++q) rank += __shfl_sync(MBF_FULL, v, q) < v ? 1 : 0;
@@ -344,16 +720,19 @@ __device__ __forceinline__ int sort_row(const int *src, int n, int *out, int a, 
         }
         __syncwarp();
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) lower += __shfl_xor_sync(MBF_FULL, lower, o);
-    return lower;
+    return __reduce_add_sync(MBF_FULL, lower);
 }
 
 // Each cell's atoms in ascending index order, so the traversal (and the
 // rows it produces) do not depend on the order of nl_fill_cells's atomics:
 // a warp per cell, the row sort above (a cell beyond NL_MAXROW atoms, which
 // no physical density reaches, by insertion on one lane).
-__global__ void nl_sort_cells(int n_cells, const int *__restrict__ cell_start, int *__restrict__ cell_atoms) {
+// With `local`, each atom's position relative to the middle of its cell, in
+// float32, beside its index, in the cells' order (NaN for an atom whose cell
+// coordinate lies beyond 4096 boxes).
+__global__ void nl_sort_cells(SysView S, const int *__restrict__ grids, int n_cells,
+                              const int *__restrict__ cell_start, int *__restrict__ cell_atoms,
+                              float4 *__restrict__ local) {
     __shared__ int srow[NL_WARPS][NL_MAXROW];
     int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
     for (int c = blockIdx.x * NL_WARPS + wid; c < n_cells; c += gridDim.x * NL_WARPS) {
@@ -372,6 +751,30 @@ __global__ void nl_sort_cells(int n_cells, const int *__restrict__ cell_start, i
             }
         }
         __syncwarp();
+        if (!local || n == 0) continue;
+        const int sidx = S.n_struct > 1 ? S.atom_struct[cell_atoms[b]] : 0;
+        const int *g = grids + 8 * sidx;
+        const double *L = S.cells + 18 * (size_t)sidx;
+        const int place = c - g[3];
+        const double m0 = ((double)(place / (g[1] * g[2])) + 0.5) / (double)g[0];
+        const double m1 = ((double)((place / g[2]) % g[1]) + 0.5) / (double)g[1];
+        const double m2 = ((double)(place % g[2]) + 0.5) / (double)g[2];
+        for (int k = lane; k < n; k += 32) {
+            const int a = cell_atoms[b + k];
+            const double *p = S.pos + 3 * (size_t)a;
+            double f[3];
+            bool far = false;
+#pragma unroll
+            for (int q = 0; q < 3; ++q) {
+                const double s = p[0] * L[9 + q] + p[1] * L[12 + q] + p[2] * L[15 + q];
+                if (!(fabs(s) <= 4096.0)) far = true;
+                f[q] = s - floor(s) - (q == 0 ? m0 : q == 1 ? m1 : m2);
+            }
+            const float x = (float)(f[0] * L[0] + f[1] * L[3] + f[2] * L[6]);
+            local[b + k] = make_float4(far ? __int_as_float(0x7fffffff) : x,
+                                       (float)(f[0] * L[1] + f[1] * L[4] + f[2] * L[7]),
+                                       (float)(f[0] * L[2] + f[1] * L[5] + f[2] * L[8]), __int_as_float(a));
+        }
     }
 }
 
@@ -395,8 +798,8 @@ __global__ void nl_sort_rows(int n_atoms, const int *__restrict__ row_off, int *
     }
 }
 
-// The staged rows (nl_cells<2>) into the CSR: each row read from its
-// stride-spaced staging slot, sorted and written at its scanned offset;
+// The staged rows (nl_cells<2>, nl_search) into the CSR: each row read from its
+// stride-spaced staging slot, sorted where it is not, and written at its scanned offset;
 // its first upper slot recorded.  Rows longer than the stride were refused
 // by the guard (their rows are empty by then).
 __global__ void nl_unstage_rows(int n_atoms, const int *__restrict__ row_off, const int *__restrict__ stage,
@@ -566,8 +969,9 @@ size_t mbf_nl_rebuild_workspace_bytes(int n_atoms, int n_cells_total, int max_ro
     return nl_staged_bytes(nl_layout(n_atoms, n_cells_total), n_atoms, max_row_limit);
 }
 
-static int nl_prepare(const SysView &S, const int *grids, int n_cells_total, double rl2, void *workspace,
-                      const NlLayout &L, int *row_off, cudaStream_t st, int *stage = nullptr, int stride = 0) {
+static int nl_prepare(const SysView &S, const int *grids, int n_cells_total, double r_list, void *workspace,
+                      const NlLayout &L, int *row_off, cudaStream_t st, int *stage = nullptr, int stride = 0,
+                      float4 *local = nullptr) {
     int N = S.n_atoms;
     int *err = ws_at<int>(workspace, L.err);
     int *atom_cell = ws_at<int>(workspace, L.atom_cell);
@@ -591,44 +995,38 @@ static int nl_prepare(const SysView &S, const int *grids, int n_cells_total, dou
     if (cudaMemcpyAsync(cursor, cell_start, sizeof(int) * (size_t)n_cells_total,
                         cudaMemcpyDeviceToDevice, st) != cudaSuccess)
         return MBF_ERR_CUDA;
+    PROF_BEGIN("nl_fill_cells", st);
     nl_fill_cells<<<(N + 255) / 256, 256, 0, st>>>(N, atom_cell, cursor, cell_atoms);
     nl_sort_cells<<<persistent_grid((n_cells_total + NL_WARPS - 1) / NL_WARPS, 32 * NL_WARPS,
                                     (const void *)nl_sort_cells),
-                    32 * NL_WARPS, 0, st>>>(n_cells_total, cell_start, cell_atoms);
+                    32 * NL_WARPS, 0, st>>>(S, grids, n_cells_total, cell_start, cell_atoms,
+                                            nl_blocks(N, n_cells_total, local) ? local : nullptr);
+    PROF_END("nl_fill_cells", st);
     MBF_CHECK_LAUNCH();
-    int cblocks = (n_cells_total + NL_WARPS - 1) / NL_WARPS;
-    int g = persistent_grid(cblocks, 32 * NL_WARPS, (const void *)nl_cells<0>);
     PROF_BEGIN("nl_count", st);
-    if (stage) {
-        g = persistent_grid(cblocks, 32 * NL_WARPS, (const void *)nl_cells<2>);
-        nl_cells<2><<<g, 32 * NL_WARPS, 0, st>>>(S, grids, cell_start, cell_atoms, n_cells_total, rl2, row_cnt, mrow,
-                                                 nullptr, stage, stride);
-    } else {
-        nl_cells<0><<<g, 32 * NL_WARPS, 0, st>>>(S, grids, cell_start, cell_atoms, n_cells_total, rl2, row_cnt, mrow,
-                                                 nullptr, nullptr, 0);
-    }
+    rc = stage ? nl_rows<2>(S, grids, cell_start, cell_atoms, local, n_cells_total, r_list, row_cnt, mrow, nullptr,
+                            stage, stride, cursor, st)
+               : nl_rows<0>(S, grids, cell_start, cell_atoms, nullptr, n_cells_total, r_list, row_cnt, mrow, nullptr,
+                            nullptr, 0, nullptr, st);
     PROF_END("nl_count", st);
-    MBF_CHECK_LAUNCH();
+    if (rc != MBF_OK) return rc;
     return exclusive_scan(row_cnt, row_off, N, scan_ws, st);
 }
 
-static int nl_finish(const SysView &S, const int *grids, int n_cells_total, double rl2, void *workspace,
+static int nl_finish(const SysView &S, const int *grids, int n_cells_total, double r_list, void *workspace,
                      const NlLayout &L, const int *row_off, int *nbr, int *rev, int *upper, cudaStream_t st,
                      const int *stage = nullptr, int stride = 0) {
     int N = S.n_atoms;
     int *err = ws_at<int>(workspace, L.err);
     int blocks = (N + NL_WARPS - 1) / NL_WARPS;
-    int cblocks = (n_cells_total + NL_WARPS - 1) / NL_WARPS;
-    int g = persistent_grid(cblocks, 32 * NL_WARPS, (const void *)nl_cells<1>);
+    int g = persistent_grid(blocks, 32 * NL_WARPS, stage ? (const void *)nl_unstage_rows : (const void *)nl_sort_rows);
     PROF_BEGIN("nl_fill", st);
     if (stage) {
-        g = persistent_grid(blocks, 32 * NL_WARPS, (const void *)nl_unstage_rows);
         nl_unstage_rows<<<g, 32 * NL_WARPS, 0, st>>>(N, row_off, stage, stride, nbr, upper, err);
     } else {
-        nl_cells<1><<<g, 32 * NL_WARPS, 0, st>>>(S, grids, ws_at<int>(workspace, L.cell_start),
-                                                 ws_at<int>(workspace, L.cell_atoms), n_cells_total, rl2, nullptr,
-                                                 nullptr, row_off, nbr, 0);
-        g = persistent_grid(blocks, 32 * NL_WARPS, (const void *)nl_sort_rows);
+        int rc = nl_rows<1>(S, grids, ws_at<int>(workspace, L.cell_start), ws_at<int>(workspace, L.cell_atoms),
+                            nullptr, n_cells_total, r_list, nullptr, nullptr, row_off, nbr, 0, nullptr, st);
+        if (rc != MBF_OK) return rc;
         nl_sort_rows<<<g, 32 * NL_WARPS, 0, st>>>(N, row_off, nbr, upper, err);
     }
     PROF_END("nl_fill", st);
@@ -659,18 +1057,25 @@ int mbf_nl_build(const mbf_system *sys, const int *grids, int n_cells_total, dou
         *max_row = 0;
         return MBF_OK;
     }
-    double rl2 = r_list * r_list;
     // workspace beyond the layout holds staging rows at the stride it allows:
     // if no row is longer, the search runs once (count and stage, then sort
-    // into the CSR), else the rows are searched again (fill)
+    // into the CSR), else the rows are searched again (fill); where it has
+    // room for both, the local coordinates of the block search come first
     int stride = 0;
-    if (workspace_bytes >= L.total + 256) {
-        size_t per = (workspace_bytes - L.total) / (sizeof(int) * (size_t)N);
+    float4 *local = nullptr;
+    size_t room = workspace_bytes - L.total, front = 0;
+    if (room >= 256) {
+        front = nl_local_bytes(N);
+        if (room >= front + sizeof(int) * (size_t)N && nl_local_ok(workspace))
+            local = ws_at<float4>(workspace, L.total);
+        else
+            front = 0;
+        size_t per = (room - front) / (sizeof(int) * (size_t)N);
         stride = (int)(per < (size_t)NL_MAXROW ? per : (size_t)NL_MAXROW);
         if ((long long)N * stride >= 0x7fffffffLL) stride = (int)(0x7ffffffeLL / N);
     }
-    int *stage = stride > 0 ? ws_at<int>(workspace, L.total) : nullptr;
-    int rc = nl_prepare(S, grids, n_cells_total, rl2, workspace, L, row_off, st, stage, stride);
+    int *stage = stride > 0 ? ws_at<int>(workspace, L.total + front) : nullptr;
+    int rc = nl_prepare(S, grids, n_cells_total, r_list, workspace, L, row_off, st, stage, stride, local);
     if (rc != MBF_OK) return rc;
     int host[2];
     if (cudaMemcpyAsync(&host[0], row_off + N, sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
@@ -684,7 +1089,7 @@ int mbf_nl_build(const mbf_system *sys, const int *grids, int n_cells_total, dou
     if (!upper) return MBF_ERR_ARGUMENT;
     if (host[1] > NL_MAXROW) return MBF_ERR_ROW_TOO_LONG;
     if (host[1] > stride) stage = nullptr;
-    rc = nl_finish(S, grids, n_cells_total, rl2, workspace, L, row_off, nbr, rev, upper, st, stage,
+    rc = nl_finish(S, grids, n_cells_total, r_list, workspace, L, row_off, nbr, rev, upper, st, stage,
                    stage ? stride : 0);
     if (rc != MBF_OK) return rc;
     int herr = 0;
@@ -709,20 +1114,27 @@ int mbf_nl_rebuild_async(const mbf_system *sys, const int *grids, int n_cells_to
     NlLayout L = nl_layout(N, n_cells_total);
     if (workspace_bytes < L.total) return MBF_ERR_WORKSPACE;
     SysView S = make_view(sys);
-    double rl2 = r_list * r_list;
     // with room for the staging rows the search runs once (count and stage),
-    // else it counts, then fills
+    // with room for the local coordinates too by blocks; else it counts, then
+    // fills
     int *stage = nullptr;
-    if (workspace_bytes >= nl_staged_bytes(L, N, max_row_limit) && (long long)N * max_row_limit < 0x7fffffffLL)
+    float4 *local = nullptr;
+    size_t rows = align256(sizeof(int) * (size_t)N * (size_t)max_row_limit);
+    if (workspace_bytes >= L.total + rows && (long long)N * max_row_limit < 0x7fffffffLL) {
         stage = ws_at<int>(workspace, L.total);
-    int rc = nl_prepare(S, grids, n_cells_total, rl2, workspace, L, row_off, st, stage, max_row_limit);
+        if (workspace_bytes >= nl_staged_bytes(L, N, max_row_limit) && nl_local_ok(workspace)) {
+            local = ws_at<float4>(workspace, L.total);
+            stage = ws_at<int>(workspace, L.total + nl_local_bytes(N));
+        }
+    }
+    int rc = nl_prepare(S, grids, n_cells_total, r_list, workspace, L, row_off, st, stage, max_row_limit, local);
     if (rc != MBF_OK) return rc;
     int *err = ws_at<int>(workspace, L.err);
     nl_guard<<<1, 32, 0, st>>>(N, row_off, ws_at<int>(workspace, L.maxrow), nbr_capacity, max_row_limit, status,
                                err + 4);
     nl_clear_if<<<(N + 256) / 256, 256, 0, st>>>(N, err + 4, row_off, upper);
     MBF_CHECK_LAUNCH();
-    rc = nl_finish(S, grids, n_cells_total, rl2, workspace, L, row_off, nbr, rev, upper, st, stage, max_row_limit);
+    rc = nl_finish(S, grids, n_cells_total, r_list, workspace, L, row_off, nbr, rev, upper, st, stage, max_row_limit);
     if (rc != MBF_OK) return rc;
     nl_status_merge<<<1, 32, 0, st>>>(err, status);
     MBF_CHECK_LAUNCH();

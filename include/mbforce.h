@@ -107,18 +107,21 @@ int mbf_version(void);
  * bit for bit.  n_cells_total = sum over structures of nc0*nc1*nc2.      */
 size_t mbf_nl_workspace_bytes(int n_atoms, int n_cells_total);
 /* The workspace with which mbf_nl_rebuild_async searches once instead of
- * twice: mbf_nl_workspace_bytes plus n_atoms x max_row_limit staging ints
+ * twice: mbf_nl_workspace_bytes plus 16 bytes per atom (coordinates for the
+ * search of cells of many atoms) plus n_atoms x max_row_limit staging ints
  * (each row kept at a fixed stride during the count, then sorted into
- * the CSR).  A smaller workspace, of at least mbf_nl_workspace_bytes, runs
- * the count-then-fill search.                                            */
+ * the CSR).  Without room for the coordinates, or at an address that is no
+ * multiple of 16, it searches once but slower; a workspace of at least
+ * mbf_nl_workspace_bytes runs the count-then-fill search.                */
 size_t mbf_nl_rebuild_workspace_bytes(int n_atoms, int n_cells_total, int max_row_limit);
 
 /* Counts, scans and fills.  If nbr_capacity < the number of slots it stops
  * after the count, stores the need in *n_slots (host) and returns
  * MBF_ERR_CAPACITY; call again with a larger nbr/rev.  *n_slots and
  * *max_row are host outputs.  Synchronises `stream` once (to read the
- * count).  Workspace beyond mbf_nl_workspace_bytes serves as staging rows
- * (stride = the extra bytes / (4 n_atoms), at most 1024): when no row is
+ * count).  Workspace beyond mbf_nl_workspace_bytes serves as coordinates (16
+ * bytes per atom, if there is more) and staging rows (stride = the remaining
+ * bytes / (4 n_atoms), at most 1024): when no row is
  * longer than that stride the search runs once, as in
  * mbf_nl_rebuild_async; size it with mbf_nl_rebuild_workspace_bytes and
  * a row bound estimate.  The list is the same either way. */
