@@ -197,6 +197,7 @@ class NeighbourList:
         self._dnl = DeviceNeighbourList(self.r_list)
         self._batch = None
         self._half = None
+        self._scratch = None
 
     @property
     def active_backend(self):
@@ -266,10 +267,8 @@ class NeighbourList:
         map since the build and d_max the largest minimum-imaged non-affine
         displacement (computed on the device)."""
         lattice = np.asarray(lattice, dtype=np.float64)
-        if np.allclose(lattice, self._lattice, atol=1e-12):
-            sigma_min = 1.0
-            M = np.eye(3)
-        else:
+        M, sigma_min = None, 1.0
+        if not (np.array_equal(lattice, self._lattice) or np.allclose(lattice, self._lattice, atol=1e-12)):
             M = np.linalg.inv(self._lattice) @ lattice
             sigma_min = float(np.linalg.svd(M, compute_uv=False)[-1])
         b = self._batch
@@ -279,8 +278,11 @@ class NeighbourList:
         else:
             b.set_positions(np.ascontiguousarray(positions, dtype=np.float64))
         dev = b.device
-        maps = torch.as_tensor(np.ascontiguousarray(M.reshape(1, 9)), device=dev)
-        dmax = torch.empty(1, dtype=torch.float64, device=dev)
+        if self._scratch is None or self._scratch.device != dev:   # the identity map and d_max
+            self._scratch = torch.tensor([1.0, 0, 0, 0, 1.0, 0, 0, 0, 1.0, 0], dtype=torch.float64, device=dev)
+        maps, dmax = self._scratch[:9], self._scratch[9:]
+        if M is not None:
+            maps = torch.as_tensor(np.ascontiguousarray(M.reshape(9)), device=dev)
         _lib.check(_lib.lib().mbf_nl_max_displacement(
             b.mbf_system(), _lib.ptr(self._ref_pos), _lib.ptr(maps), _lib.ptr(dmax),
             torch.cuda.current_stream(dev).cuda_stream), "mbf_nl_max_displacement")

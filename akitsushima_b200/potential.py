@@ -238,19 +238,18 @@ class DevicePotential:
         # a comparison
         if not batch.types_unchanged(atom_types, len(self.species)):
             batch.set_types(species_ids(atom_types, self.species))
-        res = self.evaluate(batch, dl)
-        # energy, virial and the device status words (the first 16 bytes of
-        # the workspace, carried as two doubles) in one copy
-        words = _get_last_ws(self)[:16].view(torch.float64)
-        ev = torch.cat([res.energy[:1], res.virial[0], words]).to("cpu", non_blocking=True)
-        f = batch.forces_to_host(res.forces)   # synchronises the stream
-        ev = ev.numpy()
-        self._raise_status(np.frombuffer(ev[10:12].tobytes(), dtype=np.int32))
+        # forces, energy and virial in one buffer, so one copy brings them
+        # back; the status words are the first 16 bytes of the workspace
+        packed = torch.empty(3 * n + 10, dtype=torch.float64, device=batch.device)
+        self.evaluate(batch, dl, out=EvalResult(packed[3 * n:3 * n + 1], packed[:3 * n].view(n, 3),
+                                                packed[3 * n + 1:].view(1, 9)))
+        f, ev, words = batch.results_to_host(packed, _get_last_ws(self)[:16].view(torch.float64))
+        self._raise_status(words.tolist())
         e = float(ev[0])
         if not need_stress:
             return e, f, None
         vol = abs(float(np.linalg.det(lattice)))
-        s = ev[1:10].reshape(3, 3) / vol
+        s = ev[1:].reshape(3, 3) / vol
         return e, f, s
 
 

@@ -34,14 +34,18 @@ def cell_metrics(lattice):
     return cell_widths(lat), float(np.linalg.svd(lat, compute_uv=False)[-1])
 
 
+_NEXT, _LAST = np.array([1, 2, 0]), np.array([2, 0, 1])
+
+
 def cell_widths(lattice):
     """The perpendicular widths of :func:`cell_metrics` alone."""
     lat = np.asarray(lattice, dtype=float)
     if lat.shape != (3, 3):
         raise ValueError(f"NeighbourList: lattice must have shape (3, 3), got {lat.shape}.")
     volume = abs(float(np.linalg.det(lat)))
-    cross = np.array([np.linalg.norm(np.cross(lat[(i + 1) % 3], lat[(i + 2) % 3]))
-                      for i in range(3)])
+    a, b = lat[_NEXT], lat[_LAST]   # a_j x a_k of the three axes in one expression, as np.cross rounds
+    c = a[:, _NEXT] * b[:, _LAST] - a[:, _LAST] * b[:, _NEXT]
+    cross = np.array([np.linalg.norm(v) for v in c])
     if volume <= 0.0 or not np.all(cross > 0.0) or not np.isfinite(volume):
         raise ValueError(
             f"NeighbourList: degenerate (singular) lattice with volume {volume:.6g} A^3 -- "
@@ -254,16 +258,19 @@ class Batch:
         self.pos.copy_(stage, non_blocking=True)
         self._stage_done.record(torch.cuda.current_stream(self.device))
 
-    def forces_to_host(self, forces):
-        """Device (N, 3) forces to a new host numpy array: a pinned block of
-        torch's caching host allocator, copied into directly (no second host
-        copy); the block returns to the cache when the caller drops it."""
-        if self.device.type != "cuda":
-            return forces.cpu().numpy()
-        out = torch.empty((self.n_atoms, 3), dtype=torch.float64, pin_memory=True)
-        out.copy_(forces, non_blocking=True)
+    def results_to_host(self, packed, words):
+        """Device results (a float64 vector whose first 3 N entries are the
+        forces) and the evaluation's status words on the host: (forces (N, 3),
+        the rest, words) as views of one new pinned block of torch's caching
+        host allocator, copied into directly (no second host copy) and given
+        back to the cache when the caller drops its views."""
+        n, m = 3 * self.n_atoms, packed.numel()
+        host = torch.empty(m + 2, dtype=torch.float64, pin_memory=True)
+        host[:m].copy_(packed, non_blocking=True)
+        host[m:].copy_(words, non_blocking=True)
         torch.cuda.current_stream(self.device).synchronize()
-        return out.numpy()
+        out = host.numpy()
+        return out[:n].reshape(-1, 3), out[n:m], out[m:].view(np.int32)
 
     def types_unchanged(self, type_ids, n_species):
         """True if type_ids is an integer array equal to the ids last
