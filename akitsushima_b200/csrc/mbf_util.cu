@@ -128,10 +128,17 @@ int exclusive_scan(const int *in, int *out, int n, int *ws, cudaStream_t st) {
 // adding its atom's record (entries sub and sub + 8).  Only the slots whose
 // live bit is set are read: a list radius of cutoff + skin holds two to three
 // times the slots that carry a force (32,768-atom SiC: 15.5 listed, 6 live),
-// and the others are never written.  Bound by latency: up to four slots a
-// lane are in flight at once.
+// and the others are never written.  Bound by latency, hence by how many
+// groups are resident and how much of a row each has in flight: 16 slots of a
+// row at a time take 22.9 us for the 512 uneven silicon cells and 16.1 for
+// 64,000 GeSn atoms, 32 at a time 28.6 and 18.9, 8 at a time 24.7 and 18.8;
+// two atoms a group at once 31 and 20.7; at 1536 threads an SM the registers
+// spill (30 and 20.9).
+constexpr int GATHER_K = 2;
+
 template <int NT>
-__global__ void __launch_bounds__(NT) gather_live_rows(const int *__restrict__ row_off, const double *__restrict__ G,
+__global__ void __launch_bounds__(NT, 1024 / NT) gather_live_rows(const int *__restrict__ row_off,
+                                                       const double *__restrict__ G,
                                                        const uint4 *__restrict__ live_mask, int row_limit,
                                                        int *__restrict__ err, const double *__restrict__ f_local,
                                                        double *__restrict__ forces, ChunkSums cs) {
@@ -150,57 +157,54 @@ __global__ void __launch_bounds__(NT) gather_live_rows(const int *__restrict__ r
         nm = live_mask[a0 + grp];
     }
     for (int base = a0; base < a1; base += NG) {  // uniform over the block
-        const int a = base + grp, beg = nb, n = ne - nb;
+        const int a = base + grp, beg = nb;
+        int n = ne - nb;
         const uint4 m4 = nm;
         if (a + NG < a1) {
             nb = row_off[a + NG];
             ne = row_off[a + NG + 1];
             nm = live_mask[a + NG];
         }
-        double fx = 0, fy = 0, fz = 0, fl = 0;
+        double ra = 0.0, rb = 0.0, fl = 0.0, f[3] = {0.0, 0.0, 0.0};
         if (a < a1) {
             const double *pa = cs.per_atom + (size_t)a * ATOM_ACC;
-            const double ra = pa[sub];
-            double rb = sub < ATOM_ACC - LPA ? pa[LPA + sub] : 0.0;
+            ra = pa[sub];
+            if (sub < ATOM_ACC - LPA) rb = pa[LPA + sub];
             if (sub < 3) fl = f_local[3 * (size_t)a + sub];
-            if (sub == 10 - LPA && rb < 0.0) {  // a bad index in the row (put_atom)
-                atomicOr(err, MBF_DEV_BAD_INDEX);
-                rb = 0.0;
-            }
-            if (n > row_limit) {
-                if (sub == 0) atomicOr(err, MBF_DEV_ROW_TOO_LONG);
-            } else {
-                const unsigned m[4] = {m4.x, m4.y, m4.z, m4.w};
+        } else {
+            n = 0;
+        }
+        if (n > row_limit) {
+            if (sub == 0) atomicOr(err, MBF_DEV_ROW_TOO_LONG);
+            n = 0;
+        }
+        for (int w = 0; w < n; w += GATHER_K * LPA) {
+            const unsigned m = w < 32 ? m4.x : (w < 64 ? m4.y : (w < 96 ? m4.z : m4.w));
+            double x[GATHER_K][3];
 #pragma unroll
-                for (int w = 0; w < 4; ++w) {
-                    if (32 * w >= n) break;
-                    double x[4], y[4], z[4];
+            for (int k = 0; k < GATHER_K; ++k) {
+                x[k][0] = x[k][1] = x[k][2] = 0.0;
+                if (m >> ((w & 31) + sub + LPA * k) & 1u) {
+                    const double *g = G + 3 * (size_t)(beg + w + sub + LPA * k);
 #pragma unroll
-                    for (int k = 0; k < 4; ++k) {
-                        x[k] = y[k] = z[k] = 0.0;
-                        if (m[w] >> (sub + LPA * k) & 1u) {
-                            const double *g = G + 3 * (size_t)(beg + 32 * w + sub + LPA * k);
-                            x[k] = __ldcs(g);
-                            y[k] = __ldcs(g + 1);
-                            z[k] = __ldcs(g + 2);
-                        }
-                    }
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) {
-                        fx += x[k];
-                        fy += y[k];
-                        fz += z[k];
-                    }
+                    for (int q = 0; q < 3; ++q) x[k][q] = __ldcs(g + q);
                 }
             }
-            r0 += ra;
-            r1 += rb;
+#pragma unroll
+            for (int k = 0; k < GATHER_K; ++k)
+#pragma unroll
+                for (int q = 0; q < 3; ++q) f[q] += x[k][q];
         }
-        fx = group_sum<LPA>(fx);
-        fy = group_sum<LPA>(fy);
-        fz = group_sum<LPA>(fz);
+        if (sub == 10 - LPA && rb < 0.0) {  // a bad index in the row (put_atom)
+            atomicOr(err, MBF_DEV_BAD_INDEX);
+            rb = 0.0;
+        }
+        r0 += ra;
+        r1 += rb;
+#pragma unroll
+        for (int q = 0; q < 3; ++q) f[q] = group_sum<LPA>(f[q]);
         // lane k (k < 3) of the group writes component k
-        const double g = sub == 0 ? fx : (sub == 1 ? fy : fz);
+        const double g = sub == 0 ? f[0] : (sub == 1 ? f[1] : f[2]);
         if (sub < 3 && a < a1) forces[3 * (size_t)a + sub] = fl + g;
     }
     chunk_sums_finish<NT>(cs, c, s, r0, r1);
