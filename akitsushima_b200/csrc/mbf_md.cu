@@ -15,9 +15,21 @@
 
 namespace mbf {
 
-constexpr int MD_BLOCK = 256;
-constexpr int MD_ITEMS = 4;
-constexpr int MD_CHUNK = MD_BLOCK * MD_ITEMS;
+// Threads per block of the kick kernels and the atoms a thread takes, one
+// partial sum a block.  A step
+// of a few thousand atoms waits on one atom's chain of loads and float64
+// arithmetic, not on throughput: with 1024 atoms a block in four rounds a
+// block of ten steps of 4096 Tersoff atoms took 347 us, with 128 it takes 313
+// (256: 321); 64,000 atoms 853 against 835.  A batch keeps the 1024: its grid
+// has a block column per structure for the atoms of all.
+constexpr int MD_BLOCK = 128;
+
+static int md_items(const mbf_system *sys) { return sys->n_struct > 1 ? 8 : 1; }
+
+static int md_blocks(const mbf_system *sys) {
+    const int chunk = MD_BLOCK * md_items(sys);
+    return sys->n_atoms <= 0 ? 1 : (sys->n_atoms + chunk - 1) / chunk;
+}
 
 // v += dt/2 a; r += dt v; frac = r @ inv(L), frac -= floor(frac),
 // frac >= 1 -> 0, r = frac @ L (the reference's wrap, :1981-1989).
@@ -149,7 +161,7 @@ __device__ void md_thermo_body(int n_struct, int P, const double *__restrict__ p
 
 __global__ void __launch_bounds__(MD_BLOCK) md_kick(SysView S, double *__restrict__ vel,
                                                     const double *__restrict__ F,
-                                                    const double *__restrict__ im, double dt, int P,
+                                                    const double *__restrict__ im, double dt, int items, int P,
                                                     double *__restrict__ partial,
                                                     const double *__restrict__ energy,
                                                     double *__restrict__ thermo, int rows,
@@ -160,20 +172,16 @@ __global__ void __launch_bounds__(MD_BLOCK) md_kick(SysView S, double *__restric
     int beg = S.n_struct > 1 ? S.struct_off[s] : 0;
     int end = S.n_struct > 1 ? S.struct_off[s + 1] : S.n_atoms;
     double acc = 0.0;
-    int first = beg + blockIdx.x * MD_CHUNK;
-#pragma unroll
-    for (int k = 0; k < MD_ITEMS; ++k) {
-        int a = first + k * MD_BLOCK + threadIdx.x;
-        if (a < end) {
-            size_t o = 3 * (size_t)a;
-            double w = im[a];
-            double h = 0.5 * dt * w;
-            double vx = vel[o] + h * F[o], vy = vel[o + 1] + h * F[o + 1], vz = vel[o + 2] + h * F[o + 2];
-            vel[o] = vx;
-            vel[o + 1] = vy;
-            vel[o + 2] = vz;
-            acc += (vx * vx + vy * vy + vz * vz) / w;
-        }
+    const int first = beg + blockIdx.x * (items * MD_BLOCK), stop = min(end, first + items * MD_BLOCK);
+    for (int a = first + threadIdx.x; a < stop; a += MD_BLOCK) {
+        size_t o = 3 * (size_t)a;
+        double w = im[a];
+        double h = 0.5 * dt * w;
+        double vx = vel[o] + h * F[o], vy = vel[o + 1] + h * F[o + 1], vz = vel[o + 2] + h * F[o + 2];
+        vel[o] = vx;
+        vel[o + 1] = vy;
+        vel[o + 2] = vz;
+        acc += (vx * vx + vy * vy + vz * vz) / w;
     }
     acc = block_sum<MD_BLOCK>(acc, sh);
     if (threadIdx.x == 0) {
@@ -198,7 +206,7 @@ __global__ void __launch_bounds__(MD_BLOCK) md_kick(SysView S, double *__restric
 // the rebuild decision of the next (md_kick_drift_check's tail).
 __global__ void __launch_bounds__(MD_BLOCK) md_kick_kick_drift_check(
     SysView S, double *__restrict__ pos, double *__restrict__ vel, const double *__restrict__ F,
-    const double *__restrict__ im, double dt, int P, double *__restrict__ partial,
+    const double *__restrict__ im, double dt, int items, int P, double *__restrict__ partial,
     const double *__restrict__ energy, double *__restrict__ thermo, int rows, int *__restrict__ tcounter,
     const double *__restrict__ ref, unsigned long long *__restrict__ dmax, double r_list, double r_cut,
     double *__restrict__ d_log, int *__restrict__ scounter, int *__restrict__ gate, unsigned long long cond,
@@ -211,44 +219,40 @@ __global__ void __launch_bounds__(MD_BLOCK) md_kick_kick_drift_check(
     const double *c = S.cells + 18 * (size_t)s;
     double acc = 0.0;
     unsigned long long bits = 0ull;
-    int first = beg + blockIdx.x * MD_CHUNK;
-#pragma unroll
-    for (int k = 0; k < MD_ITEMS; ++k) {
-        int a = first + k * MD_BLOCK + threadIdx.x;
-        if (a < end) {
-            size_t o = 3 * (size_t)a;
-            double w = im[a];
-            double h = 0.5 * dt * w;
-            double fx = F[o], fy = F[o + 1], fz = F[o + 2];
-            double vx = vel[o] + h * fx, vy = vel[o + 1] + h * fy, vz = vel[o + 2] + h * fz;
-            acc += (vx * vx + vy * vy + vz * vz) / w;
-            vx = vx + h * fx;
-            vy = vy + h * fy;
-            vz = vz + h * fz;
-            double x = pos[o] + dt * vx, y = pos[o + 1] + dt * vy, z = pos[o + 2] + dt * vz;
-            double s0 = x * c[9] + y * c[12] + z * c[15];
-            double s1 = x * c[10] + y * c[13] + z * c[16];
-            double s2 = x * c[11] + y * c[14] + z * c[17];
-            s0 -= floor(s0);
-            s1 -= floor(s1);
-            s2 -= floor(s2);
-            if (s0 >= 1.0) s0 = 0.0;
-            if (s1 >= 1.0) s1 = 0.0;
-            if (s2 >= 1.0) s2 = 0.0;
-            double px = s0 * c[0] + s1 * c[3] + s2 * c[6];
-            double py = s0 * c[1] + s1 * c[4] + s2 * c[7];
-            double pz = s0 * c[2] + s1 * c[5] + s2 * c[8];
-            pos[o] = px;
-            pos[o + 1] = py;
-            pos[o + 2] = pz;
-            vel[o] = vx;
-            vel[o + 1] = vy;
-            vel[o + 2] = vz;
-            double dx, dy, dz;
-            mic_exact(c, px - ref[o], py - ref[o + 1], pz - ref[o + 2], dx, dy, dz);
-            unsigned long long b = (unsigned long long)__double_as_longlong(sqrt(dx * dx + dy * dy + dz * dz));
-            bits = b > bits ? b : bits;
-        }
+    const int first = beg + blockIdx.x * (items * MD_BLOCK), stop = min(end, first + items * MD_BLOCK);
+    for (int a = first + threadIdx.x; a < stop; a += MD_BLOCK) {
+        size_t o = 3 * (size_t)a;
+        double w = im[a];
+        double h = 0.5 * dt * w;
+        double fx = F[o], fy = F[o + 1], fz = F[o + 2];
+        double vx = vel[o] + h * fx, vy = vel[o + 1] + h * fy, vz = vel[o + 2] + h * fz;
+        acc += (vx * vx + vy * vy + vz * vz) / w;
+        vx = vx + h * fx;
+        vy = vy + h * fy;
+        vz = vz + h * fz;
+        double x = pos[o] + dt * vx, y = pos[o + 1] + dt * vy, z = pos[o + 2] + dt * vz;
+        double s0 = x * c[9] + y * c[12] + z * c[15];
+        double s1 = x * c[10] + y * c[13] + z * c[16];
+        double s2 = x * c[11] + y * c[14] + z * c[17];
+        s0 -= floor(s0);
+        s1 -= floor(s1);
+        s2 -= floor(s2);
+        if (s0 >= 1.0) s0 = 0.0;
+        if (s1 >= 1.0) s1 = 0.0;
+        if (s2 >= 1.0) s2 = 0.0;
+        double px = s0 * c[0] + s1 * c[3] + s2 * c[6];
+        double py = s0 * c[1] + s1 * c[4] + s2 * c[7];
+        double pz = s0 * c[2] + s1 * c[5] + s2 * c[8];
+        pos[o] = px;
+        pos[o + 1] = py;
+        pos[o + 2] = pz;
+        vel[o] = vx;
+        vel[o + 1] = vy;
+        vel[o + 2] = vz;
+        double dx, dy, dz;
+        mic_exact(c, px - ref[o], py - ref[o + 1], pz - ref[o + 2], dx, dy, dz);
+        unsigned long long b = (unsigned long long)__double_as_longlong(sqrt(dx * dx + dy * dy + dz * dz));
+        bits = b > bits ? b : bits;
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -263,18 +267,25 @@ __global__ void __launch_bounds__(MD_BLOCK) md_kick_kick_drift_check(
     if (threadIdx.x == 0) last = atomicAdd(done, 1u) == gridDim.x * gridDim.y - 1;
     __syncthreads();
     if (!last) return;
+    // the decision's words are on their way while the thermo row is summed
+    int checks = 0;
+    unsigned long long d_first = 0ull;
+    if (threadIdx.x == 0) {
+        checks = *scounter;
+        d_first = atomicExch(dmax, 0ull);
+    }
     md_thermo_body(S.n_struct, P, partial, energy, thermo, rows, tcounter, sh);
     if (threadIdx.x != 0) return;
-    int row = *scounter % rows;
+    int row = checks % rows;
     int need = 0;
     for (int q = 0; q < S.n_struct; ++q) {
-        double d = __longlong_as_double((long long)atomicExch(dmax + q, 0ull));
+        double d = __longlong_as_double((long long)(q ? atomicExch(dmax + q, 0ull) : d_first));
         d_log[(size_t)row * S.n_struct + q] = d;
         if (r_list - 2.0 * d <= r_cut) need = 1;
     }
     *gate = need;
     if (cond) cudaGraphSetConditional((cudaGraphConditionalHandle)cond, need ? 1u : 0u);
-    *scounter += 1;
+    *scounter = checks + 1;
     *done = 0u;
 }
 
@@ -284,19 +295,20 @@ __global__ void __launch_bounds__(MD_BLOCK) md_kick_kick_drift_check(
 __device__ void md_thermo_body(int n_struct, int P, const double *__restrict__ partial,
                                const double *__restrict__ energy, double *__restrict__ thermo, int rows,
                                int *__restrict__ counter, double *sh) {
-    int row = *counter % rows;
+    const int count = *counter, row = count % rows;
     for (int s = 0; s < n_struct; ++s) {
+        const double e = energy[s];
         double v = 0.0;
         for (int k = threadIdx.x; k < P; k += MD_BLOCK) v += __ldcg(partial + (size_t)s * P + k);
         v = block_sum<MD_BLOCK>(v, sh);
         if (threadIdx.x == 0) {
             double *t = thermo + 2 * ((size_t)row * n_struct + s);
-            t[0] = energy[s];
+            t[0] = e;
             t[1] = 0.5 * v;
         }
     }
     __syncthreads();
-    if (threadIdx.x == 0) *counter += 1;
+    if (threadIdx.x == 0) *counter = count + 1;
 }
 
 }  // namespace mbf
@@ -320,7 +332,7 @@ int mbf_md_kick_drift(const mbf_system *sys, double *positions, double *velociti
     return MBF_OK;
 }
 
-int mbf_md_partial_count(int n_atoms) { return n_atoms <= 0 ? 1 : (n_atoms + MD_CHUNK - 1) / MD_CHUNK; }
+int mbf_md_partial_count(int n_atoms) { return n_atoms <= 0 ? 1 : (n_atoms + MD_BLOCK - 1) / MD_BLOCK; }
 
 int mbf_md_kick(const mbf_system *sys, double *velocities, const double *forces, const double *inv_mass,
                 double dt, const double *energy, double *partial, double *thermo, int thermo_rows,
@@ -330,10 +342,10 @@ int mbf_md_kick(const mbf_system *sys, double *velocities, const double *forces,
         return MBF_ERR_ARGUMENT;
     SysView S = make_view(sys);
     cudaStream_t st = (cudaStream_t)stream;
-    int P = mbf_md_partial_count(sys->n_atoms);
+    const int P = md_blocks(sys);
     PROF_BEGIN("md_kick", st);
-    md_kick<<<dim3(P, sys->n_struct), MD_BLOCK, 0, st>>>(S, velocities, forces, inv_mass, dt, P, partial, energy,
-                                                         thermo, thermo_rows, counter, done);
+    md_kick<<<dim3(P, sys->n_struct), MD_BLOCK, 0, st>>>(S, velocities, forces, inv_mass, dt, md_items(sys), P, partial,
+                                                         energy, thermo, thermo_rows, counter, done);
     PROF_END("md_kick", st);
     MBF_CHECK_LAUNCH();
     return MBF_OK;
@@ -371,10 +383,11 @@ int mbf_md_kick_kick_drift_check(const mbf_system *sys, double *positions, doubl
         return MBF_ERR_ARGUMENT;
     SysView S = make_view(sys);
     cudaStream_t st = (cudaStream_t)stream;
-    int P = mbf_md_partial_count(sys->n_atoms);
+    const int P = md_blocks(sys);
     PROF_BEGIN("md_kick_kick_drift", st);
     md_kick_kick_drift_check<<<dim3(P, sys->n_struct), MD_BLOCK, 0, st>>>(
-        S, positions, velocities, forces, inv_mass, dt, P, partial, energy, thermo, thermo_rows, thermo_counter,
+        S, positions, velocities, forces, inv_mass, dt, md_items(sys), P, partial, energy, thermo, thermo_rows,
+        thermo_counter,
         ref_positions, d_max, r_list, r_cut, d_log, skin_counter, gate, cond_handle, done);
     PROF_END("md_kick_kick_drift", st);
     MBF_CHECK_LAUNCH();
