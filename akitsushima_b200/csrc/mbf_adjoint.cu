@@ -39,7 +39,8 @@
 namespace mbf {
 
 constexpr int ADJ_PB = 64;           // threads of a bond block
-constexpr int ADJ_PG = 148 * 4;      // bond blocks per list at most
+constexpr int ADJ_PG = 148 * 6;      // bond blocks per list at most
+constexpr int ADJ_FB = 128;          // threads per table entry of the final sums
 constexpr int ADJ_LPA = 8;           // lanes per atom of the row pass
 constexpr double ADJ_HALF_PI = 0.5 * 3.14159265358979323846;
 
@@ -209,6 +210,12 @@ __global__ void __launch_bounds__(ADJ_TB) te_adjoint_scatter(const int *__restri
 }
 
 // The kind blockIdx.y stands for and its block's share of the list.
+// Bonds per block of a list of np over at most g blocks, whole rounds of a
+// block (a share of 46 bonds for 64 threads took 72 us in the pair pass, of
+// 64 or 128 it takes 51); the blocks behind the list's end do nothing and
+// leave no sums.
+__device__ __forceinline__ int adj_per(int np, int g) { return ((np + g - 1) / g + ADJ_PB - 1) / ADJ_PB * ADJ_PB; }
+
 struct AdjShare {
     int si, sj, lower, first, end;
     __device__ __forceinline__ void load(const AdjTab &P, int n_tiles, const int *__restrict__ pos) {
@@ -217,7 +224,7 @@ struct AdjShare {
         sj = k >> 1;
         lower = k & 1;
         const int p0 = pos[(size_t)c * n_tiles], np = pos[(size_t)(c + 1) * n_tiles] - p0;
-        const int per = (np + gridDim.x - 1) / gridDim.x;
+        const int per = adj_per(np, gridDim.x);
         first = p0 + min(np, (int)blockIdx.x * per);
         end = p0 + min(np, ((int)blockIdx.x + 1) * per);
     }
@@ -285,11 +292,12 @@ __device__ __forceinline__ void adj_block_sums(double (&o)[NV], double *__restri
 // centre's legs, then with V = 1/2 f (fR + b fA) the eight parameters'
 // derivatives and tangents; zc = {gE V_z + (V_z)_t, V_z}, through which every
 // leg parameter acts on this bond.  Bound by FP64 latency: a thread per bond,
-// site sums in registers over the block's share of the list.  This pass and
-// the leg pass together replace one kernel in generic hyper-dual arithmetic
-// that staged every bond's sites in shared memory and summed them there by
-// table entry (329 us for 220,000 bonds of 38,600 SiC atoms; ADJ_MEASURED).
-__global__ void __launch_bounds__(ADJ_PB) adj_pair_sites(SysView S, const int *__restrict__ row_off, AdjTab P, AdjIn G,
+// site sums in registers over the block's share of the list.  220,000 bonds of
+// 38,600 SiC atoms: 50 us, the leg pass 74 (at the 140 and 165 registers the
+// compiler takes by itself, 7 and 6 blocks an SM, 61 and 101; at 12 blocks an
+// SM 64 and 90); one kernel in generic hyper-dual arithmetic that staged every
+// bond's sites in shared memory and summed them there by table entry took 329.
+__global__ void __launch_bounds__(ADJ_PB, 9) adj_pair_sites(SysView S, const int *__restrict__ row_off, AdjTab P, AdjIn G,
                                                          const AdjLeg *__restrict__ legs, const int *__restrict__ meta,
                                                          int n_tiles, const int *__restrict__ pos,
                                                          const int2 *__restrict__ bonds, double2 *__restrict__ zc,
@@ -297,6 +305,7 @@ __global__ void __launch_bounds__(ADJ_PB) adj_pair_sites(SysView S, const int *_
     const int ns = P.ns;
     AdjShare sh;
     sh.load(P, n_tiles, pos);
+    if (sh.first >= sh.end) return;  // uniform over the block
     const double *tp = P.tb + 10 * (sh.lower ? sh.si * ns + sh.sj : sh.sj * ns + sh.si);
     const double *tij = P.tb + 10 * (sh.si * ns + sh.sj);
     const double A = __ldg(tp + 1), B = __ldg(tp + 2), l1 = __ldg(tp + 3), l2 = __ldg(tp + 4), R = __ldg(tp + 5),
@@ -375,7 +384,7 @@ __global__ void __launch_bounds__(ADJ_PB) adj_pair_sites(SysView S, const int *_
 // The leg sites of one list for third atoms of species blockIdx.z: each term
 // z = gamma f g ex once more, with its derivatives in c, d, h, lambda3, gamma,
 // R, D and their tangents, weighted by the bond's coefficients.
-__global__ void __launch_bounds__(ADJ_PB) adj_leg_sites(const int *__restrict__ row_off, AdjTab P,
+__global__ void __launch_bounds__(ADJ_PB, 8) adj_leg_sites(const int *__restrict__ row_off, AdjTab P,
                                                         const AdjLeg *__restrict__ legs, const int *__restrict__ meta,
                                                         int n_tiles, const int *__restrict__ pos,
                                                         const int2 *__restrict__ bonds, const double2 *__restrict__ zc,
@@ -383,6 +392,7 @@ __global__ void __launch_bounds__(ADJ_PB) adj_leg_sites(const int *__restrict__ 
     const int ns = P.ns, sk = blockIdx.z;
     AdjShare sh;
     sh.load(P, n_tiles, pos);
+    if (sh.first >= sh.end) return;  // uniform over the block
     const double *tk = P.tb + 10 * (sh.si * ns + sk), *t3 = P.tri + 8 * ((sh.si * ns + sh.sj) * ns + sk);
     const bool valid = __ldg(tk) != 0.0 && __ldg(t3) != 0.0;
     const double pc = __ldg(t3 + 1), pd = __ldg(t3 + 2), ph = __ldg(t3 + 3), l3 = __ldg(t3 + 4), pm = __ldg(t3 + 5),
@@ -433,45 +443,54 @@ __global__ void __launch_bounds__(ADJ_PB) adj_leg_sites(const int *__restrict__ 
     adj_block_sums<7>(o, partial + ((size_t)blockIdx.y * ns + sk) * 7 * gridDim.x);
 }
 
-// One warp per table entry (tb (ns*ns, 10), then tri (ns^3, 8)): the block
+// One block per table entry (tb (ns*ns, 10), then tri (ns^3, 8)): the block
 // values of every (kind, site) row that reads the entry, then a fixed tree.
-__global__ void te_adjoint_final(int ns, int gP, const double *__restrict__ pair, const double *__restrict__ leg,
+__global__ void __launch_bounds__(ADJ_FB) te_adjoint_final(int ns, int gP, int n_tiles, const int *__restrict__ pos,
+                                 const double *__restrict__ pair, const double *__restrict__ leg,
                                  double *__restrict__ d_tb, double *__restrict__ d_tri) {
-    const int ne = 10 * ns * ns + 8 * ns * ns * ns;
-    const int e = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, l = threadIdx.x & 31;
-    if (e >= ne) return;  // whole warps leave together
+    const int e = blockIdx.x, l = threadIdx.x;
+    __shared__ double sums[ADJ_FB / 32];
     double acc = 0.0;
-    auto add_row = [&](const double *p) {  // four loads in flight a lane
+    auto kind = [&](int si, int sj, int lower) { return (si * ns + sj) * 2 + lower; };
+    // the block sums of one site of a list: four loads in flight a lane
+    auto add_row = [&](int c, const double *p) {
+        const int np = pos[(size_t)(c + 1) * n_tiles] - pos[(size_t)c * n_tiles];
+        if (np <= 0) return;
+        const int per = adj_per(np, gP), busy = (np + per - 1) / per;
         double x[4] = {0.0, 0.0, 0.0, 0.0};
-        for (int b = l; b < gP; b += 128) {
+        for (int b = l; b < busy; b += 4 * ADJ_FB) {
 #pragma unroll
             for (int k = 0; k < 4; ++k)
-                if (b + 32 * k < gP) x[k] += p[b + 32 * k];
+                if (b + ADJ_FB * k < busy) x[k] += p[b + ADJ_FB * k];
         }
         acc += (x[0] + x[1]) + (x[2] + x[3]);
     };
-    auto kind = [&](int si, int sj, int lower) { return (si * ns + sj) * 2 + lower; };
+    auto add_pair = [&](int c, int site) { add_row(c, pair + ((size_t)c * 8 + site) * gP); };
+    auto add_leg = [&](int c, int k, int site) { add_row(c, leg + (((size_t)c * ns + k) * 7 + site) * gP); };
     if (e < 10 * ns * ns) {
         const int ra = e / 10 / ns, rb = e / 10 % ns, col = e % 10;
         if (col >= 1 && col <= 6) {  // the pair record: read with lo = ra, hi = rb
-            add_row(pair + ((size_t)kind(ra, rb, 1) * 8 + col - 1) * gP);
-            add_row(pair + ((size_t)kind(rb, ra, 0) * 8 + col - 1) * gP);
+            add_pair(kind(ra, rb, 1), col - 1);
+            add_pair(kind(rb, ra, 0), col - 1);
         }
         if (col == 7 || col == 8)
-            for (int o = 0; o < 2; ++o) add_row(pair + ((size_t)kind(ra, rb, o) * 8 + col - 1) * gP);
+            for (int o = 0; o < 2; ++o) add_pair(kind(ra, rb, o), col - 1);
         if (col == 5 || col == 6)
             for (int sj = 0; sj < ns; ++sj)
-                for (int o = 0; o < 2; ++o) add_row(leg + (((size_t)kind(ra, sj, o) * ns + rb) * 7 + col) * gP);
+                for (int o = 0; o < 2; ++o) add_leg(kind(ra, sj, o), rb, col);
     } else {
         const int e3 = e - 10 * ns * ns, row = e3 / 8, col = e3 % 8;
         const int ra = row / (ns * ns), rb = row / ns % ns, k = row % ns;
         const int site = col >= 1 && col <= 4 ? col - 1 : (col == 6 ? 4 : -1);
         if (site >= 0)
-            for (int o = 0; o < 2; ++o) add_row(leg + (((size_t)kind(ra, rb, o) * ns + k) * 7 + site) * gP);
+            for (int o = 0; o < 2; ++o) add_leg(kind(ra, rb, o), k, site);
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(MBF_FULL, acc, o);
+    if ((l & 31) == 0) sums[l >> 5] = acc;
+    __syncthreads();
     if (l == 0) {
+        for (int w = 1; w < ADJ_FB / 32; ++w) acc += sums[w];
         if (e < 10 * ns * ns) d_tb[e] = acc;
         else d_tri[e - 10 * ns * ns] = acc;
     }
@@ -585,7 +604,7 @@ int mbf_tersoff_adjoint(const mbf_system *sys, const mbf_nlist *nl, const mbf_te
     PROF_END("te_adjoint_leg", st);
     MBF_CHECK_LAUNCH();
     PROF_BEGIN("te_adjoint_reduce", st);
-    te_adjoint_final<<<(L.ne * 32 + 127) / 128, 128, 0, st>>>(ns, L.gP, pair, leg, d_tb, d_tri);
+    te_adjoint_final<<<L.ne, ADJ_FB, 0, st>>>(ns, L.gP, L.n_tiles, pos, pair, leg, d_tb, d_tri);
     PROF_END("te_adjoint_reduce", st);
     MBF_CHECK_LAUNCH();
     return MBF_OK;
