@@ -332,29 +332,28 @@ __global__ void __launch_bounds__(EADJ_TA) eam_adjoint_embed(SysView S, EamAdjTa
     }
 }
 
-// Compaction, EADJ_LPA lanes per atom: the marked slots of its upper half as
-// pairs (atom of the earlier species, atom of the later) at the scanned
-// offsets, each list in atom then slot order.
+// Compaction, a warp per atom: the marked slots of its upper half as pairs
+// (atom of the earlier species, atom of the later) at the scanned offsets,
+// each list in atom then slot order.  A chain of loads: with 8 lanes an atom,
+// nine rounds over a half row of 67, it took 65 us with its scan for the 6.8 M
+// slots of 101,000 Ni3Al atoms, with 16 lanes 49, with 32 41.
 __global__ void __launch_bounds__(128) eam_adjoint_compact(int n_atoms, int ns, const int *__restrict__ types,
                                                            const int *__restrict__ row_off,
                                                            const int *__restrict__ upper, const int *__restrict__ nbr,
                                                            const unsigned char *__restrict__ mark,
                                                            const int *__restrict__ pos, int2 *__restrict__ pairs) {
-    constexpr int LPA = EADJ_LPA;
-    const int i = (blockIdx.x * blockDim.x + threadIdx.x) / LPA, sub = threadIdx.x & (LPA - 1);
-    if (i >= n_atoms) return;  // whole groups leave together
-    const int gl = threadIdx.x & 31 & ~(LPA - 1);
-    const unsigned gones = (1u << LPA) - 1u, gmask = gones << gl;
+    const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, sub = threadIdx.x & 31;
+    if (i >= n_atoms) return;  // whole warps leave together
     const int si = types[i], beg = upper[i], end = row_off[i + 1];
-    // lane b of the group keeps the next position in species b's list
+    // lane b keeps the next position in species b's list
     int next = sub < ns ? pos[(size_t)pair_code(si, sub, ns) * n_atoms + i] : 0;
     int mn = 0, jn = 0;
     if (beg + sub < end) {
         mn = mark[beg + sub];
         jn = nbr[beg + sub];
     }
-    for (int s0 = beg; s0 < end; s0 += LPA) {
-        const int m = mn, j = jn, s1 = s0 + LPA + sub;
+    for (int s0 = beg; s0 < end; s0 += 32) {
+        const int m = mn, j = jn, s1 = s0 + 32 + sub;
         mn = 0;
         if (s1 < end) {
             mn = mark[s1];
@@ -362,8 +361,8 @@ __global__ void __launch_bounds__(128) eam_adjoint_compact(int n_atoms, int ns, 
         }
         int o = -1;
         for (int b = 0; b < ns; ++b) {
-            const unsigned hit = (__ballot_sync(gmask, m == 1 + b) >> gl) & gones;
-            const int base = __shfl_sync(gmask, next, b, LPA);
+            const unsigned hit = __ballot_sync(MBF_FULL, m == 1 + b);
+            const int base = __shfl_sync(MBF_FULL, next, b);
             if (m == 1 + b) o = base + __popc(hit & ((1u << sub) - 1u));
             if (sub == b) next += __popc(hit);
         }
@@ -666,7 +665,7 @@ int mbf_eam_adjoint(const mbf_system *sys, const mbf_nlist *nl, const mbf_eam_ta
     PROF_BEGIN("eam_adjoint_compact", st);
     int rc = exclusive_scan(cnt, pos, L.nc * N, ws_at<int>(workspace, L.scan), st);
     if (rc != MBF_OK) return rc;
-    eam_adjoint_compact<<<rows, 128, 0, st>>>(N, ns, S.types, nl->row_off, nl->upper, nl->nbr, mark, pos, pairs);
+    eam_adjoint_compact<<<(N + 3) / 4, 128, 0, st>>>(N, ns, S.types, nl->row_off, nl->upper, nl->nbr, mark, pos, pairs);
     PROF_END("eam_adjoint_compact", st);
     MBF_CHECK_LAUNCH();
     PROF_BEGIN("eam_adjoint_pairs", st);
