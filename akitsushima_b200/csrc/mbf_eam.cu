@@ -930,7 +930,7 @@ struct CellView {
 
 // The gather reads each pair force once: a streaming load (evict-first),
 // so the forces do not displace the per-atom records from the caches
-// (60 against 66.6 us at 256k).
+// (60 against 66.6 us at 256k, before the loads went in rounds of K).
 __device__ __forceinline__ float4 ld_slot(const float4 *p) { return __ldcs(p); }
 __device__ __forceinline__ double3 ld_slot(const double3 *p) { return *p; }
 
@@ -1165,18 +1165,21 @@ __global__ void __launch_bounds__(EAM_BLOCK, Pol::Bounds::force(sizeof(T), CM))
 // (ChunkSums): a block per chunk of the reduction plan, 8 lanes per atom;
 // besides its atom's force each group adds the atom's record (entries sub
 // and sub + 8 of its 8 lanes), and the block finishes the chunk's and, if
-// last, the structure's sums.  The kernel waits on memory, so every load of
-// an atom is issued before any is used: its first GATHER_UNROLL x 8 lower
-// slots (an fcc row's lower half is about 40), its record and its
-// upper-pair force, with the next atom's row bounds one iteration ahead.
-constexpr int GATHER_UNROLL = 5;
+// last, the structure's sums.  The kernel waits on memory, so an atom's record,
+// its upper-pair force and K x 8 of its lower slots (an fcc row's lower half
+// is about 40) are requested before any is used, with the next atom's row
+// bounds one iteration ahead.  K = 4 for the 24-byte forces and 6 for the
+// 16-byte ones: 15.0 us for 32,000 atoms in float64 (18.7 with 5 and the rest
+// of a row one by one, 14.8 with 3, 16.9 with 6), 50.5 for 101,000 Ni3Al atoms
+// of 134 neighbours (64.5; 52.4; 53.4), 56.0 for 256,000 atoms mixed (59.9;
+// 60.5 with 3, 57.4 with 4).
 
 template <typename V3, int NT>
 __global__ void __launch_bounds__(NT, 1024 / NT) eam_gather_reduce(int n_slots, const int *__restrict__ row_off,
                                                         const int *__restrict__ upper, const V3 *__restrict__ slot_f,
                                                         const double *__restrict__ f_local,
                                                         double *__restrict__ forces, ChunkSums cs, Chk ck) {
-    constexpr int LPA = 8, G = NT / LPA;
+    constexpr int LPA = 8, G = NT / LPA, K = sizeof(V3) == 16 ? 6 : 4;
     const int c = blockIdx.x;
     const int s = cs.chunk[3 * c], a0 = cs.chunk[3 * c + 1], a1 = cs.chunk[3 * c + 2];
     const int sub = threadIdx.x & (LPA - 1), grp = threadIdx.x / LPA;
@@ -1206,25 +1209,19 @@ __global__ void __launch_bounds__(NT, 1024 / NT) eam_gather_reduce(int n_slots, 
             const double ra = rec[sub];
             const double rb = sub < ATOM_ACC - LPA ? rec[LPA + sub] : 0.0;
             if (sub < 3) fl = f_local[3 * (size_t)a + sub];
-            V3 w[GATHER_UNROLL];
+            for (int q = beg + sub; q < up; q += K * LPA) {
+                V3 w[K];
 #pragma unroll
-            for (int k = 0; k < GATHER_UNROLL; ++k) {
-                const int q = beg + sub + k * LPA;
-                if (q < up) w[k] = ld_slot(slot_f + q);
-            }
+                for (int k = 0; k < K; ++k)
+                    if (q + k * LPA < up) w[k] = ld_slot(slot_f + q + k * LPA);
 #pragma unroll
-            for (int k = 0; k < GATHER_UNROLL; ++k) {
-                if (beg + sub + k * LPA < up) {
-                    fx += (double)w[k].x;
-                    fy += (double)w[k].y;
-                    fz += (double)w[k].z;
+                for (int k = 0; k < K; ++k) {
+                    if (q + k * LPA < up) {
+                        fx += (double)w[k].x;
+                        fy += (double)w[k].y;
+                        fz += (double)w[k].z;
+                    }
                 }
-            }
-            for (int q = beg + sub + GATHER_UNROLL * LPA; q < up; q += LPA) {
-                const V3 v = ld_slot(slot_f + q);
-                fx += (double)v.x;
-                fy += (double)v.y;
-                fz += (double)v.z;
             }
             r0 += ra;
             r1 += rb;
