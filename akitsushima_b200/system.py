@@ -258,6 +258,17 @@ class Batch:
         self.pos.copy_(stage, non_blocking=True)
         self._stage_done.record(torch.cuda.current_stream(self.device))
 
+    def forces_to_host(self, forces):
+        """Device (N, 3) forces to a new host numpy array: a pinned block of
+        torch's caching host allocator, copied into directly (no second host
+        copy); the block returns to the cache when the caller drops it."""
+        if self.device.type != "cuda":
+            return forces.cpu().numpy()
+        out = torch.empty((self.n_atoms, 3), dtype=torch.float64, pin_memory=True)
+        out.copy_(forces, non_blocking=True)
+        torch.cuda.current_stream(self.device).synchronize()
+        return out.numpy()
+
     def results_to_host(self, packed, words):
         """Device results (a float64 vector whose first 3 N entries are the
         forces) and the evaluation's status words on the host: (forces (N, 3),
