@@ -524,6 +524,7 @@ __global__ void __launch_bounds__(NL_T, 4) nl_search(SysView S, const int *__res
                 if (lane >= o) ahead += t;
             }
             ahead_w[wid][lane] = ahead - chunk[lane];
+            __syncwarp();  // rank() below reads the other lanes' entries
             total = __shfl_sync(MBF_FULL, ahead, 31);
             wide = wide && total <= NL_CAP;
         }
