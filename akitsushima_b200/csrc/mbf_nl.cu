@@ -730,7 +730,9 @@ __device__ __forceinline__ int sort_row(const int *src, int n, int *out, int a, 
 // no physical density reaches, by insertion on one lane).
 // With `local`, each atom's position relative to the middle of its cell, in
 // float32, beside its index, in the cells' order (NaN for an atom whose cell
-// coordinate lies beyond 4096 boxes).
+// coordinate lies beyond 4096 boxes): the periodic image next to the cell
+// that nl_assign chose, whatever side of a cell face or of the box's own face
+// the rounding here puts the atom on.
 __global__ void nl_sort_cells(SysView S, const int *__restrict__ grids, int n_cells,
                               const int *__restrict__ cell_start, int *__restrict__ cell_atoms,
                               float4 *__restrict__ local) {
@@ -770,6 +772,7 @@ __global__ void nl_sort_cells(SysView S, const int *__restrict__ grids, int n_ce
                 const double s = p[0] * L[9 + q] + p[1] * L[12 + q] + p[2] * L[15 + q];
                 if (!(fabs(s) <= 4096.0)) far = true;
                 f[q] = s - floor(s) - (q == 0 ? m0 : q == 1 ? m1 : m2);
+                f[q] -= rint(f[q]);
             }
             const float x = (float)(f[0] * L[0] + f[1] * L[3] + f[2] * L[6]);
             local[b + k] = make_float4(far ? __int_as_float(0x7fffffff) : x,
