@@ -85,7 +85,11 @@ __device__ __forceinline__ RowStage stage_row(const SysView &S, const RowHead &h
     const unsigned gones = (1u << LPA) - 1u, gmask = gones << gl;
     RowStage o = {h.beg, 0, 0, h.si, h.bad};
     const int n = h.n;
-    if (n == 0) return o;
+    if (n == 0) {
+        // a rejected row (bad bounds or species) has no live slot
+        if (h.bad && sub < 4) live_mask[4 * (size_t)i + sub] = 0u;
+        return o;
+    }
     RowCell cell;
     cell.load(S, i);
     const double rc2 = rc * rc;

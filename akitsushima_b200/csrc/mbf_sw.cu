@@ -399,9 +399,9 @@ static int sw_eval(const mbf_system *sys, const mbf_nlist *nl, const mbf_sw_tabl
     else
         rc = tab->ns == 1 ? sw_dispatch<float, true>(mr, lpa, A, st) : sw_dispatch<float, false>(mr, lpa, A, st);
     if (rc != MBF_OK) return rc;
-    return gather_live(sys->n_struct, sys->n_atoms, nl->row_off, A.slot_G, A.live_mask, sw_row_limit(mr), err,
-                       A.f_local, forces, A.per_atom, plan, ws_at<double>(workspace, L.partial), energy, virial, sdone,
-                       st);
+    return gather_live(sys->n_struct, sys->n_atoms, nl->row_off, (int)nl->n_slots, A.slot_G, A.live_mask,
+                       sw_row_limit(mr), err, A.f_local, forces, A.per_atom, plan,
+                       ws_at<double>(workspace, L.partial), energy, virial, sdone, st);
 }
 
 extern "C" int mbf_sw_eval(const mbf_system *sys, const mbf_nlist *nl, const mbf_sw_tables *tab,

@@ -518,9 +518,9 @@ static int tersoff_eval(const mbf_system *sys, const mbf_nlist *nl, const mbf_te
     const int lpa = lanes_per_atom > 0 ? lanes_per_atom : 8;
     int rc = precision == MBF_FP64 ? te_rows<double>(nl->max_row, lpa, A, st) : te_rows<float>(nl->max_row, lpa, A, st);
     if (rc != MBF_OK) return rc;
-    return gather_live(sys->n_struct, sys->n_atoms, nl->row_off, A.slot_G, A.live_mask, te_row_limit(nl->max_row), err,
-                       A.f_local, forces, A.per_atom, plan, ws_at<double>(workspace, L.partial), energy, virial, sdone,
-                       st);
+    return gather_live(sys->n_struct, sys->n_atoms, nl->row_off, (int)nl->n_slots, A.slot_G, A.live_mask,
+                       te_row_limit(nl->max_row), err, A.f_local, forces, A.per_atom, plan,
+                       ws_at<double>(workspace, L.partial), energy, virial, sdone, st);
 }
 
 extern "C" int mbf_tersoff_eval(const mbf_system *sys, const mbf_nlist *nl, const mbf_tersoff_tables *tab,

@@ -137,7 +137,7 @@ int exclusive_scan(const int *in, int *out, int n, int *ws, cudaStream_t st) {
 constexpr int GATHER_K = 2;
 
 template <int NT>
-__global__ void __launch_bounds__(NT, 1024 / NT) gather_live_rows(const int *__restrict__ row_off,
+__global__ void __launch_bounds__(NT, 1024 / NT) gather_live_rows(const int *__restrict__ row_off, int n_slots,
                                                        const double *__restrict__ G,
                                                        const uint4 *__restrict__ live_mask, int row_limit,
                                                        int *__restrict__ err, const double *__restrict__ f_local,
@@ -174,7 +174,10 @@ __global__ void __launch_bounds__(NT, 1024 / NT) gather_live_rows(const int *__r
         } else {
             n = 0;
         }
-        if (n > row_limit) {
+        if ((unsigned)beg > (unsigned)n_slots || (unsigned)n > (unsigned)(n_slots - beg)) {
+            if (sub == 0) atomicOr(err, MBF_DEV_BAD_INDEX);
+            n = 0;
+        } else if (n > row_limit) {
             if (sub == 0) atomicOr(err, MBF_DEV_ROW_TOO_LONG);
             n = 0;
         }
@@ -210,20 +213,24 @@ __global__ void __launch_bounds__(NT, 1024 / NT) gather_live_rows(const int *__r
     chunk_sums_finish<NT>(cs, c, s, r0, r1);
 }
 
-int gather_live(int n_struct, int n_atoms, const int *row_off, const double *G, const unsigned *live_mask, int row_limit,
-                int *err, const double *f_local, double *forces, const double *per_atom, const mbf_reduce_plan *plan,
-                double *partial, double *energy, double *virial, unsigned *sdone, cudaStream_t st) {
+int gather_live(int n_struct, int n_atoms, const int *row_off, int n_slots, const double *G, const unsigned *live_mask,
+                int row_limit, int *err, const double *f_local, double *forces, const double *per_atom,
+                const mbf_reduce_plan *plan, double *partial, double *energy, double *virial, unsigned *sdone,
+                cudaStream_t st) {
     if (plan->n_chunks <= 0 || n_struct <= 0 || plan->n_chunks < n_struct || !sdone) return MBF_ERR_ARGUMENT;
     ChunkSums cs = {plan->chunk, plan->chunk_first, per_atom, partial, energy, virial, sdone};
     const uint4 *mask = reinterpret_cast<const uint4 *>(live_mask);
     PROF_BEGIN("gather_reduce", st);
     const int nt = chunk_block(n_atoms, plan->n_chunks);
     if (nt == 128)
-        gather_live_rows<128><<<plan->n_chunks, 128, 0, st>>>(row_off, G, mask, row_limit, err, f_local, forces, cs);
+        gather_live_rows<128><<<plan->n_chunks, 128, 0, st>>>(row_off, n_slots, G, mask, row_limit, err, f_local,
+                                                              forces, cs);
     else if (nt == 256)
-        gather_live_rows<256><<<plan->n_chunks, 256, 0, st>>>(row_off, G, mask, row_limit, err, f_local, forces, cs);
+        gather_live_rows<256><<<plan->n_chunks, 256, 0, st>>>(row_off, n_slots, G, mask, row_limit, err, f_local,
+                                                              forces, cs);
     else
-        gather_live_rows<512><<<plan->n_chunks, 512, 0, st>>>(row_off, G, mask, row_limit, err, f_local, forces, cs);
+        gather_live_rows<512><<<plan->n_chunks, 512, 0, st>>>(row_off, n_slots, G, mask, row_limit, err, f_local,
+                                                              forces, cs);
     PROF_END("gather_reduce", st);
     MBF_CHECK_LAUNCH();
     return MBF_OK;

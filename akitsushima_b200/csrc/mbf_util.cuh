@@ -21,12 +21,14 @@ int exclusive_scan(const int *in, int *out, int n, int *ws, cudaStream_t st);
 // per_atom into energy / virial (ChunkSums below).  A slot is read where the
 // row's bit in live_mask (4 words an atom, slot s of the row in word s / 32)
 // is set.  A row of more than row_limit entries (the evaluation's staging
-// bound) adds nothing and sets MBF_DEV_ROW_TOO_LONG in err, a pair count below
-// 0 MBF_DEV_BAD_INDEX.  sdone (n_struct words, the workspace's sdone region)
+// bound) adds nothing and sets MBF_DEV_ROW_TOO_LONG in err; one whose bounds
+// lie outside the n_slots slots adds nothing and sets MBF_DEV_BAD_INDEX, as
+// does a pair count below 0.  sdone (n_struct words, the workspace's sdone region)
 // must have been cleared by an earlier kernel of the evaluation (ClearWords).
-int gather_live(int n_struct, int n_atoms, const int *row_off, const double *G, const unsigned *live_mask, int row_limit,
-                int *err, const double *f_local, double *forces, const double *per_atom, const mbf_reduce_plan *plan,
-                double *partial, double *energy, double *virial, unsigned *sdone, cudaStream_t st);
+int gather_live(int n_struct, int n_atoms, const int *row_off, int n_slots, const double *G, const unsigned *live_mask,
+                int row_limit, int *err, const double *f_local, double *forces, const double *per_atom,
+                const mbf_reduce_plan *plan, double *partial, double *energy, double *virial, unsigned *sdone,
+                cudaStream_t st);
 
 // Words an evaluation needs zero in its later kernels (error words, the
 // completion counters), cleared by its first kernel instead of by memsets of
