@@ -13,15 +13,18 @@ namespace mbf {
 
 // Lanes per atom (LPA) is a template parameter chosen by the host (the
 // autotuner); GPB lane groups per block keep the staged rows near 15 KB, so
-// that registers and not shared memory bound the resident warps.
+// that registers and not shared memory bound the resident warps.  A block is
+// whole warps: where shared memory holds the rows of half a warp's groups
+// only, the other groups have no row.
 template <int MAXN, int LPA> struct SwGeom {
     static constexpr int WIDE = 512 / MAXN < 32 / LPA ? 512 / MAXN : 32 / LPA;  // a whole warp, if 48 KB hold it
     static constexpr int GPB = 256 / MAXN > WIDE ? 256 / MAXN : WIDE;
-    static constexpr int BLOCK = GPB * LPA;
+    static constexpr int BLOCK = GPB * LPA < 32 ? 32 : GPB * LPA;
+    static_assert(BLOCK % 32 == 0, "the record sums are over whole warps");
     // Resident threads per SM the kernel is compiled for (its registers):
     // with the gather, 64,000-atom Ge-Sn mixed at 640 / 768 / 896 threads 103 /
     // 98 / 96 us, 32,768-atom Ge-Sn float64 at 512 / 640 78 / 83.
-    static constexpr int min_blocks(int size) { return (size == 8 ? 512 : 896) / (BLOCK < 32 ? 32 : BLOCK); }
+    static constexpr int min_blocks(int size) { return (size == 8 ? 512 : 896) / BLOCK; }
 };
 
 struct SwDev {
@@ -169,7 +172,7 @@ __global__ void __launch_bounds__(SwGeom<MAXN, LPA>::BLOCK, SwGeom<MAXN, LPA>::m
     constexpr int NB = LPA < 8 ? LPA : 8, KS = LPA / NB;
     __shared__ SwRow<T, MAXN> rows[GPB];
     __shared__ SwTab<T> B;
-    const int i = blockIdx.x * GPB + threadIdx.x / LPA;
+    const int g = threadIdx.x / LPA, i = g < GPB ? blockIdx.x * GPB + g : S.n_atoms;
     RowHead head;
     head.load(S, row_off, i);
     clr.run();
@@ -177,7 +180,7 @@ __global__ void __launch_bounds__(SwGeom<MAXN, LPA>::BLOCK, SwGeom<MAXN, LPA>::m
     const int sub = threadIdx.x & (LPA - 1), gl = threadIdx.x & 31 & ~(LPA - 1);
     const unsigned gmask = ((1u << LPA) - 1u) << gl;
     const int lt = sub & (NB - 1), ks = sub / NB;
-    SwRow<T, MAXN> &R = rows[threadIdx.x / LPA];
+    SwRow<T, MAXN> &R = rows[g < GPB ? g : 0];
     const int ns = P.ns;
     const bool small = ns <= SW_SH;
     double fx = 0, fy = 0, fz = 0, e = 0;
