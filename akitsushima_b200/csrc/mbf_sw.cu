@@ -68,28 +68,41 @@ __device__ __forceinline__ double sw_reach2(const SwDev &P, int a, int b) {
     return r * r * (1.0 + 1e-6);
 }
 
-// The tables of up to SW_SH species in shared memory.
+// The records of an evaluation: of up to SW_SH species staged in shared
+// memory in T, of more read from the tables.  The kernel is compiled for
+// either, so every access is to one address space.
 constexpr int SW_SH = 3;
-template <typename T>
+template <typename T, bool STAGED>
 struct SwTab {
-    SwPair<T> pair[SW_SH * SW_SH];
-    SwLeg<T> leg[SW_SH * SW_SH];
-    SwTri<T> tri[SW_SH * SW_SH * SW_SH];
-    double reach2[SW_SH * SW_SH];
+    __device__ __forceinline__ void load(const SwDev &) {}
+    __device__ __forceinline__ SwPair<T> pair(const SwDev &P, int q) const { return sw_pair_row<T>(P.tb + 8 * q); }
+    __device__ __forceinline__ SwLeg<T> leg(const SwDev &P, int q) const { return sw_leg_row<T>(P.leg + 4 * q); }
+    __device__ __forceinline__ SwTri<T> tri(const SwDev &P, int q) const { return sw_tri_row<T>(P.tri + 4 * q); }
+    __device__ __forceinline__ double reach2(const SwDev &P, int a, int b) const { return sw_reach2(P, a, b); }
 };
 
 template <typename T>
-__device__ __forceinline__ void sw_load_tab(const SwDev &P, SwTab<T> &B) {
-    const int ns = P.ns;
-    if (ns > SW_SH) return;
-    for (int q = threadIdx.x; q < ns * ns; q += blockDim.x) {
-        B.pair[q] = sw_pair_row<T>(P.tb + 8 * q);
-        B.leg[q] = sw_leg_row<T>(P.leg + 4 * q);
-        B.reach2[q] = sw_reach2(P, q / ns, q % ns);
+struct SwTab<T, true> {
+    SwPair<T> pairs[SW_SH * SW_SH];
+    SwLeg<T> legs[SW_SH * SW_SH];
+    SwTri<T> tris[SW_SH * SW_SH * SW_SH];
+    double reach[SW_SH * SW_SH];
+    __device__ __forceinline__ SwPair<T> pair(const SwDev &, int q) const { return pairs[q]; }
+    __device__ __forceinline__ SwLeg<T> leg(const SwDev &, int q) const { return legs[q]; }
+    __device__ __forceinline__ SwTri<T> tri(const SwDev &, int q) const { return tris[q]; }
+    __device__ __forceinline__ double reach2(const SwDev &P, int a, int b) const { return reach[a * P.ns + b]; }
+    // By the whole block; ends in a barrier.
+    __device__ __forceinline__ void load(const SwDev &P) {
+        const int ns = P.ns;
+        for (int q = threadIdx.x; q < ns * ns; q += blockDim.x) {
+            pairs[q] = sw_pair_row<T>(P.tb + 8 * q);
+            legs[q] = sw_leg_row<T>(P.leg + 4 * q);
+            reach[q] = sw_reach2(P, q / ns, q % ns);
+        }
+        for (int q = threadIdx.x; q < ns * ns * ns; q += blockDim.x) tris[q] = sw_tri_row<T>(P.tri + 4 * q);
+        __syncthreads();
     }
-    for (int q = threadIdx.x; q < ns * ns * ns; q += blockDim.x) B.tri[q] = sw_tri_row<T>(P.tri + 4 * q);
-    __syncthreads();
-}
+};
 
 // Per-leg factors of the three-body term (engine/stillinger_weber.py:96-154):
 // h(i, j, k) = c3 E_j E_k (cos theta_jik - cos0)^2 with E_x = exp(gamma_x /
@@ -163,7 +176,7 @@ struct SwRow {
 // unit vectors: 136 -> 96 us there with the gather, mixed.  (The legs of a
 // block as one list, as the Tersoff kernel has them, took 104: its 23 KB of
 // staged legs leave fewer warps resident than the fuller lanes gain.)
-template <typename T, int MAXN, bool SYM, int LPA>
+template <typename T, int MAXN, bool SYM, bool STAGED, int LPA>
 __global__ void __launch_bounds__(SwGeom<MAXN, LPA>::BLOCK, SwGeom<MAXN, LPA>::min_blocks(sizeof(T)))
     sw_center(SysView S, const int *__restrict__ row_off, const int *__restrict__ nbr, const int *__restrict__ rev,
               SwDev P, double *__restrict__ slot_G, double *__restrict__ f_local, double *__restrict__ per_atom,
@@ -171,24 +184,23 @@ __global__ void __launch_bounds__(SwGeom<MAXN, LPA>::BLOCK, SwGeom<MAXN, LPA>::m
     constexpr int GPB = SwGeom<MAXN, LPA>::GPB;
     constexpr int NB = LPA < 8 ? LPA : 8, KS = LPA / NB;
     __shared__ SwRow<T, MAXN> rows[GPB];
-    __shared__ SwTab<T> B;
+    __shared__ SwTab<T, STAGED> B;
     const int g = threadIdx.x / LPA, i = g < GPB ? blockIdx.x * GPB + g : S.n_atoms;
     RowHead head;
     head.load(S, row_off, i);
     clr.run();
-    sw_load_tab<T>(P, B);
+    B.load(P);
     const int sub = threadIdx.x & (LPA - 1), gl = threadIdx.x & 31 & ~(LPA - 1);
     const unsigned gmask = ((1u << LPA) - 1u) << gl;
     const int lt = sub & (NB - 1), ks = sub / NB;
     SwRow<T, MAXN> &R = rows[g < GPB ? g : 0];
     const int ns = P.ns;
-    const bool small = ns <= SW_SH;
     double fx = 0, fy = 0, fz = 0, e = 0;
     double v[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
     head.slots<LPA>(nbr, rev, n_slots, ns, MAXN);
     const RowStage st = stage_row<LPA>(
         S, head, nbr, rev, n_slots, ns, P.rc, i, live_mask, so.vec,
-        [&](int a, int b) { return small ? B.reach2[a * ns + b] : sw_reach2(P, a, b); },
+        [&](int a, int b) { return B.reach2(P, a, b); },
         [&](int q, int s, int j, int sj, int rs, double dx, double dy, double dz, double r2) {
             R.x[q] = (T)dx;
             R.y[q] = (T)dy;
@@ -209,13 +221,13 @@ __global__ void __launch_bounds__(SwGeom<MAXN, LPA>::BLOCK, SwGeom<MAXN, LPA>::m
     for (int q = sub; q < nl; q += LPA) {
         const int ij = si * ns + R.sp[q];
         T E, D;
-        sw_leg<T>(R.r[q], small ? B.leg[ij] : sw_leg_row<T>(P.leg + 4 * ij), E, D);
+        sw_leg<T>(R.r[q], B.leg(P, ij), E, D);
         R.E[q] = E;
         R.D[q] = D;
     }
     __syncwarp(gmask);
     SwTri<T> own = {T(0), T(0)};
-    if (SYM) own = B.tri[0];
+    if (SYM) own = B.tri(P, 0);
     for (int t0 = 0; t0 < nl; t0 += NB) {
         const int t = t0 + lt;
         const bool act = t < nl;
@@ -242,8 +254,8 @@ __global__ void __launch_bounds__(SwGeom<MAXN, LPA>::BLOCK, SwGeom<MAXN, LPA>::m
                         Bc = T(4) * own.c * dc;
                     } else {
                         const int sk = R.sp[k], ra = rowj + sk, rb = (si * ns + sk) * ns + R.sp[t];
-                        const SwTri<T> q1 = small ? B.tri[ra] : sw_tri_row<T>(P.tri + 4 * ra);
-                        const SwTri<T> q2 = small ? B.tri[rb] : sw_tri_row<T>(P.tri + 4 * rb);
+                        const SwTri<T> q1 = B.tri(P, ra);
+                        const SwTri<T> q2 = B.tri(P, rb);
                         const T dc1 = cs - q1.cos0, dc2 = cs - q2.cos0;
                         const T b1 = q1.c * dc1, b2 = q2.c * dc2;
                         eh = b1 * dc1;
@@ -275,7 +287,7 @@ __global__ void __launch_bounds__(SwGeom<MAXN, LPA>::BLOCK, SwGeom<MAXN, LPA>::m
             // the pair record of the lower-indexed atom's species order
             const int pr = mt & 256 ? si * ns + sj : sj * ns + si;
             T V2, dV2;
-            sw_two<T>(r, small ? B.pair[pr] : sw_pair_row<T>(P.tb + 8 * pr), V2, dV2);
+            sw_two<T>(r, B.pair(P, pr), V2, dV2);
             e += 0.5 * (double)V2;
             const double hx = 0.5 * (double)(dV2 * ir);
             const T su = R.D[t] * sA - sB * ir;
@@ -322,34 +334,41 @@ struct SwArgs {
     SiteOut so;
 };
 
-template <typename T, int MAXN, bool SYM, int LPA>
+template <typename T, int MAXN, bool SYM, bool STAGED, int LPA>
 static int sw_launch(const SwArgs &A, cudaStream_t st) {
     constexpr int GPB = SwGeom<MAXN, LPA>::GPB, BLOCK = SwGeom<MAXN, LPA>::BLOCK;
     const int blocks = (A.S.n_atoms + GPB - 1) / GPB;
     PROF_BEGIN("sw_center", st);
-    sw_center<T, MAXN, SYM, LPA><<<blocks, BLOCK, 0, st>>>(A.S, A.nl->row_off, A.nl->nbr, A.nl->rev, A.P, A.slot_G,
-                                                           A.f_local, A.per_atom, A.live_mask,
-                                                      (int)A.nl->n_slots, A.clr, A.so);
+    sw_center<T, MAXN, SYM, STAGED, LPA><<<blocks, BLOCK, 0, st>>>(
+        A.S, A.nl->row_off, A.nl->nbr, A.nl->rev, A.P, A.slot_G, A.f_local, A.per_atom, A.live_mask,
+        (int)A.nl->n_slots, A.clr, A.so);
     PROF_END("sw_center", st);
     MBF_CHECK_LAUNCH();
     return MBF_OK;   // the eval's gather_live adds the slot forces
 }
 
-template <typename T, int MAXN, bool SYM>
+template <typename T, int MAXN, bool SYM, bool STAGED>
 static int sw_lpa(int lpa, const SwArgs &A, cudaStream_t st) {
     switch (lpa) {
-        case 4: return sw_launch<T, MAXN, SYM, 4>(A, st);
-        case 8: return sw_launch<T, MAXN, SYM, 8>(A, st);
-        case 16: return sw_launch<T, MAXN, SYM, 16>(A, st);
+        case 4: return sw_launch<T, MAXN, SYM, STAGED, 4>(A, st);
+        case 8: return sw_launch<T, MAXN, SYM, STAGED, 8>(A, st);
+        case 16: return sw_launch<T, MAXN, SYM, STAGED, 16>(A, st);
         default: return MBF_ERR_ARGUMENT;
     }
 }
 
-template <typename T, bool SYM>
+template <typename T, bool SYM, bool STAGED>
 static int sw_dispatch(int mr, int lpa, const SwArgs &A, cudaStream_t st) {
-    if (mr <= 32) return sw_lpa<T, 32, SYM>(lpa, A, st);
-    if (mr <= 64) return sw_lpa<T, 64, SYM>(lpa, A, st);
-    return sw_lpa<T, 128, SYM>(lpa, A, st);
+    if (mr <= 32) return sw_lpa<T, 32, SYM, STAGED>(lpa, A, st);
+    if (mr <= 64) return sw_lpa<T, 64, SYM, STAGED>(lpa, A, st);
+    return sw_lpa<T, 128, SYM, STAGED>(lpa, A, st);
+}
+
+// One species: every angle has one record; up to SW_SH: staged.
+template <typename T>
+static int sw_tables(int mr, int lpa, const SwArgs &A, cudaStream_t st) {
+    if (A.P.ns == 1) return sw_dispatch<T, true, true>(mr, lpa, A, st);
+    return A.P.ns <= SW_SH ? sw_dispatch<T, false, true>(mr, lpa, A, st) : sw_dispatch<T, false, false>(mr, lpa, A, st);
 }
 
 // The longest row sw_dispatch's choice for `mr` stages.
@@ -396,11 +415,7 @@ static int sw_eval(const mbf_system *sys, const mbf_nlist *nl, const mbf_sw_tabl
     A.clr = {(unsigned *)err, ERR_CLEAR_BYTES / 4, sdone, sys->n_struct};
     A.so = so;
     const int lpa = lanes_per_atom > 0 ? lanes_per_atom : 8, mr = nl->max_row;
-    int rc;
-    if (precision == MBF_FP64)
-        rc = tab->ns == 1 ? sw_dispatch<double, true>(mr, lpa, A, st) : sw_dispatch<double, false>(mr, lpa, A, st);
-    else
-        rc = tab->ns == 1 ? sw_dispatch<float, true>(mr, lpa, A, st) : sw_dispatch<float, false>(mr, lpa, A, st);
+    const int rc = precision == MBF_FP64 ? sw_tables<double>(mr, lpa, A, st) : sw_tables<float>(mr, lpa, A, st);
     if (rc != MBF_OK) return rc;
     return gather_live(sys->n_struct, sys->n_atoms, nl->row_off, (int)nl->n_slots, A.slot_G, A.live_mask,
                        sw_row_limit(mr), err, A.f_local, forces, A.per_atom, plan,
