@@ -530,7 +530,7 @@ static AdjLayout adj_layout(long long n_slots, int ns) {
     o = align256(o + sizeof(int) * ((size_t)L.kinds * L.n_tiles + 1));
     L.scan = o;
     o = align256(o + sizeof(int) * scan_workspace_ints(L.kinds * L.n_tiles));
-    L.total = o;
+    L.total = o + 16;  // the layout starts at the workspace's first 16-byte boundary
     return L;
 }
 
@@ -553,6 +553,7 @@ int mbf_tersoff_adjoint(const mbf_system *sys, const mbf_nlist *nl, const mbf_te
     if (nl->n_atoms != sys->n_atoms) return MBF_ERR_ARGUMENT;
     AdjLayout L = adj_layout(nl->n_slots, tab->ns);
     if (workspace_bytes < L.total) return MBF_ERR_WORKSPACE;
+    workspace = align16(workspace);
     cudaStream_t st = (cudaStream_t)stream;
     int ns = tab->ns;
     if (sys->n_atoms == 0 || nl->n_slots == 0) {

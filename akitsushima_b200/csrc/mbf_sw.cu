@@ -409,7 +409,7 @@ static int sw_eval(const mbf_system *sys, const mbf_nlist *nl, const mbf_sw_tabl
     A.slot_G = ws_at<double>(workspace, L.slot);
     A.f_local = ws_at<double>(workspace, L.f_local);
     A.per_atom = ws_at<double>(workspace, L.per_atom);
-    A.live_mask = ws_at<unsigned>(workspace, L.atom_aux);
+    A.live_mask = live_mask_at(workspace, L);
     unsigned *sdone = ws_at<unsigned>(workspace, L.sdone);
     int *err = ws_at<int>(workspace, L.err);
     A.clr = {(unsigned *)err, ERR_CLEAR_BYTES / 4, sdone, sys->n_struct};

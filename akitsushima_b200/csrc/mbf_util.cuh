@@ -180,6 +180,18 @@ static inline T *ws_at(void *ws, size_t off) {
     return reinterpret_cast<T *>(static_cast<char *>(ws) + off);
 }
 
+// The first 16-byte boundary at or after p: for a workspace at any multiple of
+// 8 bytes whose region is read in 16-byte words.
+static inline void *align16(void *p) { return reinterpret_cast<void *>(((size_t)p + 15) & ~(size_t)15); }
+
+// The three-body live masks, 16 bytes an atom, read as uint4: the atom_aux
+// region from its first 16-byte boundary on.  In a workspace that starts at
+// an odd multiple of 8 bytes the last mask ends in the region behind (pack),
+// which the three-body evaluations leave unused.
+static inline unsigned *live_mask_at(void *ws, const EvalLayout &L) {
+    return static_cast<unsigned *>(align16(ws_at<char>(ws, L.atom_aux)));
+}
+
 }  // namespace mbf
 
 // ---- launch profiler (CUDA events on the launching stream) -----------------

@@ -169,7 +169,9 @@ int mbf_nl_half_pairs(const mbf_nlist *nl, int *pair_i, int *pair_j, void *works
 
 /* ---- per-structure reduction workspace --------------------------------- */
 /* Bytes of the workspace every *_eval below needs (per-atom accumulators,
- * per-slot three-body forces and bond orders, reduction partials). */
+ * per-slot forces, live-slot masks, reduction partials).  A workspace starts at
+ * a multiple of 16 bytes for EAM, of 8 bytes for Tersoff and Stillinger-Weber
+ * (their adjoints likewise). */
 size_t mbf_eval_workspace_bytes(int n_atoms, long long n_slots, int n_chunks);
 
 /* Status words of the last evaluation that used `workspace` (host_words[4],
