@@ -1442,8 +1442,11 @@ static bool make_zk(const mbf_eam_tables *tab, ZK<T> &K) {
 }
 
 // The common grid of the pair and density tables, from the host copy of the
-// parameter rows: every one a spline on uniform knots (a row [1, x0, 1 / h, 0
-// ...]) with the same x0 and h; false otherwise.
+// parameter rows: every one a spline whose knots are x0 + k h up to rounding (a
+// row [1, x0, 1 / h, 1, 0 ...]) with the same x0 and h; false otherwise.
+// Knots that are uniform only to the 1e-9 that the interval's guess needs ([1,
+// x0, 1 / h, 0 ...]) keep the generic path, which reads them: an offset of
+// 1e-9 A is a force error of 1e-8 eV/A.
 static bool spline_grid(const mbf_eam_tables *tab, double &x0, double &ih) {
     if (tab->zhou_fused || tab->ns < 1 || tab->ns > SPL_MAXSP || !tab->P_host || !tab->rho_f_host || !tab->phi_f_host)
         return false;
@@ -1451,8 +1454,8 @@ static bool spline_grid(const mbf_eam_tables *tab, double &x0, double &ih) {
     for (int k = 0; k < ns + ns * ns; ++k) {
         const int f = k < ns ? tab->rho_f_host[k] : tab->phi_f_host[k - ns];
         const double *p = tab->P_host + (size_t)f * EAM_NCOL;
-        if (p[0] != 1.0 || !(p[2] > 0.0)) return false;
-        for (int c = 3; c < EAM_NCOL; ++c)
+        if (p[0] != 1.0 || !(p[2] > 0.0) || p[3] != 1.0) return false;
+        for (int c = 4; c < EAM_NCOL; ++c)
             if (p[c] != 0.0) return false;
         if (k == 0) {
             x0 = p[1];

@@ -232,6 +232,10 @@ class EAMPotential(DevicePotential):
                 h = (x[-1] - x[0]) / (len(x) - 1) if len(x) > 1 else 0.0
                 if len(x) > 2 and h > 0 and np.allclose(np.diff(x), h, rtol=1e-9, atol=0.0):
                     P[f, 0], P[f, 1], P[f, 2] = 1.0, x[0], 1.0 / h   # uniform knots
+                    # ... equal to x0 + k h up to rounding: the offset from a
+                    # knot may then be taken without reading it
+                    off_grid = np.abs(x - (x[0] + np.arange(len(x)) * (1.0 / P[f, 2]))).max()
+                    P[f, 3] = 1.0 if off_grid <= 4.0 * np.spacing(np.abs(x).max()) else 0.0
                 Xs.append(x)
                 cc = np.zeros((4, len(x)))
                 cc[:, :len(x) - 1] = c

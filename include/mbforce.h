@@ -192,7 +192,10 @@ int mbf_eval_status(const void *workspace, int *host_words, void *stream);
  *         uniform: P[0] = 1, P[1] = the first knot, P[2] = 1 / spacing
  *         (setfl tables are); its interval is then computed, not searched
  *         -- the same interval as searchsorted(side='right').  P row 0
- *         otherwise (binary search).
+ *         otherwise (binary search).  P[3] = 1 declares besides that every
+ *         knot equals P[1] + k / P[2] up to a few units in the last place of
+ *         the largest: the offset from a knot is then taken without reading
+ *         X.  P[3] = 0: the offset is from X.
  *   rho_f, F_f (ns,) int32 and phi_f (ns, ns) int32 function ids.        */
 typedef struct mbf_eam_tables {
     int ns;
