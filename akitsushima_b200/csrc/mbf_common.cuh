@@ -141,17 +141,6 @@ struct RowCell {
     }
 };
 
-// sqrt(r2) in float64 for a float32 evaluation: one Newton step on the
-// float32 inverse root (about 1e-14 relative), a fifth of sqrt()'s
-// instructions.  r2 within float32's range.
-__device__ __forceinline__ double root_near(double r2) {
-    const double q = (double)rsqrtf((float)r2), r0 = r2 * q;
-    return fma(0.5 * q, fma(-r0, r0, r2), r0);
-}
-template <typename T> __device__ __forceinline__ double leg_root(double r2);
-template <> __device__ __forceinline__ double leg_root<double>(double r2) { return sqrt(r2); }
-template <> __device__ __forceinline__ double leg_root<float>(double r2) { return root_near(r2); }
-
 // r and 1 / r of a leg in float64: the inverse root by one Newton step on the
 // float32 one for a float32 evaluation.
 template <typename T> __device__ __forceinline__ void leg_dist(double r2, double &r, double &ir);

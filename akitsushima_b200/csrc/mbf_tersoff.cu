@@ -72,18 +72,19 @@ __device__ __forceinline__ T te_g(T c2, T d2, T hc) {
     return T(1) + c2 * hc2 / (d2 * (d2 + hc2));
 }
 
-// g and dg/dcos from one reciprocal.
+// g and dg/dcos from one reciprocal, cd = c^2/d^2 with the record (for the
+// forces alone: a rounded cd would put the same error on every zeta).
 template <typename T>
-__device__ __forceinline__ void te_gdg(T c2, T d2, T hc, T &g, T &dg) {
-    const T hc2 = hc * hc, w = T(1) / (d2 * (d2 + hc2)), q = d2 * w;
-    g = T(1) + c2 * hc2 * w;
+__device__ __forceinline__ void te_gdg(T c2, T cd, T d2, T hc, T &g, T &dg) {
+    const T hc2 = hc * hc, q = T(1) / (d2 + hc2);
+    g = T(1) + cd * (hc2 * q);
     dg = T(-2) * c2 * hc * (q * q);
 }
 
 // An (i, j, k) record as the angle loops read it.
 template <typename T>
 struct TeTri {
-    T c2, d2, h, gam, l3, m, valid, pad;
+    T c2, d2, h, gam, l3, m, valid, cd;
 };
 
 template <typename T>
@@ -97,7 +98,7 @@ __device__ __forceinline__ TeTri<T> te_tri_row(const double *__restrict__ t) {
     q.l3 = (T)__ldg(t + 4);
     q.m = (T)__ldg(t + 5);
     q.valid = __ldg(t) != 0.0 ? T(1) : T(0);
-    q.pad = T(0);
+    q.cd = q.c2 / q.d2;
     return q;
 }
 
@@ -133,7 +134,11 @@ __device__ __forceinline__ void te_load_tab(const TeDev &P, TeTab<T> &B) {
     if (ns > TE_SH) return;
     for (int q = threadIdx.x; q < 10 * ns * ns; q += blockDim.x) B.tb[q] = P.tb[q];
     for (int q = threadIdx.x; q < ns * ns; q += blockDim.x) B.reach2[q] = te_reach2(P, q / ns, q % ns);
-    for (int q = threadIdx.x; q < ns * ns * ns; q += blockDim.x) B.tri[q] = te_tri_row<T>(P.tri + 8 * q);
+    for (int q = threadIdx.x; q < ns * ns * ns; q += blockDim.x) {
+        const double c = P.tri[8 * q + 1], d = P.tri[8 * q + 2];
+        B.tri[q] = te_tri_row<T>(P.tri + 8 * q);
+        B.tri[q].cd = (T)((c * c) / (d * d));
+    }
     __syncthreads();
     for (int a = threadIdx.x; a < ns; a += blockDim.x) {
         const TeTri<T> *t = B.tri + a * ns * ns;
@@ -245,16 +250,17 @@ __global__ void __launch_bounds__(TeGeom<MAXN, LPA>::BLOCK, TeGeom<MAXN, LPA>::m
         mine.si = st.si;
     }
     const int total = flatten_legs<GPB, MAXN, LPA>(F, g, sub, st.nl);
-    // a lane per leg: length and cutoff function
+    // a lane per leg: length (float64 in both precisions: the two-body part's)
+    // and cutoff function
     for (int q = threadIdx.x; q < total; q += BLOCK) {
         const int m = F.map[q], t = m & (MAXN - 1);
         TeRow<T, MAXN> &R = rows[m / MAXN];
-        const double r = leg_root<T>(R.e[t]);
+        const double r = sqrt(R.e[t]);
         const double *tk = tb + 10 * (R.si * ns + (R.meta[t] >> 9));
         T fk = T(0), dfk = T(0);
         if (tk[0] != 0.0) te_cut<T>((T)r, (T)tk[5], (T)tk[6], fk, dfk);
         te_put_r(R, t, r);
-        R.ir[t] = T(1) / (T)r;
+        R.ir[t] = (T)(1.0 / r);
         R.fk[t] = fk;
         R.dfk[t] = dfk;
     }
@@ -366,7 +372,7 @@ __global__ void __launch_bounds__(TeGeom<MAXN, LPA>::BLOCK, TeGeom<MAXN, LPA>::m
                 const T xk = R.x[k], yk = R.y[k], zk = R.z[k], ii = irs * R.ir[k];
                 const T c = (xs * xk + ys * yk + zs * zk) * ii;
                 T gg, dg;
-                te_gdg<T>(own.c2, own.d2, own.h - c, gg, dg);
+                te_gdg<T>(own.c2, own.cd, own.d2, own.h - c, gg, dg);
                 add(own.gam * w * dg, own.gam * ck * dft * gg * irs, c, ii, xk, yk, zk);
             }
         } else {
@@ -383,7 +389,7 @@ __global__ void __launch_bounds__(TeGeom<MAXN, LPA>::BLOCK, TeGeom<MAXN, LPA>::m
                 if (as_j) {
                     const TeTri<T> u = tri_row((si * ns + s_t) * ns + s_k);
                     if (u.valid != T(0)) {
-                        te_gdg<T>(u.c2, u.d2, u.h - c, gg, dg);
+                        te_gdg<T>(u.c2, u.cd, u.d2, u.h - c, gg, dg);
                         te_expo<T>(u.l3, u.m, rs - R.r[k], ex, dex);
                         const T w = ct * u.gam * fk;
                         A += w * dg * ex;
@@ -393,7 +399,7 @@ __global__ void __launch_bounds__(TeGeom<MAXN, LPA>::BLOCK, TeGeom<MAXN, LPA>::m
                 if (as_k) {
                     const TeTri<T> u = tri_row((si * ns + s_k) * ns + s_t);
                     if (u.valid != T(0)) {
-                        te_gdg<T>(u.c2, u.d2, u.h - c, gg, dg);
+                        te_gdg<T>(u.c2, u.cd, u.d2, u.h - c, gg, dg);
                         te_expo<T>(u.l3, u.m, R.r[k] - rs, ex, dex);
                         const T w = ck * u.gam;
                         A += w * ft * dg * ex;

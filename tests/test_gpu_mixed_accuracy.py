@@ -1,0 +1,44 @@
+"""Mixed precision is as accurate as its float32 terms allow: isolated pairs
+over the whole range of distances, site energies against the float64
+evaluation's."""
+import numpy as np
+import pytest
+
+from conftest import SW_SI
+
+pytestmark = pytest.mark.gpu
+
+ak = pytest.importorskip("akitsushima_b200")
+
+
+def _dimers(lo, hi, n=24, seed=3):
+    """n^3 pairs, 12 A apart, of distances spread evenly over (lo, hi) in
+    random directions: (lattice, positions, distances)."""
+    rng = np.random.default_rng(seed)
+    g = np.stack(np.meshgrid(*[np.arange(n)] * 3, indexing="ij"), -1).reshape(-1, 3) * 12.0
+    r = np.linspace(lo, hi, len(g) + 2)[1:-1]
+    u = rng.normal(size=g.shape)
+    u /= np.linalg.norm(u, axis=1)[:, None]
+    return np.eye(3) * 12.0 * n, np.concatenate([g, g + u * r[:, None]]), r
+
+
+def _site_energies(pot, lat, pos, device):
+    batch = ak.Batch.single(lat, pos, np.zeros(len(pos), np.int32), device=device)
+    dl = ak.DeviceNeighbourList(pot.r_cut + 0.3).build(batch)
+    out = {}
+    for prec in ("mixed", "fp64"):
+        out[prec] = pot.evaluate_sites(batch, dl, precision=prec)[1].cpu().numpy().copy()
+        pot.status()
+    return out["mixed"], out["fp64"]
+
+
+def test_tersoff_two_body_terms_are_float64(cuda_device):
+    """A pair alone has no zeta term, so its energy is the two-body part with
+    bond order 1, float64 in both precisions: the same operations on the same
+    distance.  2e-15 of the energy scale allows for a compiler's different
+    contraction."""
+    pot = ak.TersoffPotential(ak.TERSOFF_SI_1988, species=["Si"])
+    lat, pos, _ = _dimers(1.9, pot.r_cut)
+    mixed, fp64 = _site_energies(pot, lat, pos, cuda_device)
+    assert np.abs(fp64).max() > 0.5
+    assert np.abs(mixed - fp64).max() <= 2e-15 * np.abs(fp64).max()
