@@ -122,6 +122,17 @@ __device__ __forceinline__ void sw_leg(T r, const SwLeg<T> &l, T &E, T &D) {
     if (E != T(0)) D = -l.gam / (l.sig * d * d);
 }
 
+// x^-4 as accurate as pow(): in float64 for a float32 evaluation (once per
+// leg), with the square's rounding carried along in float64.
+__device__ __forceinline__ float sw_inv4(float x) {
+    const double x2 = (double)x * (double)x;
+    return (float)(1.0 / (x2 * x2));
+}
+__device__ __forceinline__ double sw_inv4(double x) {
+    const double x2 = x * x, e = fma(x, x, -x2);
+    return 1.0 / fma(x2, x2, 2.0 * x2 * e);
+}
+
 // Two-body energy and its r-derivative (engine/stillinger_weber.py:23-52).
 template <typename T>
 __device__ __forceinline__ void sw_two(T r, const SwPair<T> &t, T &V2, T &dV2) {
@@ -129,18 +140,14 @@ __device__ __forceinline__ void sw_two(T r, const SwPair<T> &t, T &V2, T &dV2) {
     dV2 = T(0);
     const T x = r / t.sig;
     if (t.valid == T(0) || !(x < t.a)) return;
-    const T tt = T(1) / (x - t.a), ex = clamped_exp<T>(tt), ix = T(1) / x;
+    const T tt = T(1) / (x - t.a), ex = clamped_exp<T>(tt);
     T xp, xq;
-    if (t.p == T(4)) {  // the published silicon exponents need no pow
-        const T i2 = ix * ix;
-        xp = i2 * i2;
-    } else {
-        xp = RT<T>::pw(x, -t.p);
-    }
+    if (t.p == T(4)) xp = sw_inv4(x);  // the published silicon exponents need no pow
+    else xp = RT<T>::pw(x, -t.p);
     xq = t.q == T(0) ? T(1) : RT<T>::pw(x, -t.q);
     const T w = t.eps * t.A * ex, u = t.B * xp - xq;
     V2 = w * u;
-    dV2 = w * ((-t.p * t.B * xp + t.q * xq) * ix - u * (tt * tt)) / t.sig;
+    dV2 = w * ((-t.p * t.B * xp + t.q * xq) / x - u * (tt * tt)) / t.sig;
 }
 
 // One centre's legs in shared memory, compacted in slot order: displacement

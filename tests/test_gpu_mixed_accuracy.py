@@ -42,3 +42,24 @@ def test_tersoff_two_body_terms_are_float64(cuda_device):
     mixed, fp64 = _site_energies(pot, lat, pos, cuda_device)
     assert np.abs(fp64).max() > 0.5
     assert np.abs(mixed - fp64).max() <= 2e-15 * np.abs(fp64).max()
+
+
+def test_sw_pair_term_rounds_its_power_once(cuda_device):
+    """The float32 pair term of silicon (p = 4) errs as its formula does in
+    float32 with x^-4 rounded once, emulated here: the same rms over 13,824
+    distances.  The rms of so many has a spread of 0.6 %; 1.5 % is allowed.
+    x^-4 from 1 / x by two squarings errs 3.4 % more."""
+    f = np.float32
+    pot = ak.StillingerWeberPotential(SW_SI, species=["Si"])
+    lat, pos, r = _dimers(2.0, 3.6)
+    mixed, fp64 = _site_energies(pot, lat, pos, cuda_device)
+    n = len(r)
+    e = mixed[:n] + mixed[n:]
+    np.testing.assert_allclose(fp64[:n], fp64[n:], rtol=1e-12)
+    eps, sig, a, A, B = (f(SW_SI[k]) for k in ("epsilon", "sigma", "a", "A", "B"))
+    x = r.astype(f) / sig
+    ex = np.exp((f(1) / (x - a)).astype(float)).astype(f)
+    emulated = eps * A * ex * (B * (x.astype(float) ** -4).astype(f) - f(1))
+    exact = 2.0 * fp64[:n]
+    rms = lambda v: np.sqrt(np.mean((v - exact) ** 2))  # noqa: E731
+    assert rms(e) <= 1.015 * rms(emulated)
