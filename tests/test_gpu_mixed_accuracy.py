@@ -4,11 +4,13 @@ evaluation's."""
 import numpy as np
 import pytest
 
-from conftest import SW_SI
+from conftest import FCC, SW_SI, cubic
 
 pytestmark = pytest.mark.gpu
 
 ak = pytest.importorskip("akitsushima_b200")
+from akitsushima_b200 import eam  # noqa: E402
+from akitsushima_b200.published_parameters import ZHOU_2004  # noqa: E402
 
 
 def _dimers(lo, hi, n=24, seed=3):
@@ -63,3 +65,18 @@ def test_sw_pair_term_rounds_its_power_once(cuda_device):
     exact = 2.0 * fp64[:n]
     rms = lambda v: np.sqrt(np.mean((v - exact) ** 2))  # noqa: E731
     assert rms(e) <= 1.015 * rms(emulated)
+
+
+def test_setfl_energy_has_no_bias(cuda_device):
+    """Each pair's float32 value errs by parts of 1e-7 of tenths of an eV in
+    either direction, so over 4000 atoms of about 40 pairs each the mean
+    energy error averages to some 1e-9 eV an atom (3e-9 measured with a
+    float64 1 / r); an inverse distance that errs to one side leaves 2e-8."""
+    lat, pos, _ = cubic(FCC, 3.58, 10, ["x"] * 4, rattle=0.08, seed=1)
+    ids = np.random.default_rng(6).integers(0, 2, len(pos)).astype(np.int32)
+    pot = eam.tabulate(ak.zhou_eam({s: ZHOU_2004[s] for s in ("Cu", "Ni")}, ["Cu", "Ni"]))
+    batch = ak.Batch.single(lat, pos, ids, device=cuda_device)
+    dl = ak.DeviceNeighbourList(pot.r_cut + 0.3).build(batch)
+    e = {p: float(pot.evaluate(batch, dl, precision=p).energy[0]) for p in ("mixed", "fp64")}
+    pot.status()
+    assert abs(e["mixed"] - e["fp64"]) < 1e-8 * len(pos)
