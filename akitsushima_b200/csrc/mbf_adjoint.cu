@@ -397,7 +397,8 @@ __global__ void __launch_bounds__(ADJ_PB, 8) adj_leg_sites(const int *__restrict
     const bool valid = __ldg(tk) != 0.0 && __ldg(t3) != 0.0;
     const double pc = __ldg(t3 + 1), pd = __ldg(t3 + 2), ph = __ldg(t3 + 3), l3 = __ldg(t3 + 4), pm = __ldg(t3 + 5),
                  gam = __ldg(t3 + 6), R = __ldg(tk + 5), D = __ldg(tk + 6);
-    const double d2 = pd * pd, c2 = pc * pc, id2 = 1.0 / d2, id3 = id2 / pd, iD = 1.0 / D;
+    const double d2 = pd * pd, c2 = pc * pc, id2 = 1.0 / d2, id3 = id2 / pd;
+    const double iD = D != 0.0 ? 1.0 / D : 0.0;  // a sharp cutoff has no slope to scale
     double o[7];
 #pragma unroll
     for (int k = 0; k < 7; ++k) o[k] = 0.0;
