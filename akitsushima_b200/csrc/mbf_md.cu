@@ -15,20 +15,26 @@
 
 namespace mbf {
 
-// Threads per block of the kick kernels and the atoms a thread takes, one
-// partial sum a block.  A step
-// of a few thousand atoms waits on one atom's chain of loads and float64
-// arithmetic, not on throughput: with 1024 atoms a block in four rounds a
-// block of ten steps of 4096 Tersoff atoms took 347 us, with 128 it takes 313
-// (256: 321); 64,000 atoms 853 against 835.  A batch keeps the 1024: its grid
-// has a block column per structure for the atoms of all.
-constexpr int MD_BLOCK = 128;
+// Threads per block of the kick kernels (NT) and the atoms a thread takes
+// (ITEMS), one partial sum a block.  A step of a few thousand atoms waits on
+// one atom's chain of loads and float64 arithmetic, not on throughput, so one
+// structure of up to 65,536 atoms takes an atom a thread in blocks of 128: the
+// fused kick of 4096 atoms 7.4 us against 10.3 with four a thread in blocks of
+// 256, a block of ten steps of 4096 Tersoff atoms 303 against 347.  Beyond, the
+// last block's sum over one partial of every 128 atoms costs more than that
+// gains: fused kick at 64,000 atoms 8.8 against 10.3 us, at 96,000 both 10.3,
+// at 256,000 20.4 against 12.3, at four million 181 against 126.  A batch has a
+// block column per structure for the atoms of all, most of them empty: four a
+// thread too (4 x 100,000 atoms, second half kick: 15.4 us; eight a thread in
+// blocks of 128 took 16.3).
+constexpr int MD_SMALL_ATOMS = 65536;
+constexpr int MD_SMALL_NT = 128, MD_NT = 256, MD_ITEMS = 4;
 
-static int md_items(const mbf_system *sys) { return sys->n_struct > 1 ? 8 : 1; }
+static bool md_small(const mbf_system *sys) { return sys->n_struct == 1 && sys->n_atoms <= MD_SMALL_ATOMS; }
 
-static int md_blocks(const mbf_system *sys) {
-    const int chunk = MD_BLOCK * md_items(sys);
-    return sys->n_atoms <= 0 ? 1 : (sys->n_atoms + chunk - 1) / chunk;
+static int md_blocks(int n_atoms, bool small) {
+    const int chunk = small ? MD_SMALL_NT : MD_NT * MD_ITEMS;
+    return n_atoms <= 0 ? 1 : (n_atoms + chunk - 1) / chunk;
 }
 
 // v += dt/2 a; r += dt v; frac = r @ inv(L), frac -= floor(frac),
@@ -155,35 +161,41 @@ __device__ __forceinline__ double block_sum(double v, double *sh) {
 // (mass = 1 / inv_mass in amu / conv units: conv cancels in m v^2 / conv).
 // The block that finishes last then sums the partials into the thermo row
 // (md_thermo's arithmetic, so the same bits) and resets `done`.
+template <int NT>
 __device__ void md_thermo_body(int n_struct, int P, const double *__restrict__ partial,
                                const double *__restrict__ energy, double *__restrict__ thermo, int rows,
                                int *__restrict__ counter, double *sh);
 
-__global__ void __launch_bounds__(MD_BLOCK) md_kick(SysView S, double *__restrict__ vel,
+template <int NT, int ITEMS>
+__global__ void __launch_bounds__(NT) md_kick(SysView S, double *__restrict__ vel,
                                                     const double *__restrict__ F,
-                                                    const double *__restrict__ im, double dt, int items, int P,
+                                                    const double *__restrict__ im, double dt, int P,
                                                     double *__restrict__ partial,
                                                     const double *__restrict__ energy,
                                                     double *__restrict__ thermo, int rows,
                                                     int *__restrict__ counter, unsigned *__restrict__ done) {
-    __shared__ double sh[MD_BLOCK / 32];
+    __shared__ double sh[NT / 32];
     __shared__ bool last;
     int s = blockIdx.y;
     int beg = S.n_struct > 1 ? S.struct_off[s] : 0;
     int end = S.n_struct > 1 ? S.struct_off[s + 1] : S.n_atoms;
     double acc = 0.0;
-    const int first = beg + blockIdx.x * (items * MD_BLOCK), stop = min(end, first + items * MD_BLOCK);
-    for (int a = first + threadIdx.x; a < stop; a += MD_BLOCK) {
-        size_t o = 3 * (size_t)a;
-        double w = im[a];
-        double h = 0.5 * dt * w;
-        double vx = vel[o] + h * F[o], vy = vel[o + 1] + h * F[o + 1], vz = vel[o + 2] + h * F[o + 2];
-        vel[o] = vx;
-        vel[o + 1] = vy;
-        vel[o + 2] = vz;
-        acc += (vx * vx + vy * vy + vz * vz) / w;
+    const int first = beg + blockIdx.x * (NT * ITEMS);
+#pragma unroll
+    for (int k = 0; k < ITEMS; ++k) {
+        const int a = first + k * NT + threadIdx.x;
+        if (a < end) {
+            size_t o = 3 * (size_t)a;
+            double w = im[a];
+            double h = 0.5 * dt * w;
+            double vx = vel[o] + h * F[o], vy = vel[o + 1] + h * F[o + 1], vz = vel[o + 2] + h * F[o + 2];
+            vel[o] = vx;
+            vel[o + 1] = vy;
+            vel[o + 2] = vz;
+            acc += (vx * vx + vy * vy + vz * vz) / w;
+        }
     }
-    acc = block_sum<MD_BLOCK>(acc, sh);
+    acc = block_sum<NT>(acc, sh);
     if (threadIdx.x == 0) {
         partial[(size_t)s * P + blockIdx.x] = acc;
         __threadfence();
@@ -191,7 +203,7 @@ __global__ void __launch_bounds__(MD_BLOCK) md_kick(SysView S, double *__restric
     }
     __syncthreads();
     if (!last) return;
-    md_thermo_body(S.n_struct, P, partial, energy, thermo, rows, counter, sh);
+    md_thermo_body<NT>(S.n_struct, P, partial, energy, thermo, rows, counter, sh);
     if (threadIdx.x == 0) *done = 0u;
 }
 
@@ -204,14 +216,15 @@ __global__ void __launch_bounds__(MD_BLOCK) md_kick(SysView S, double *__restric
 // displacement maximum of a warp belongs to one structure); the block that
 // finishes last writes the thermo row of the step that ended and then takes
 // the rebuild decision of the next (md_kick_drift_check's tail).
-__global__ void __launch_bounds__(MD_BLOCK) md_kick_kick_drift_check(
+template <int NT, int ITEMS>
+__global__ void __launch_bounds__(NT) md_kick_kick_drift_check(
     SysView S, double *__restrict__ pos, double *__restrict__ vel, const double *__restrict__ F,
-    const double *__restrict__ im, double dt, int items, int P, double *__restrict__ partial,
+    const double *__restrict__ im, double dt, int P, double *__restrict__ partial,
     const double *__restrict__ energy, double *__restrict__ thermo, int rows, int *__restrict__ tcounter,
     const double *__restrict__ ref, unsigned long long *__restrict__ dmax, double r_list, double r_cut,
     double *__restrict__ d_log, int *__restrict__ scounter, int *__restrict__ gate, unsigned long long cond,
     unsigned *__restrict__ done) {
-    __shared__ double sh[MD_BLOCK / 32];
+    __shared__ double sh[NT / 32];
     __shared__ bool last;
     int s = blockIdx.y;
     int beg = S.n_struct > 1 ? S.struct_off[s] : 0;
@@ -219,40 +232,44 @@ __global__ void __launch_bounds__(MD_BLOCK) md_kick_kick_drift_check(
     const double *c = S.cells + 18 * (size_t)s;
     double acc = 0.0;
     unsigned long long bits = 0ull;
-    const int first = beg + blockIdx.x * (items * MD_BLOCK), stop = min(end, first + items * MD_BLOCK);
-    for (int a = first + threadIdx.x; a < stop; a += MD_BLOCK) {
-        size_t o = 3 * (size_t)a;
-        double w = im[a];
-        double h = 0.5 * dt * w;
-        double fx = F[o], fy = F[o + 1], fz = F[o + 2];
-        double vx = vel[o] + h * fx, vy = vel[o + 1] + h * fy, vz = vel[o + 2] + h * fz;
-        acc += (vx * vx + vy * vy + vz * vz) / w;
-        vx = vx + h * fx;
-        vy = vy + h * fy;
-        vz = vz + h * fz;
-        double x = pos[o] + dt * vx, y = pos[o + 1] + dt * vy, z = pos[o + 2] + dt * vz;
-        double s0 = x * c[9] + y * c[12] + z * c[15];
-        double s1 = x * c[10] + y * c[13] + z * c[16];
-        double s2 = x * c[11] + y * c[14] + z * c[17];
-        s0 -= floor(s0);
-        s1 -= floor(s1);
-        s2 -= floor(s2);
-        if (s0 >= 1.0) s0 = 0.0;
-        if (s1 >= 1.0) s1 = 0.0;
-        if (s2 >= 1.0) s2 = 0.0;
-        double px = s0 * c[0] + s1 * c[3] + s2 * c[6];
-        double py = s0 * c[1] + s1 * c[4] + s2 * c[7];
-        double pz = s0 * c[2] + s1 * c[5] + s2 * c[8];
-        pos[o] = px;
-        pos[o + 1] = py;
-        pos[o + 2] = pz;
-        vel[o] = vx;
-        vel[o + 1] = vy;
-        vel[o + 2] = vz;
-        double dx, dy, dz;
-        mic_exact(c, px - ref[o], py - ref[o + 1], pz - ref[o + 2], dx, dy, dz);
-        unsigned long long b = (unsigned long long)__double_as_longlong(sqrt(dx * dx + dy * dy + dz * dz));
-        bits = b > bits ? b : bits;
+    const int first = beg + blockIdx.x * (NT * ITEMS);
+#pragma unroll
+    for (int k = 0; k < ITEMS; ++k) {
+        const int a = first + k * NT + threadIdx.x;
+        if (a < end) {
+            size_t o = 3 * (size_t)a;
+            double w = im[a];
+            double h = 0.5 * dt * w;
+            double fx = F[o], fy = F[o + 1], fz = F[o + 2];
+            double vx = vel[o] + h * fx, vy = vel[o + 1] + h * fy, vz = vel[o + 2] + h * fz;
+            acc += (vx * vx + vy * vy + vz * vz) / w;
+            vx = vx + h * fx;
+            vy = vy + h * fy;
+            vz = vz + h * fz;
+            double x = pos[o] + dt * vx, y = pos[o + 1] + dt * vy, z = pos[o + 2] + dt * vz;
+            double s0 = x * c[9] + y * c[12] + z * c[15];
+            double s1 = x * c[10] + y * c[13] + z * c[16];
+            double s2 = x * c[11] + y * c[14] + z * c[17];
+            s0 -= floor(s0);
+            s1 -= floor(s1);
+            s2 -= floor(s2);
+            if (s0 >= 1.0) s0 = 0.0;
+            if (s1 >= 1.0) s1 = 0.0;
+            if (s2 >= 1.0) s2 = 0.0;
+            double px = s0 * c[0] + s1 * c[3] + s2 * c[6];
+            double py = s0 * c[1] + s1 * c[4] + s2 * c[7];
+            double pz = s0 * c[2] + s1 * c[5] + s2 * c[8];
+            pos[o] = px;
+            pos[o + 1] = py;
+            pos[o + 2] = pz;
+            vel[o] = vx;
+            vel[o + 1] = vy;
+            vel[o + 2] = vz;
+            double dx, dy, dz;
+            mic_exact(c, px - ref[o], py - ref[o + 1], pz - ref[o + 2], dx, dy, dz);
+            unsigned long long b = (unsigned long long)__double_as_longlong(sqrt(dx * dx + dy * dy + dz * dz));
+            bits = b > bits ? b : bits;
+        }
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -260,7 +277,7 @@ __global__ void __launch_bounds__(MD_BLOCK) md_kick_kick_drift_check(
         bits = b > bits ? b : bits;
     }
     if ((threadIdx.x & 31) == 0 && bits) atomicMax(dmax + s, bits);
-    acc = block_sum<MD_BLOCK>(acc, sh);
+    acc = block_sum<NT>(acc, sh);
     if (threadIdx.x == 0) partial[(size_t)s * P + blockIdx.x] = acc;
     __threadfence();
     __syncthreads();
@@ -274,7 +291,7 @@ __global__ void __launch_bounds__(MD_BLOCK) md_kick_kick_drift_check(
         checks = *scounter;
         d_first = atomicExch(dmax, 0ull);
     }
-    md_thermo_body(S.n_struct, P, partial, energy, thermo, rows, tcounter, sh);
+    md_thermo_body<NT>(S.n_struct, P, partial, energy, thermo, rows, tcounter, sh);
     if (threadIdx.x != 0) return;
     int row = checks % rows;
     int need = 0;
@@ -292,6 +309,7 @@ __global__ void __launch_bounds__(MD_BLOCK) md_kick_kick_drift_check(
 // With inv_mass = conv / m the partials hold sum m v^2 / conv, so the
 // kinetic energy is half their sum, in eV (the reference's
 // 0.5 sum m v^2 / EV_ANG_TO_AMU_ANG_FS2, :243-244).
+template <int NT>
 __device__ void md_thermo_body(int n_struct, int P, const double *__restrict__ partial,
                                const double *__restrict__ energy, double *__restrict__ thermo, int rows,
                                int *__restrict__ counter, double *sh) {
@@ -299,8 +317,8 @@ __device__ void md_thermo_body(int n_struct, int P, const double *__restrict__ p
     for (int s = 0; s < n_struct; ++s) {
         const double e = energy[s];
         double v = 0.0;
-        for (int k = threadIdx.x; k < P; k += MD_BLOCK) v += __ldcg(partial + (size_t)s * P + k);
-        v = block_sum<MD_BLOCK>(v, sh);
+        for (int k = threadIdx.x; k < P; k += NT) v += __ldcg(partial + (size_t)s * P + k);
+        v = block_sum<NT>(v, sh);
         if (threadIdx.x == 0) {
             double *t = thermo + 2 * ((size_t)row * n_struct + s);
             t[0] = e;
@@ -325,14 +343,13 @@ int mbf_md_kick_drift(const mbf_system *sys, double *positions, double *velociti
     SysView S = make_view(sys);
     cudaStream_t st = (cudaStream_t)stream;
     PROF_BEGIN("md_kick_drift", st);
-    md_kick_drift<<<(sys->n_atoms + MD_BLOCK - 1) / MD_BLOCK, MD_BLOCK, 0, st>>>(S, positions, velocities, forces,
-                                                                               inv_mass, dt);
+    md_kick_drift<<<(sys->n_atoms + MD_NT - 1) / MD_NT, MD_NT, 0, st>>>(S, positions, velocities, forces, inv_mass, dt);
     PROF_END("md_kick_drift", st);
     MBF_CHECK_LAUNCH();
     return MBF_OK;
 }
 
-int mbf_md_partial_count(int n_atoms) { return n_atoms <= 0 ? 1 : (n_atoms + MD_BLOCK - 1) / MD_BLOCK; }
+int mbf_md_partial_count(int n_atoms) { return md_blocks(n_atoms, n_atoms <= MD_SMALL_ATOMS); }
 
 int mbf_md_kick(const mbf_system *sys, double *velocities, const double *forces, const double *inv_mass,
                 double dt, const double *energy, double *partial, double *thermo, int thermo_rows,
@@ -342,10 +359,16 @@ int mbf_md_kick(const mbf_system *sys, double *velocities, const double *forces,
         return MBF_ERR_ARGUMENT;
     SysView S = make_view(sys);
     cudaStream_t st = (cudaStream_t)stream;
-    const int P = md_blocks(sys);
+    const bool small = md_small(sys);
+    const int P = md_blocks(sys->n_atoms, small);
+    const dim3 grid(P, sys->n_struct);
     PROF_BEGIN("md_kick", st);
-    md_kick<<<dim3(P, sys->n_struct), MD_BLOCK, 0, st>>>(S, velocities, forces, inv_mass, dt, md_items(sys), P, partial,
-                                                         energy, thermo, thermo_rows, counter, done);
+    if (small)
+        md_kick<MD_SMALL_NT, 1><<<grid, MD_SMALL_NT, 0, st>>>(S, velocities, forces, inv_mass, dt, P, partial, energy,
+                                                              thermo, thermo_rows, counter, done);
+    else
+        md_kick<MD_NT, MD_ITEMS><<<grid, MD_NT, 0, st>>>(S, velocities, forces, inv_mass, dt, P, partial, energy,
+                                                         thermo, thermo_rows, counter, done);
     PROF_END("md_kick", st);
     MBF_CHECK_LAUNCH();
     return MBF_OK;
@@ -362,7 +385,7 @@ int mbf_md_kick_drift_check(const mbf_system *sys, double *positions, double *ve
     SysView S = make_view(sys);
     cudaStream_t st = (cudaStream_t)stream;
     PROF_BEGIN("md_kick_drift", st);
-    md_kick_drift_check<<<(sys->n_atoms + MD_BLOCK - 1) / MD_BLOCK, MD_BLOCK, 0, st>>>(
+    md_kick_drift_check<<<(sys->n_atoms + MD_NT - 1) / MD_NT, MD_NT, 0, st>>>(
         S, positions, velocities, forces, inv_mass, dt, ref_positions, d_max, done, r_list, r_cut, d_log, rows,
         counter, gate, cond_handle);
     PROF_END("md_kick_drift", st);
@@ -383,12 +406,18 @@ int mbf_md_kick_kick_drift_check(const mbf_system *sys, double *positions, doubl
         return MBF_ERR_ARGUMENT;
     SysView S = make_view(sys);
     cudaStream_t st = (cudaStream_t)stream;
-    const int P = md_blocks(sys);
+    const bool small = md_small(sys);
+    const int P = md_blocks(sys->n_atoms, small);
+    const dim3 grid(P, sys->n_struct);
     PROF_BEGIN("md_kick_kick_drift", st);
-    md_kick_kick_drift_check<<<dim3(P, sys->n_struct), MD_BLOCK, 0, st>>>(
-        S, positions, velocities, forces, inv_mass, dt, md_items(sys), P, partial, energy, thermo, thermo_rows,
-        thermo_counter,
-        ref_positions, d_max, r_list, r_cut, d_log, skin_counter, gate, cond_handle, done);
+    if (small)
+        md_kick_kick_drift_check<MD_SMALL_NT, 1><<<grid, MD_SMALL_NT, 0, st>>>(
+            S, positions, velocities, forces, inv_mass, dt, P, partial, energy, thermo, thermo_rows, thermo_counter,
+            ref_positions, d_max, r_list, r_cut, d_log, skin_counter, gate, cond_handle, done);
+    else
+        md_kick_kick_drift_check<MD_NT, MD_ITEMS><<<grid, MD_NT, 0, st>>>(
+            S, positions, velocities, forces, inv_mass, dt, P, partial, energy, thermo, thermo_rows, thermo_counter,
+            ref_positions, d_max, r_list, r_cut, d_log, skin_counter, gate, cond_handle, done);
     PROF_END("md_kick_kick_drift", st);
     MBF_CHECK_LAUNCH();
     return MBF_OK;
