@@ -304,7 +304,7 @@ __global__ void nl_cells(SysView S, const int *__restrict__ grids, const int *__
 //
 // Issue-bound, the rank and the tests about half each: 256,000 Cu-Ni atoms at
 // 80 neighbours (21 atoms a cell, 27 x 21 candidates, 62 % of them kept) take
-// 276 us and leave 66 for the rows' copy into the CSR; a warp per cell with
+// 275 us and leave 60 for the rows' copy into the CSR; a warp per cell with
 // the exact test on every candidate took 463 and left 198 for the rows'
 // sorts.  Merging the 27 runs in shared memory instead of ranking by bits
 // took 240 us alone.  Atoms a warp: 3 as 4 (279), 2 worse (the candidates are
@@ -383,7 +383,9 @@ __global__ void __launch_bounds__(NL_T, 4) nl_search(SysView S, const int *__res
                                                   const int *__restrict__ cell_start,
                                                   const float4 *__restrict__ local, int n_cells, double r_list,
                                                   int *__restrict__ row_cnt, int *__restrict__ max_row,
-                                                  int *__restrict__ stage, int stride, int *__restrict__ done) {
+                                                  int *__restrict__ stage, int stride, int *__restrict__ done,
+                                                  const int *__restrict__ searched) {
+    if (*searched == 0) return;  // no cell to try
     __shared__ Stencil st;
     __shared__ float4 cand[NL_CAP];             // x, y, z, atom; ascending
     __shared__ uint4 bits[NL_BITS / 128];       // all zero between cells
@@ -402,7 +404,7 @@ __global__ void __launch_bounds__(NL_T, 4) nl_search(SysView S, const int *__res
     int longest = 0;
     for (int c = blockIdx.x; c < n_cells; c += gridDim.x) {
         const int cs = cell_start[c], na = cell_start[c + 1] - cs;
-        if (na == 0) continue;  // uniform over the block
+        if (na == 0 || !done[c]) continue;  // uniform over the block
         const int mid = __float_as_int(local[cs + na / 2].w);
         const int sidx = S.n_struct > 1 ? S.atom_struct[mid] : 0;
         const double *cell = S.cells + 18 * (size_t)sidx;
@@ -479,7 +481,7 @@ __global__ void __launch_bounds__(NL_T, 4) nl_search(SysView S, const int *__res
         __syncthreads();
         const int base = base_sh, range = range_sh;
         int total = 0;
-        bool wide = grid_is_wide(g) && na <= NL_CAP && range < NL_BITS && bound[0] > 0.0f && bound[1] < 1e30f;
+        bool wide = range < NL_BITS && bound[0] > 0.0f && bound[1] < 1e30f;
         if (wide) {
             // candidates within r_list of the box of the cell's atoms
             bool far = false;
@@ -528,8 +530,8 @@ __global__ void __launch_bounds__(NL_T, 4) nl_search(SysView S, const int *__res
             total = __shfl_sync(MBF_FULL, ahead, 31);
             wide = wide && total <= NL_CAP;
         }
-        if (tid == 0) done[c] = wide ? 1 : 0;
         if (!wide) {  // uniform over the block
+            if (tid == 0) done[c] = 0;
             if (range < NL_BITS)
                 for (int k = tid; k <= range >> 7; k += NL_T) bits[k] = make_uint4(0, 0, 0, 0);
             continue;
@@ -587,18 +589,24 @@ __global__ void __launch_bounds__(NL_T, 4) nl_search(SysView S, const int *__res
 // 4,000 atoms the lines cross at 6 a cell.
 constexpr int NL_BLOCK_ATOMS = 10;
 
-static bool nl_blocks(int n_atoms, int n_cells, const float4 *local) {
-    return local && (long long)n_atoms >= (long long)NL_BLOCK_ATOMS * n_cells;
+// A structure with five cells on each axis, which nl_search needs, has at least
+// NL_WIDE_CELLS; with fewer than that on average its launch is spared (4 cells
+// on an axis, 2048 atoms: 8 us).
+constexpr int NL_WIDE_CELLS = 100;
+
+static bool nl_blocks(const SysView &S, int n_cells, const float4 *local) {
+    return local && (long long)S.n_atoms >= (long long)NL_BLOCK_ATOMS * n_cells &&
+           (long long)n_cells >= (long long)NL_WIDE_CELLS * S.n_struct;
 }
 
 template <int MODE>
 static int nl_rows(const SysView &S, const int *grids, const int *cell_start, const int *cell_atoms,
                    const float4 *local, int n_cells, double r_list, int *row_cnt, int *max_row, const int *row_off,
                    int *nbr, int stride, int *done, cudaStream_t st) {
-    if (MODE == 2 && nl_blocks(S.n_atoms, n_cells, local)) {
+    if (MODE == 2 && nl_blocks(S, n_cells, local)) {
         const int g = persistent_grid(n_cells, NL_T, (const void *)nl_search);
         nl_search<<<g, NL_T, 0, st>>>(S, grids, cell_start, local, n_cells, r_list, row_cnt, max_row, nbr, stride,
-                                      done);
+                                      done, max_row + 1);
     } else {
         done = nullptr;
     }
@@ -671,34 +679,48 @@ __device__ __forceinline__ int sort_row_bitonic(const int *src, int n, int *out,
 // Sorts the n entries src[0..n) (n <= NL_MAXROW) ascending into out[0..n)
 // (src and out may be the same row: every entry is read before any is
 // written) and returns how many are below `a` (warp-uniform).  `row` is
-// the warp's shared scratch of NL_MAXROW ints.
+// the warp's shared scratch of NL_MAXROW ints.  COPIED: a row that is
+// ascending already (the block search's) is only copied.
+template <bool COPIED>
 __device__ __forceinline__ int sort_row(const int *src, int n, int *out, int a, int *row) {
     int lane = threadIdx.x & 31;
     int lower = 0;
-    // a row that is ascending already (the block search's) is only copied;
-    // any other is sorted below, over what was copied
-    bool asc = true;
-    int prev = -1;
-    for (int k0 = 0; k0 < n; k0 += 128) {
+    if (COPIED && n <= 128) {
         int v[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            const int k = k0 + 32 * j + lane;
+            const int k = 32 * j + lane;
             v[j] = k < n ? src[k] : NL_PAD;
         }
+        bool asc = true;
+        int prev = -1;
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            const int k = k0 + 32 * j + lane;
             const int u = __shfl_up_sync(MBF_FULL, v[j], 1);
-            asc = asc && (k >= n || (lane ? u : prev) < v[j]);
+            asc = asc && (32 * j + lane >= n || (lane ? u : prev) < v[j]);
             prev = __shfl_sync(MBF_FULL, v[j], 31);
-            if (k < n && src != out) out[k] = v[j];
-            lower += k < n && v[j] < a ? 1 : 0;
+        }
+        if (__all_sync(MBF_FULL, asc)) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int k = 32 * j + lane;
+                if (k < n && src != out) out[k] = v[j];
+                lower += k < n && v[j] < a ? 1 : 0;
+            }
+            return __reduce_add_sync(MBF_FULL, lower);
+        }
+    } else if (COPIED) {
+        bool asc = true;
+        for (int k = lane; k < n - 1; k += 32) asc = asc && src[k] < src[k + 1];
+        if (__all_sync(MBF_FULL, asc)) {
+            for (int k = lane; k < n; k += 32) {
+                const int v = src[k];
+                if (src != out) out[k] = v;
+                lower += v < a ? 1 : 0;
+            }
+            return __reduce_add_sync(MBF_FULL, lower);
         }
     }
-    if (__all_sync(MBF_FULL, asc)) return __reduce_add_sync(MBF_FULL, lower);
-    __syncwarp();
-    lower = 0;
     if (n <= 32) {
         int v = lane < n ? src[lane] : NL_PAD, rank = 0;
         for (int q = 0; q < n; ++q) rank += __shfl_sync(MBF_FULL, v, q) < v ? 1 : 0;
@@ -732,16 +754,22 @@ __device__ __forceinline__ int sort_row(const int *src, int n, int *out, int a, 
 // float32, beside its index, in the cells' order (NaN for an atom whose cell
 // coordinate lies beyond 4096 boxes): the periodic image next to the cell
 // that nl_assign chose, whatever side of a cell face or of the box's own face
-// the rounding here puts the atom on.
+// the rounding here puts the atom on.  Then too which cells nl_search is to try
+// (done), and whether any: not those of a structure with too few cells on an
+// axis, nor those whose own atoms span nearly all of the index that its map
+// reaches, as in a large structure whose atoms are in no spatial order (the
+// stencil spans more still).  Left to nl_search itself that cost 50 us for
+// 256,000 such atoms.
 __global__ void nl_sort_cells(SysView S, const int *__restrict__ grids, int n_cells,
                               const int *__restrict__ cell_start, int *__restrict__ cell_atoms,
-                              float4 *__restrict__ local) {
+                              float4 *__restrict__ local, int *__restrict__ done, int *__restrict__ searched) {
     __shared__ int srow[NL_WARPS][NL_MAXROW];
     int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    bool any = false;
     for (int c = blockIdx.x * NL_WARPS + wid; c < n_cells; c += gridDim.x * NL_WARPS) {
         int b = cell_start[c], n = cell_start[c + 1] - b;
         if (n <= NL_MAXROW) {
-            sort_row(cell_atoms + b, n, cell_atoms + b, NL_PAD, srow[wid]);
+            sort_row<false>(cell_atoms + b, n, cell_atoms + b, NL_PAD, srow[wid]);
         } else if (lane == 0) {
             for (int i = b + 1; i < b + n; ++i) {
                 int v = cell_atoms[i];
@@ -758,6 +786,21 @@ __global__ void nl_sort_cells(SysView S, const int *__restrict__ grids, int n_ce
         const int sidx = S.n_struct > 1 ? S.atom_struct[cell_atoms[b]] : 0;
         const int *g = grids + 8 * sidx;
         const double *L = S.cells + 18 * (size_t)sidx;
+        const bool wide = grid_is_wide(g);
+        bool take = wide && n <= NL_CAP;
+        if (take && S.n_atoms > NL_BITS) {  // the cell's span as nl_search counts its range
+            const int N = S.n_atoms, mid = cell_atoms[b + n / 2] - N / 2, base = mid + (mid < 0 ? N : 0);
+            int low = N, high = 0;
+            for (int k = lane; k < n; k += 32) {
+                const int v = cell_atoms[b + k], x = v - base + (v < base ? N : 0);
+                low = min(low, x);
+                high = max(high, x);
+            }
+            take = __reduce_max_sync(MBF_FULL, high) - __reduce_min_sync(MBF_FULL, low) < NL_BITS - NL_BITS / 8;
+        }
+        if (lane == 0) done[c] = take ? 1 : 0;
+        any = any || take;
+        if (!wide) continue;  // no cell of the structure is searched by a block
         const int place = c - g[3];
         const double m0 = ((double)(place / (g[1] * g[2])) + 0.5) / (double)g[0];
         const double m1 = ((double)((place / g[2]) % g[1]) + 0.5) / (double)g[1];
@@ -780,6 +823,7 @@ __global__ void nl_sort_cells(SysView S, const int *__restrict__ grids, int n_ce
                                        (float)(f[0] * L[2] + f[1] * L[5] + f[2] * L[8]), __int_as_float(a));
         }
     }
+    if (any && lane == 0) *searched = 1;
 }
 
 // Rows written in traversal order by nl_cells<1>: sorted in place, and
@@ -797,18 +841,22 @@ __global__ void nl_sort_rows(int n_atoms, const int *__restrict__ row_off, int *
             }
             continue;
         }
-        int lower = sort_row(nbr + beg, n, nbr + beg, a, srow[wid]);
+        int lower = sort_row<false>(nbr + beg, n, nbr + beg, a, srow[wid]);
         if (lane == 0) upper[a] = beg + lower;
     }
 }
 
 // The staged rows (nl_cells<2>, nl_search) into the CSR: each row read from its
-// stride-spaced staging slot, sorted where it is not, and written at its scanned offset;
-// its first upper slot recorded.  Rows longer than the stride were refused
-// by the guard (their rows are empty by then).
-__global__ void nl_unstage_rows(int n_atoms, const int *__restrict__ row_off, const int *__restrict__ stage,
-                                int stride, int *__restrict__ nbr, int *__restrict__ upper, int *__restrict__ err) {
-    __shared__ int srow[NL_WARPS][NL_MAXROW];
+// stride-spaced staging slot, sorted where it is not, and written at its scanned
+// offset; its first upper slot recorded.  Rows longer than the stride were
+// refused by the guard (their rows are empty by then).  COPIED where nl_search
+// was launched, *searched whether it had cells: a look at rows that it did not
+// leave costs a tenth of their sorts (256,000 atoms in no order: 229 against 209
+// us, 198 in the kernel without that choice).
+template <bool COPIED>
+__device__ __forceinline__ void unstage_rows(int n_atoms, const int *__restrict__ row_off, const int *__restrict__ stage,
+                                             int stride, int *__restrict__ nbr, int *__restrict__ upper,
+                                             int *__restrict__ err, int *row) {
     int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
     for (int a = blockIdx.x * NL_WARPS + wid; a < n_atoms; a += gridDim.x * NL_WARPS) {
         int beg = row_off[a], n = row_off[a + 1] - beg;
@@ -819,9 +867,20 @@ __global__ void nl_unstage_rows(int n_atoms, const int *__restrict__ row_off, co
             }
             continue;
         }
-        int lower = sort_row(stage + (size_t)a * stride, n, nbr + beg, a, srow[wid]);
+        int lower = sort_row<COPIED>(stage + (size_t)a * stride, n, nbr + beg, a, row);
         if (lane == 0) upper[a] = beg + lower;
     }
+}
+
+template <bool COPIED>
+__global__ void __launch_bounds__(32 * NL_WARPS, COPIED ? 10 : 1)
+    nl_unstage_rows(int n_atoms, const int *__restrict__ row_off, const int *__restrict__ stage, int stride,
+                    const int *__restrict__ searched, int *__restrict__ nbr, int *__restrict__ upper,
+                    int *__restrict__ err) {
+    __shared__ int srow[NL_WARPS][NL_MAXROW];
+    int *row = srow[threadIdx.x >> 5];
+    if (COPIED && *searched) unstage_rows<true>(n_atoms, row_off, stage, stride, nbr, upper, err, row);
+    else unstage_rows<false>(n_atoms, row_off, stage, stride, nbr, upper, err, row);
 }
 
 // Reverse slot of every slot.  rev is an involution, so only the upper
@@ -987,7 +1046,8 @@ static int nl_prepare(const SysView &S, const int *grids, int n_cells_total, dou
     int *mrow = ws_at<int>(workspace, L.maxrow);
     int *scan_ws = ws_at<int>(workspace, L.scan);
     if (cudaMemsetAsync(err, 0, 64, st) != cudaSuccess) return MBF_ERR_CUDA;
-    if (cudaMemsetAsync(mrow, 0, sizeof(int), st) != cudaSuccess) return MBF_ERR_CUDA;
+    // the longest row, and whether nl_search has cells
+    if (cudaMemsetAsync(mrow, 0, 2 * sizeof(int), st) != cudaSuccess) return MBF_ERR_CUDA;
     if (cudaMemsetAsync(cell_count, 0, sizeof(int) * (size_t)n_cells_total, st) != cudaSuccess)
         return MBF_ERR_CUDA;
     PROF_BEGIN("nl_assign", st);
@@ -1004,7 +1064,7 @@ static int nl_prepare(const SysView &S, const int *grids, int n_cells_total, dou
     nl_sort_cells<<<persistent_grid((n_cells_total + NL_WARPS - 1) / NL_WARPS, 32 * NL_WARPS,
                                     (const void *)nl_sort_cells),
                     32 * NL_WARPS, 0, st>>>(S, grids, n_cells_total, cell_start, cell_atoms,
-                                            nl_blocks(N, n_cells_total, local) ? local : nullptr);
+                                            nl_blocks(S, n_cells_total, local) ? local : nullptr, cursor, mrow + 1);
     PROF_END("nl_fill_cells", st);
     MBF_CHECK_LAUNCH();
     PROF_BEGIN("nl_count", st);
@@ -1019,14 +1079,21 @@ static int nl_prepare(const SysView &S, const int *grids, int n_cells_total, dou
 
 static int nl_finish(const SysView &S, const int *grids, int n_cells_total, double r_list, void *workspace,
                      const NlLayout &L, const int *row_off, int *nbr, int *rev, int *upper, cudaStream_t st,
-                     const int *stage = nullptr, int stride = 0) {
+                     const int *stage, int stride, const float4 *local) {
     int N = S.n_atoms;
     int *err = ws_at<int>(workspace, L.err);
     int blocks = (N + NL_WARPS - 1) / NL_WARPS;
-    int g = persistent_grid(blocks, 32 * NL_WARPS, stage ? (const void *)nl_unstage_rows : (const void *)nl_sort_rows);
+    const bool copied = nl_blocks(S, n_cells_total, local);
+    int g = persistent_grid(blocks, 32 * NL_WARPS, !stage   ? (const void *)nl_sort_rows
+                                                   : copied ? (const void *)nl_unstage_rows<true>
+                                                            : (const void *)nl_unstage_rows<false>);
     PROF_BEGIN("nl_fill", st);
     if (stage) {
-        nl_unstage_rows<<<g, 32 * NL_WARPS, 0, st>>>(N, row_off, stage, stride, nbr, upper, err);
+        const int *searched = ws_at<int>(workspace, L.maxrow) + 1;
+        if (copied)
+            nl_unstage_rows<true><<<g, 32 * NL_WARPS, 0, st>>>(N, row_off, stage, stride, searched, nbr, upper, err);
+        else
+            nl_unstage_rows<false><<<g, 32 * NL_WARPS, 0, st>>>(N, row_off, stage, stride, searched, nbr, upper, err);
     } else {
         int rc = nl_rows<1>(S, grids, ws_at<int>(workspace, L.cell_start), ws_at<int>(workspace, L.cell_atoms),
                             nullptr, n_cells_total, r_list, nullptr, nullptr, row_off, nbr, 0, nullptr, st);
@@ -1094,7 +1161,7 @@ int mbf_nl_build(const mbf_system *sys, const int *grids, int n_cells_total, dou
     if (host[1] > NL_MAXROW) return MBF_ERR_ROW_TOO_LONG;
     if (host[1] > stride) stage = nullptr;
     rc = nl_finish(S, grids, n_cells_total, r_list, workspace, L, row_off, nbr, rev, upper, st, stage,
-                   stage ? stride : 0);
+                   stage ? stride : 0, local);
     if (rc != MBF_OK) return rc;
     int herr = 0;
     if (cudaMemcpyAsync(&herr, ws_at<int>(workspace, L.err), sizeof(int), cudaMemcpyDeviceToHost, st) !=
@@ -1138,7 +1205,7 @@ int mbf_nl_rebuild_async(const mbf_system *sys, const int *grids, int n_cells_to
                                err + 4);
     nl_clear_if<<<(N + 256) / 256, 256, 0, st>>>(N, err + 4, row_off, upper);
     MBF_CHECK_LAUNCH();
-    rc = nl_finish(S, grids, n_cells_total, r_list, workspace, L, row_off, nbr, rev, upper, st, stage, max_row_limit);
+    rc = nl_finish(S, grids, n_cells_total, r_list, workspace, L, row_off, nbr, rev, upper, st, stage, max_row_limit, local);
     if (rc != MBF_OK) return rc;
     nl_status_merge<<<1, 32, 0, st>>>(err, status);
     MBF_CHECK_LAUNCH();
