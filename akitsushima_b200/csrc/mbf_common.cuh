@@ -166,19 +166,11 @@ __device__ __forceinline__ T group_sum(T v) {
 template <typename T> struct RT;
 template <> struct RT<double> {
     static __device__ __forceinline__ double ex(double x) { return exp(x); }
-    static __device__ __forceinline__ double sn(double x) { return sin(x); }
-    static __device__ __forceinline__ double cs(double x) { return cos(x); }
     static __device__ __forceinline__ double pw(double x, double y) { return pow(x, y); }
-    static __device__ __forceinline__ double lg(double x) { return log(x); }
-    static __device__ __forceinline__ double sq(double x) { return sqrt(x); }
 };
 template <> struct RT<float> {
     static __device__ __forceinline__ float ex(float x) { return expf(x); }
-    static __device__ __forceinline__ float sn(float x) { return sinf(x); }
-    static __device__ __forceinline__ float cs(float x) { return cosf(x); }
     static __device__ __forceinline__ float pw(float x, float y) { return powf(x, y); }
-    static __device__ __forceinline__ float lg(float x) { return logf(x); }
-    static __device__ __forceinline__ float sq(float x) { return sqrtf(x); }
 };
 
 // Exponential clamped at +-500 (reference engine/_numba_common.py:12-33).

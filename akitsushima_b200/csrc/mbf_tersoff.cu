@@ -11,7 +11,7 @@
 //
 // Owner computes, no atomics: the lane group of centre i evaluates every
 // term of U_i, keeps the force on i and writes -dU_i/dr_x into x's own slot
-// (x -> i); atom a later sums its own row of slots (gather_reduce).
+// (x -> i); atom a later sums its own row of slots (gather_live).
 #include "mbf_rows.cuh"
 
 namespace mbf {
@@ -459,7 +459,7 @@ static int te_launch(const TeArgs &A, cudaStream_t st) {
                                                       (int)A.nl->n_slots, A.clr, A.so);
     PROF_END("te_center", st);
     MBF_CHECK_LAUNCH();
-    return MBF_OK;   // the eval's gather_reduce adds the slot forces
+    return MBF_OK;   // the eval's gather_live adds the slot forces
 }
 
 template <typename T, int MAXN>

@@ -220,7 +220,7 @@ int gather_live(int n_struct, int n_atoms, const int *row_off, int n_slots, cons
     if (plan->n_chunks <= 0 || n_struct <= 0 || plan->n_chunks < n_struct || !sdone) return MBF_ERR_ARGUMENT;
     ChunkSums cs = {plan->chunk, plan->chunk_first, per_atom, partial, energy, virial, sdone};
     const uint4 *mask = reinterpret_cast<const uint4 *>(live_mask);
-    PROF_BEGIN("gather_reduce", st);
+    PROF_BEGIN("gather_live", st);
     const int nt = chunk_block(n_atoms, plan->n_chunks);
     if (nt == 128)
         gather_live_rows<128><<<plan->n_chunks, 128, 0, st>>>(row_off, n_slots, G, mask, row_limit, err, f_local,
@@ -231,7 +231,7 @@ int gather_live(int n_struct, int n_atoms, const int *row_off, int n_slots, cons
     else
         gather_live_rows<512><<<plan->n_chunks, 512, 0, st>>>(row_off, n_slots, G, mask, row_limit, err, f_local,
                                                               forces, cs);
-    PROF_END("gather_reduce", st);
+    PROF_END("gather_live", st);
     MBF_CHECK_LAUNCH();
     return MBF_OK;
 }
