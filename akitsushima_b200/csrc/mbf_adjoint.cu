@@ -430,7 +430,10 @@ __global__ void __launch_bounds__(ADJ_PB, 8) adj_leg_sites(const int *__restrict
                     return w.x * y * a * e + w.y * (yt * a * e + y * at * e + y * a * et);
                 };
                 const double gc = 2.0 * pc * hc2 * iq2 * id2, gct = 4.0 * pc * hc * iq4 * hct;
-                const double gd = c2 * (2.0 * pd * iq4 - 2.0 * id3), gdt = -8.0 * c2 * pd * hc * iq4 * iq2 * hct;
+                // (the difference 2 d / q^2 - 2 / d^3, written without it: q = d^2
+                // + (h - cos)^2 is d^2 to a part in 1e3 to 1e5 for silicon)
+                const double gd = -2.0 * c2 * hc2 * (2.0 * d2 + hc2) * iq4 * id3;
+                const double gdt = -8.0 * c2 * pd * hc * iq4 * iq2 * hct;
                 o[0] += gam * add(gc, gct, f, ft, ex, ext);
                 o[1] += gam * add(gd, gdt, f, ft, ex, ext);
                 o[2] += gam * add(gh, ght, f, ft, ex, ext);
