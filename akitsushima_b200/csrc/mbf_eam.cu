@@ -458,11 +458,11 @@ struct PolGeneric {
 // each function is one aligned vector load of an interval's four
 // coefficients (float4, or double4 in float64) from a table packed into the
 // workspace at the start of the evaluation (4 us).  256k atoms, 2000 knots,
-// mixed: density 289 -> 121 us, force 470 -> 161 us against PolGeneric's
+// mixed: density 289 -> 121 us, force 470 -> 159 us against PolGeneric's
 // search and strided loads (code, parameter row, two knots, four columns, one
 // after the other), which wait on memory.  What bounds it now is the L1 data
-// pipe (72 % of its wavefronts in the density pass): the scattered neighbour
-// records and table records.
+// pipe (85 % of its peak in the density pass, 76 in the force pass): the
+// scattered neighbour records and table records.
 
 template <typename T> struct Vec4;
 template <> struct Vec4<float> {

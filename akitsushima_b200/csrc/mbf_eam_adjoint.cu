@@ -400,7 +400,7 @@ __device__ __forceinline__ bool same_decay(const double *dr, const double *blk) 
 // staged in shared memory per tile of pairs and summed there by entry, with
 // the decays in generic hyper-dual arithmetic, took 714 us for the 4.9 M
 // pairs of 101,000 Ni3Al atoms; this pass takes 228.  Bound by FP64 issue and
-// its latency (36-40 % of the FP64 pipe).
+// its latency (38-45 % of the FP64 pipe).
 // Resident blocks: 4 of 128 registers for the like pairs, 2 of 202 for the
 // cross pairs (101,000 atoms, both: 228 us; 5 spills: 259; 3 cross blocks: 241).
 template <bool LIKE>

@@ -180,7 +180,7 @@ struct SwRow {
 // centre in 64,000-atom Ge-Sn.  The record tables are staged in T (an angle's
 // records were six float64 loads and conversions), legs beyond their own
 // pair's reach are dropped before the angle loop, and the sums over k are in
-// unit vectors: 136 -> 96 us there with the gather, mixed.  (The legs of a
+// unit vectors: 136 -> 92 us there with the gather, mixed.  (The legs of a
 // block as one list, as the Tersoff kernel has them, took 104: its 23 KB of
 // staged legs leave fewer warps resident than the fuller lanes gain.)
 template <typename T, int MAXN, bool SYM, bool STAGED, int LPA>

@@ -202,7 +202,7 @@ __device__ __forceinline__ void te_expo(T l3, T m, T u, T &ex, T &dex) {
 // angle, one angle gives zeta_j's term k and zeta_k's term j one common
 // geometry, and g and g' take one reciprocal.  Blocks are persistent: the
 // tables are loaded once, and the next row's loads are in flight during the
-// current one.  With the gather, SiC above: 62 us (80 with a lane group per
+// current one.  With the gather, SiC above: 60 us (80 with a lane group per
 // centre in every pass and one-shot blocks), against 415 us for a zeta and a
 // force kernel of a lane per bond that evaluated the cutoff functions per
 // angle, each gradient from both of its bonds, and a bond order for the
